@@ -1,6 +1,6 @@
 // Interaction terms shared by the traversal kernels (traverse.cu,
 // traverse_group.cu): the fast 1/sqrt, the cell and particle terms, the
-// far-node expansion, compensated accumulators and the packed-pair terms.
+// far-node expansion and compensated accumulators.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -372,44 +372,5 @@ struct Accum {
     }
 };
 
-
-// Packed-pair terms of the fast path: two sources at once (one instruction
-// for both), each term rounded as the one-at-a-time form rounds it. (x, y, z,
-// m) are the sources, (nmx, nmy, nmz) the negated target position, e2 eps^2;
-// the terms (without G) are added to (sx, sy, sz).
-__device__ __forceinline__ void mono_pair(float2 x, float2 y, float2 z, float2 m, float2 nmx,
-                                          float2 nmy, float2 nmz, float2 e2, float2& sx, float2& sy,
-                                          float2& sz) {
-    const float2 dx = __fadd2_rn(x, nmx), dy = __fadd2_rn(y, nmy), dz = __fadd2_rn(z, nmz);
-    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
-    const float2 inv = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
-    const float2 sc = __fmul2_rn(m, __fmul2_rn(__fmul2_rn(inv, inv), inv));
-    sx = __ffma2_rn(dx, sc, sx);
-    sy = __ffma2_rn(dy, sc, sy);
-    sz = __ffma2_rn(dz, sc, sz);
-}
-// A cell with its quadrupole, given negated (nxx = -Qxx, ..., nzz = -Qzz):
-// inv^3 (M + 5/2 u^2 d.Qd) d - inv^5 Qd with u = 1/r^2, where qx.. = -(Qd)
-// and dqd = -d.Qd, so no negation is needed (IEEE round-to-nearest is
-// symmetric in sign).
-__device__ __forceinline__ void cell_pair_quad(float2 x, float2 y, float2 z, float2 m, float2 nxx,
-                                               float2 nyy, float2 nxy, float2 nxz, float2 nyz,
-                                               float2 nzz, float2 nmx, float2 nmy, float2 nmz,
-                                               float2 e2, float2& sx, float2& sy, float2& sz) {
-    const float2 dx = __fadd2_rn(x, nmx), dy = __fadd2_rn(y, nmy), dz = __fadd2_rn(z, nmz);
-    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
-    const float2 inv = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
-    const float2 u = __fmul2_rn(inv, inv), inv3 = __fmul2_rn(u, inv);
-    const float2 qx = __ffma2_rn(nxx, dx, __ffma2_rn(nxy, dy, __fmul2_rn(nxz, dz)));
-    const float2 qy = __ffma2_rn(nxy, dx, __ffma2_rn(nyy, dy, __fmul2_rn(nyz, dz)));
-    const float2 qz = __ffma2_rn(nxz, dx, __ffma2_rn(nyz, dy, __fmul2_rn(nzz, dz)));
-    const float2 dqd = __ffma2_rn(dx, qx, __ffma2_rn(dy, qy, __fmul2_rn(dz, qz)));
-    const float2 uu = __fmul2_rn(__fmul2_rn(make_float2(-2.5f, -2.5f), u), u);
-    const float2 sa = __fmul2_rn(inv3, __ffma2_rn(uu, dqd, m));
-    const float2 sb = __fmul2_rn(inv3, u);
-    sx = __ffma2_rn(sb, qx, __ffma2_rn(sa, dx, sx));
-    sy = __ffma2_rn(sb, qy, __ffma2_rn(sa, dy, sy));
-    sz = __ffma2_rn(sb, qz, __ffma2_rn(sa, dz, sz));
-}
 
 }  // namespace astro

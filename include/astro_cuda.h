@@ -171,7 +171,9 @@ typedef struct astro_params {
     uint32_t bucket;          /* PHYSICAL: an opened node holding <= bucket
                                  particles is summed particle by particle
                                  (0 = only at layer 0) */
-    uint32_t block_warps;     /* traversal: warps per block (0 = autotuned/default) */
+    uint32_t block_warps;     /* per-particle traversal: warps per block, 2, 4 or 8
+                                 (0 = default); the group walk's kernels have
+                                 their own block sizes */
     uint32_t group_size;      /* PHYSICAL group walk: at most this many consecutive
                                  particles share one tree walk (one warp; two
                                  particles per lane above 32), 1..64; 0 = 32 */
