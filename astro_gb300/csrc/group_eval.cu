@@ -62,7 +62,8 @@ __device__ __forceinline__ void store_particle(const TraverseArgs& a, uint32_t i
 }
 
 // The walk's summed far-node coefficients (group_far_kernel).
-__device__ __forceinline__ void load_far(const float* far_co, float (&fc)[kFarCoefs]) {
+template <bool kExact>
+__device__ __forceinline__ void load_far(const float* far_co, float eps2, float (&fc)[kFarCoefs]) {
     float buf[kFarCoefs + 1];
 #pragma unroll
     for (int k = 0; k < (kFarCoefs + 1) / 4; ++k) {
@@ -71,6 +72,7 @@ __device__ __forceinline__ void load_far(const float* far_co, float (&fc)[kFarCo
     }
 #pragma unroll
     for (int k = 0; k < kFarCoefs; ++k) fc[k] = buf[k];
+    if constexpr (!kExact) far_finish(eps2, fc);
 }
 
 // One warp adds its counts (the same in every lane) to the statistics.
@@ -454,7 +456,7 @@ __global__ __launch_bounds__(kFastWarps * 32, kFastBlocks) void group_eval_fast_
         cell_inter += (uint64_t)gcount * (d.n_far + d.n_cell);
         far_inter += (uint64_t)gcount * d.n_far;
         float fc[kFarCoefs];
-        if (d.n_far > 0) load_far(dp->far_co, fc);
+        if (d.n_far > 0) load_far<false>(dp->far_co, a.eps2, fc);
         for (uint32_t t = lane; t < gcount; t += 32u) {
             const uint32_t k = t / width, q = k >> 1, slot = t % width;
             float s[3];
@@ -524,7 +526,7 @@ __device__ __forceinline__ void eval_group(const TraverseArgs& a, const uint2 gr
     for (int k = 0; k < kPer; ++k) fx[k] = fy[k] = fz[k] = 0.f;
     if (d.n_far > 0) {
         float fc[kFarCoefs];
-        load_far(far_co, fc);
+        load_far<kExact>(far_co, eps2, fc);
 #pragma unroll
         for (int k = 0; k < kPer; ++k)
             far_eval<kExact>(fc, xadd<kExact>(me[k].x, -d.gcx), xadd<kExact>(me[k].y, -d.gcy),

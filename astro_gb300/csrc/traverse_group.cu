@@ -335,13 +335,41 @@ __global__ __launch_bounds__(kWalkWarps * 32, kWalkWarpsPerSm / kWalkWarps) void
 
 // ------------------------------------------------------------ far nodes --
 
+namespace {
+
+// Blocks of four warps per SM (64 registers): the record loaded ahead takes
+// 9 of them. 524,288-body disk 168 us, 4,194,304-body merger 749 us, 256
+// systems 757 us; at 9 blocks (56 registers) 195, 873 and 843 us; 7 blocks
+// the same as 8.
+constexpr int kFarBlocks = 8;
+
+// v[0 .. 2 kHalf) of lane and of lane ^ kBit added; the lane with kBit clear
+// keeps the first half of the sums, the other the second, in v[0 .. kHalf).
+template <int kHalf, int kBit>
+__device__ __forceinline__ void fold_halves(float* v, uint32_t lane) {
+    const bool up = (lane & kBit) != 0;
+#pragma unroll
+    for (int k = 0; k < kHalf; ++k) {
+        const float keep = up ? v[k + kHalf] : v[k], give = up ? v[k] : v[k + kHalf];
+        v[k] = keep + __shfl_xor_sync(kFullMask, give, kBit);
+    }
+}
+
+}  // namespace
+
 // The far-node expansion of every walk, once: lane l sums the coefficients
-// of far nodes l, l + 32, ... in walk order; the partials are combined
-// pairwise (lane l + lane l^o, o = 16 .. 1), leaving the sum in every lane;
-// the 19 sums go into the walk's record, where the evaluation of each group
-// sharing the walk reads them. One warp per record, records in order.
+// of far nodes l, l + 32, ... in walk order, the lanes' partials are combined,
+// and the sums go into the walk's record, where the evaluation of each group
+// sharing the walk reads them (the exact form: pairwise, lane l + lane l^o,
+// o = 16 .. 1; the fast form's sums are finished by far_finish there). One
+// warp per record, records in order.
+//
+// What bounds it: FMA work behind gathered node records. With about 115
+// operations a node instead of 170 (far_coefs_fast) and the next record
+// loaded while the current one is expanded: disk 213 -> 168 us, merger
+// 910 -> 749 us, 16,777,216-body cube 1182 -> 981 us.
 template <bool kExact, bool kQuad>
-__global__ __launch_bounds__(128) void group_far_kernel(TraverseArgs a) {
+__global__ __launch_bounds__(128, kExact ? 1 : kFarBlocks) void group_far_kernel(TraverseArgs a) {
     const uint32_t lane = threadIdx.x & 31;
     // A walk that ran out of room left incomplete lists: nothing to expand.
     if (*reinterpret_cast<volatile const uint32_t*>(a.err) & kErrFrontier) return;
@@ -359,41 +387,69 @@ __global__ __launch_bounds__(128) void group_far_kernel(TraverseArgs a) {
 #pragma unroll
         for (int k = 0; k < kFarCoefs; ++k) fc[k] = 0.f;
         // Far node f sits at position f mod 64 of block f / 64 of the chain.
-        // Each lane reads its next node id (f + 32) before it expands node
-        // f, so only the node record's load waits at the top of an
-        // iteration; the expansions stay in walk order.
-        ChainCursor cur{dp->far_first};
-        uint32_t nd = lane < n_far ? cur.words(a)[lane] : 0u;
-        for (uint32_t f = lane; f < n_far; f += 32u) {
-            const float4 c = __ldg(&a.node_cm[nd]);
-            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-            float qyz = 0.f;
+        // Each lane loads node f + 32's record and reads node f + 64's id
+        // before it expands node f; the expansions stay in walk order.
+        struct Record {
+            float4 c, q;
+            float qyz;
+        };
+        auto load = [&](uint32_t nd) {
+            Record r{__ldg(&a.node_cm[nd]), make_float4(0.f, 0.f, 0.f, 0.f), 0.f};
             if constexpr (kQuad) {
-                q = __ldg(&a.node_q[nd]);
-                qyz = __ldg(&a.node_qyz[nd]);
+                r.q = __ldg(&a.node_q[nd]);
+                r.qyz = __ldg(&a.node_qyz[nd]);
             }
-            const uint32_t fn = f + 32u;
-            if (fn < n_far) {
-                if ((fn % kListBlockWords) < 32u) cur.advance(a);
-                nd = cur.words(a)[fn % kListBlockWords];
-            }
-            if constexpr (kQuad)
-                far_coefs<kExact, true>(c, q, qyz, -(q.x + q.y), gcx, gcy, gcz, eps2, fc);
+            return r;
+        };
+        ChainCursor cur{dp->far_first};
+        // Id of node f, f growing by 32 from call to call.
+        auto id = [&](uint32_t f) -> uint32_t {
+            if (f >= n_far) return 0u;
+            if (f >= kListBlockWords && (f % kListBlockWords) < 32u) cur.advance(a);
+            return __ldg(cur.words(a) + f % kListBlockWords);
+        };
+        Record next = load(id(lane));
+        uint32_t nd = id(lane + 32u);
+        for (uint32_t f = lane; f < n_far; f += 32u) {
+            const Record r = next;
+            next = load(nd);
+            nd = id(f + 64u);
+            if constexpr (kExact)
+                far_coefs_exact<kQuad>(r.c, r.q, r.qyz, -(r.q.x + r.q.y), gcx, gcy, gcz, eps2, fc);
             else
-                far_coefs<kExact, false>(c, q, 0.f, 0.f, gcx, gcy, gcz, eps2, fc);
+                far_coefs_fast<kQuad>(r.c, r.q, r.qyz, gcx, gcy, gcz, eps2, fc);
         }
+        if constexpr (kExact) {
 #pragma unroll
-        for (int k = 0; k < kFarCoefs; ++k) {
-            float v = fc[k];
+            for (int k = 0; k < kFarCoefs; ++k) {
+                float v = fc[k];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v = xadd<kExact>(v, __shfl_xor_sync(kFullMask, v, o));
-            fc[k] = v;
+                for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(kFullMask, v, o));
+                fc[k] = v;
+            }
+            float v = fc[0];
+#pragma unroll
+            for (int k = 1; k < kFarCoefs; ++k)
+                if (lane == (uint32_t)k) v = fc[k];
+            if (lane < (uint32_t)kFarCoefs) dp->far_co[lane] = v;
+        } else {
+            // Each step a lane gives half of its sums to its partner and keeps
+            // the other half: 21 shuffles instead of 95, one sum a lane at the end.
+            float v[20];
+#pragma unroll
+            for (int k = 0; k < kFarCoefs; ++k) v[k] = fc[k];
+            v[19] = 0.f;
+            fold_halves<10, 16>(v, lane);
+            fold_halves<5, 8>(v, lane);
+            v[5] = 0.f;
+            fold_halves<3, 4>(v, lane);
+            v[3] = 0.f;
+            fold_halves<2, 2>(v, lane);
+            fold_halves<1, 1>(v, lane);
+            const uint32_t k3 = 2u * ((lane >> 1) & 1u) + (lane & 1u);
+            const uint32_t k5 = 3u * ((lane >> 2) & 1u) + k3;
+            if (k3 < 3u && k5 < 5u) dp->far_co[10u * (lane >> 4) + 5u * ((lane >> 3) & 1u) + k5] = v[0];
         }
-        float v = fc[0];
-#pragma unroll
-        for (int k = 1; k < kFarCoefs; ++k)
-            if (lane == (uint32_t)k) v = fc[k];
-        if (lane < (uint32_t)kFarCoefs) dp->far_co[lane] = v;
     }
 }
 
@@ -469,7 +525,7 @@ cudaError_t launch_traverse_groups(const TraverseArgs& a, const TraverseConfig& 
     if (e != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[1], st)) != cudaSuccess) return e;
     if (a.far2 > 0.f) {
-        const uint32_t blocks = walk_blocks();
+        const uint32_t blocks = (uint32_t)sm_count() * kFarBlocks;
         if (c.exact)
             c.quad ? group_far_kernel<true, true><<<blocks, 128, 0, st>>>(a)
                    : group_far_kernel<true, false><<<blocks, 128, 0, st>>>(a);
