@@ -72,7 +72,7 @@ __device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v) {
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+    asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(m));  // kept, not read again at each use
     return m;
 }
 

@@ -441,7 +441,6 @@ astro::TraverseArgs traverse_args(astro_ctx* ctx, float dt, bool integrate) {
     // scrambled chunks of 256 measured 4% faster (a single system: 0-2%
     // slower, so it keeps the Morton order).
     a.group_chunk = ctx->nsys > 1 ? 256u : 0u;
-    a.walk_runs = ctx->p.walk_frontier == 0 ? 1u : 0u;
     a.quad = (ctx->p.flags & ASTRO_FLAG_QUADRUPOLE) ? 1u : 0u;
     a.node_crit2 = ctx->node_crit2;
     a.node_q = ctx->node_q;

@@ -35,15 +35,20 @@
 namespace astro {
 namespace {
 
-// Walk kernel: warps per block and the resident warps per SM it is sized for.
+// Walk kernel: warps per block; the resident warps per SM its registers are
+// sized for (80; it uses up to 72) and the ones launched, which then fit.
+// Sized for 28 or 32 (72 and 64 registers) the compiler computes the distances
+// twice, 178 instead of 144 instructions for 32 nodes: 524,288-body disk 248
+// and 245 us against 207; 24 launched: 217 us.
 constexpr int kWalkWarps = 4;
-constexpr int kWalkWarpsPerSm = 32;
+constexpr int kWalkWarpsSized = 24;
+constexpr int kWalkWarpsPerSm = 28;
 constexpr uint32_t kNoBlock = 0xFFFFFFFFu;
 
-// The tail of one list of the group being walked: its first and current
-// blocks, the items in the current block and in the list.
-struct ListTail {
-    uint32_t first, blk, fill, count;
+// A list of the group being walked: its first and last written blocks of the
+// pool and the items in them.
+struct ListOut {
+    uint32_t first, last, done;
 };
 
 // Blocks of the pool a walk warp holds for its lists: [next, end), taken
@@ -51,78 +56,133 @@ struct ListTail {
 constexpr uint32_t kBlockBatch = 16;
 struct BlockCache {
     uint32_t next, end;
+    bool failed;  // a list of this group ran past the pool's end
 };
 
-// Appends the items of the lanes in `mask` (in lane order) to list L, whose
-// items are kWords words each (this lane's words w0, w1). A full block is
-// chained to a new one. Blocks numbered past the pool's end are not
-// written: the walk goes on counting them (the pool counter ends at the
-// demand), `failed` marks the group and the error bit makes the evaluation
-// skip, so the host can grow the pool and run the traversal again.
-// `mask` is warp-uniform.
-template <uint32_t kWords>
-__device__ __forceinline__ void list_append(const TraverseArgs& a, ListTail& L, BlockCache& bc,
-                                            uint32_t mask, uint32_t lane, uint32_t lt, uint32_t w0,
-                                            uint32_t w1, bool& failed) {
-    constexpr uint32_t kCap = kListBlockWords / kWords;
-    const uint32_t cnt = __popc(mask);
-    const uint32_t rank = __popc(mask & lt);
-    auto alloc = [&]() {
-        if (bc.next == bc.end) {
-            uint32_t b = 0;
-            if (lane == 0) b = atomicAdd(a.lists_used, kBlockBatch);
-            b = __shfl_sync(kFullMask, b, 0);
-            bc.next = b;
-            bc.end = b + kBlockBatch;
-        }
-        const uint32_t blk = bc.next++;
-        if (blk >= a.lists_blocks && !failed) {
-            if (lane == 0) atomicOr(a.err, kErrFrontier);
-            failed = true;
-        }
-        return blk;
-    };
-    if (L.blk == kNoBlock) {
-        L.blk = L.first = alloc();
-        L.fill = 0;
+// A warp's buffers, one after the other in slots of two words: the far and
+// cell lists (one block and one chunk's 32 items each), the leaf list (ranges)
+// and the next frontier (runs). A tested node becomes one item of one of them.
+constexpr uint32_t kFarSlot = 0u, kCellSlot = kFarSlot + kListBlockWords + 32u;
+constexpr uint32_t kLeafSlot = kCellSlot + kListBlockWords + 32u, kRunSlot = kLeafSlot + 64u;
+constexpr uint32_t kWalkSlots = kRunSlot + 64u;
+
+// Takes the next block for list L and chains it to the list's last one; n of
+// its items are in it. Blocks numbered past the pool's end are not written:
+// the walk goes on counting them (the pool counter ends at the demand),
+// `failed` marks the group and the error bit makes the evaluation skip, so
+// the host can grow the pool and run the traversal again.
+__device__ __forceinline__ uint32_t next_block(const TraverseArgs& a, ListOut& L, BlockCache& bc,
+                                               uint32_t lane, uint32_t n) {
+    if (bc.next == bc.end) {
+        uint32_t b = 0;
+        if (lane == 0) b = atomicAdd(a.lists_used, kBlockBatch);
+        b = __shfl_sync(kFullMask, b, 0);
+        bc.next = b;
+        bc.end = b + kBlockBatch;
     }
-    uint32_t b = L.blk, slot = L.fill + rank;
-    const uint32_t room = kCap - L.fill;
-    if (cnt > room) {
-        const uint32_t nb = alloc();
-        if (lane == 0 && L.blk < a.lists_blocks && nb < a.lists_blocks) a.list_next[L.blk] = nb;
-        if (rank >= room) {
-            b = nb;
-            slot = rank - room;
-        }
-        L.blk = nb;
-        L.fill = cnt - room;
-    } else {
-        L.fill += cnt;
+    const uint32_t blk = bc.next++;
+    if (blk >= a.lists_blocks) {
+        if (lane == 0 && !bc.failed) atomicOr(a.err, kErrFrontier);
+        bc.failed = true;
+    } else if (lane == 0 && L.last < a.lists_blocks) {
+        a.list_next[L.last] = blk;
     }
-    L.count += cnt;
-    if (((mask >> lane) & 1u) && b < a.lists_blocks) {
-        uint32_t* dst = a.lists + (size_t)b * kListBlockWords + slot * kWords;
-        if constexpr (kWords == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(w0, w1);
-        else *dst = w0;
+    if (L.last == kNoBlock) L.first = blk;
+    L.last = blk;
+    L.done += n;
+    return blk;
+}
+
+// Writes the first n items (at most a block) of a list's buffer to the pool
+// and moves what lies behind the block to the buffer's front: node ids (first
+// words), 64 a block, or ranges, 32 a block.
+__device__ __forceinline__ void write_ids(const TraverseArgs& a, ListOut& L, BlockCache& bc,
+                                          uint2* buf, uint32_t lane, uint32_t n) {
+    const uint32_t blk = next_block(a, L, bc, lane, n);
+    __syncwarp();
+    if (blk < a.lists_blocks) {
+        uint32_t* dst = a.lists + (size_t)blk * kListBlockWords;
+        dst[lane] = buf[lane].x;
+        dst[lane + 32u] = buf[lane + 32u].x;
     }
+    const uint2 rest = buf[kListBlockWords + lane];
+    __syncwarp();
+    buf[lane] = rest;
+}
+__device__ __forceinline__ void write_ranges(const TraverseArgs& a, ListOut& L, BlockCache& bc,
+                                             uint2* buf, uint32_t lane, uint32_t n) {
+    const uint32_t blk = next_block(a, L, bc, lane, n);
+    __syncwarp();
+    if (blk < a.lists_blocks)
+        reinterpret_cast<uint2*>(a.lists + (size_t)blk * kListBlockWords)[lane] = buf[lane];
+    const uint2 rest = buf[32u + lane];
+    __syncwarp();
+    buf[lane] = rest;
+}
+// The same for n <= 32 runs of the next frontier, at position `at` of nxt; a
+// frontier buffer that is too small records what it wanted and drops them.
+__device__ __forceinline__ uint32_t write_runs(const TraverseArgs& a, uint2* nxt, uint32_t at,
+                                               uint2* buf, uint32_t lane, uint32_t n) {
+    __syncwarp();
+    const bool fits = at + n <= a.frontier_cap / 2u;
+    if (fits) {
+        if (lane < n) nxt[at + lane] = buf[lane];
+    } else if (lane == 0) {
+        atomicOr(a.err, kErrFrontier);
+        atomicMax(a.frontier_need, 2u * (at + n));
+    }
+    const uint2 rest = buf[32u + lane];
+    __syncwarp();
+    buf[lane] = rest;
+    return fits ? at + n : at;
+}
+
+// A left shift that gives 0 for counts of 32 and more.
+__device__ __forceinline__ uint32_t shl_clamped(uint32_t v, uint32_t n) {
+    uint32_t r;
+    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(n));
+    return r;
+}
+
+// Minimum and maximum over the warp (NaNs lose, as with fminf / fmaxf).
+__device__ __forceinline__ float warp_min_f32(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max_f32(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
 }
 
 }  // namespace
 
 // ------------------------------------------------------------------ walk --
 
-__global__ __launch_bounds__(kWalkWarps * 32, kWalkWarpsPerSm / kWalkWarps) void group_walk_kernel(
+// What bounds it: instruction issue (72% of the cycles with 24 warps), then the
+// latency of the node records. So the work for 32 nodes is kept short: a
+// node's run comes from one reduction and a population count; three votes
+// give the four classes (far, near, leaf, opened), and each lane stores its
+// one item into its class's shared buffer without a branch; blocks of the
+// lists and the frontier go to memory when a buffer is full. 182 -> 144
+// instructions for 32 nodes. Walks of a 524,288-body disk 333 -> 207 us, two
+// Plummer spheres of 4,194,304 1180 -> 733 us, 256 systems 1740 -> 1090 us,
+// 16,777,216-body cube 1262 -> 842 us, 16,384-body sphere 41 -> 25 us.
+template <bool kDelta, bool kFar>
+__global__ __launch_bounds__(kWalkWarps * 32, kWalkWarpsSized / kWalkWarps) void group_walk_kernel(
     TraverseArgs a) {
+    __shared__ uint2 s_walk[kWalkWarps][kWalkSlots];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t lt = lanemask_lt();
+    uint2* const buf = s_walk[warp];
+    const uint32_t lt = lanemask_lt(), le = lt | (1u << lane);
     const uint32_t gw = blockIdx.x * kWalkWarps + warp;
-    uint32_t* const buf0 = a.frontier + (size_t)gw * 2 * a.frontier_cap;
-    uint32_t* const buf1 = buf0 + a.frontier_cap;
+    uint32_t* const words = a.frontier + (size_t)gw * 2 * a.frontier_cap;
+    uint2* const buf0 = reinterpret_cast<uint2*>(words);
+    uint2* const buf1 = reinterpret_cast<uint2*>(words + a.frontier_cap);
     const uint32_t ngroups = *a.group_count;
-    const bool far_on = a.far2 > 0.f;
     unsigned long long visits = 0, far_nodes = 0;
-    BlockCache bcache{0u, 0u};
+    BlockCache bcache{0u, 0u, false};
 
     while (true) {
         uint32_t gi = 0;
@@ -151,15 +211,8 @@ __global__ __launch_bounds__(kWalkWarps * 32, kWalkWarpsPerSm / kWalkWarps) void
                 hi_x = fmaxf(hi_x, p1.x), hi_y = fmaxf(hi_y, p1.y), hi_z = fmaxf(hi_z, p1.z);
             }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo_x = fminf(lo_x, __shfl_xor_sync(kFullMask, lo_x, o));
-            lo_y = fminf(lo_y, __shfl_xor_sync(kFullMask, lo_y, o));
-            lo_z = fminf(lo_z, __shfl_xor_sync(kFullMask, lo_z, o));
-            hi_x = fmaxf(hi_x, __shfl_xor_sync(kFullMask, hi_x, o));
-            hi_y = fmaxf(hi_y, __shfl_xor_sync(kFullMask, hi_y, o));
-            hi_z = fmaxf(hi_z, __shfl_xor_sync(kFullMask, hi_z, o));
-        }
+        lo_x = warp_min_f32(lo_x), lo_y = warp_min_f32(lo_y), lo_z = warp_min_f32(lo_z);
+        hi_x = warp_max_f32(hi_x), hi_y = warp_max_f32(hi_y), hi_z = warp_max_f32(hi_z);
         const float gcx = __fmul_rn(__fadd_rn(lo_x, hi_x), 0.5f);
         const float gcy = __fmul_rn(__fadd_rn(lo_y, hi_y), 0.5f);
         const float gcz = __fmul_rn(__fadd_rn(lo_z, hi_z), 0.5f);
@@ -170,152 +223,134 @@ __global__ __launch_bounds__(kWalkWarps * 32, kWalkWarpsPerSm / kWalkWarps) void
             __fadd_rn(__fmul_rn(hrx, hrx), __fadd_rn(__fmul_rn(hry, hry), __fmul_rn(hrz, hrz)));
         const uint32_t sys = a.nsys > 1 ? (uint32_t)(a.sorted_keys[gr.x] >> (3u * a.lbits)) : 0u;
         const float* crit_layer = a.sys[sys].crit2;
-        ListTail cells{kNoBlock, kNoBlock, 0u, 0u}, leaves = cells, fars = cells;
-        bool failed = false;
+        ListOut cells{kNoBlock, kNoBlock, 0u}, leaves = cells, fars = cells;
+        uint32_t far_n = 0, cell_n = 0, leaf_n = 0;  // items in the buffers
+        bcache.failed = false;
         uint32_t tested = 0;
 
-        // One frontier chunk: node nd (when `has`) at `layer`. Appends the
-        // accepted, far and opened-leaf nodes to the lists in frontier order
-        // and returns the opened node's child range (empty otherwise).
-        auto test_nodes = [&](bool has, uint32_t nd, int layer) -> uint2 {
-            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-            uint4 r = make_uint4(0u, 0u, 0u, 0u);
-            float crit = 0.f;
-            if (has) {
-                c = __ldg(&a.node_cm[nd]);
-                r = __ldg(&a.node_rng[nd]);
-                crit = a.delta ? __ldg(&a.node_crit2[nd]) : __ldg(&crit_layer[layer]);
-            }
-            const float bx = fmaxf(fmaxf(__fsub_rn(lo_x, c.x), __fsub_rn(c.x, hi_x)), 0.f);
-            const float by = fmaxf(fmaxf(__fsub_rn(lo_y, c.y), __fsub_rn(c.y, hi_y)), 0.f);
-            const float bz = fmaxf(fmaxf(__fsub_rn(lo_z, c.z), __fsub_rn(c.z, hi_z)), 0.f);
-            const float dist2 =
-                __fadd_rn(__fadd_rn(__fmul_rn(bx, bx), __fmul_rn(by, by)), __fmul_rn(bz, bz));
-            const bool accepted = has && dist2 > crit;
-            const bool leaf = has && !accepted && (layer == 0 || r.w - r.z <= a.bucket);
-            const bool opn = has && !accepted && !leaf;
-            bool far = false;
-            if (far_on && accepted) {
-                const float Dx = __fsub_rn(c.x, gcx), Dy = __fsub_rn(c.y, gcy), Dz = __fsub_rn(c.z, gcz);
-                const float D2 =
-                    __fadd_rn(__fmul_rn(Dx, Dx), __fadd_rn(__fmul_rn(Dy, Dy), __fmul_rn(Dz, Dz)));
-                far = __fmul_rn(a.far2, D2) > rg2;
-            }
-            const bool acc = accepted && !far;
-            tested += __popc(__ballot_sync(kFullMask, has));
-            const uint32_t bfar = __ballot_sync(kFullMask, far);
-            if (bfar) list_append<1>(a, fars, bcache, bfar, lane, lt, nd, 0u, failed);
-            const uint32_t bacc = __ballot_sync(kFullMask, acc);
-            if (bacc) list_append<1>(a, cells, bcache, bacc, lane, lt, nd, 0u, failed);
-            const uint32_t bleaf = __ballot_sync(kFullMask, leaf);
-            if (bleaf) list_append<2>(a, leaves, bcache, bleaf, lane, lt, r.z, r.w, failed);
-            return opn ? make_uint2(r.x, r.y) : make_uint2(0u, 0u);
-        };
-
-        if (a.walk_runs) {
-            // The frontier holds runs of consecutive node indices (first,
-            // count) in walk order: an opened node's children are consecutive,
-            // so it adds one run, and a chunk of 32 nodes is found by a shuffle
-            // search over 32 runs loaded at once.
-            uint2* cur = reinterpret_cast<uint2*>(buf0);
-            uint2* nxt = reinterpret_cast<uint2*>(buf1);
-            const uint32_t run_cap = a.frontier_cap / 2u;
-            if (lane == 0) cur[0] = make_uint2(a.sys[sys].root, 1u);
-            uint32_t ncur = 1;
-            int layer = (int)a.lbits;
-            __syncwarp();
-            while (ncur > 0) {
-                uint32_t nnext = 0;
-                for (uint32_t rb = 0; rb < ncur; rb += 32u) {
-                    const uint32_t nrun = min(32u, ncur - rb);
-                    const uint2 run = lane < nrun ? cur[rb + lane] : make_uint2(0u, 0u);
-                    uint32_t rincl = run.y;
+        // The frontier holds runs of consecutive node indices (first, count)
+        // in walk order: an opened node's children are consecutive, so it
+        // adds one run. 32 runs are taken at once and their nodes tested 32
+        // at a time: the runs starting in a window of 32 nodes set a bit, and
+        // a node's run is the count of starts up to it. A frontier of at most
+        // 32 runs stays in registers and shared memory.
+        uint2* cur = buf0;
+        uint2* nxt = buf1;
+        const uint32_t root = a.sys[sys].root;
+        uint2 first_runs = lane == 0 ? make_uint2(root, 1u) : make_uint2(0u, 0u);
+        bool stored = false;  // the frontier is in cur (else in first_runs)
+        uint32_t ncur = 1;
+        int layer = (int)a.lbits;
+        while (ncur > 0) {
+            uint32_t nnext = 0, run_n = 0;
+            float crit_l = 0.f;
+            if constexpr (!kDelta) crit_l = __ldg(&crit_layer[layer]);
+            for (uint32_t rb = 0; rb < ncur; rb += 32u) {
+                const bool is_run = rb + lane < ncur;
+                uint2 run = first_runs;
+                if (stored) run = is_run ? cur[rb + lane] : make_uint2(0u, 0u);
+                uint32_t incl = run.y;
 #pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t y = __shfl_up_sync(kFullMask, rincl, o);
-                        if (lane >= (uint32_t)o) rincl += y;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+                    if (lane >= (uint32_t)o) incl += y;
+                }
+                const uint32_t total = __shfl_sync(kFullMask, incl, 31);
+                // First node of this lane's run; lanes without one never start.
+                const uint32_t pre = is_run ? incl - run.y : 0x80000000u;
+                const uint32_t base = run.x - (incl - run.y);
+                uint32_t before = ~0u;  // runs started in earlier windows, less one
+                tested += total;
+                for (uint32_t t0 = 0; t0 < total; t0 += 32u) {
+                    const uint32_t starts = __reduce_or_sync(kFullMask, shl_clamped(1u, pre - t0));
+                    const uint32_t e = before + __popc(starts & le);
+                    before += __popc(starts);
+                    // Lanes past the last node load the root, and drop it.
+                    const uint32_t present = min(32u, total - t0);
+                    const bool has = lane < present;
+                    const uint32_t at = __shfl_sync(kFullMask, base, e & 31u) + t0 + lane;
+                    const uint32_t nd = has ? at : root;
+                    const float4 c = __ldg(&a.node_cm[nd]);
+                    const uint4 r = __ldg(&a.node_rng[nd]);
+                    const float crit = kDelta ? __ldg(&a.node_crit2[nd]) : crit_l;
+                    const float bx = fmaxf(fmaxf(__fsub_rn(lo_x, c.x), __fsub_rn(c.x, hi_x)), 0.f);
+                    const float by = fmaxf(fmaxf(__fsub_rn(lo_y, c.y), __fsub_rn(c.y, hi_y)), 0.f);
+                    const float bz = fmaxf(fmaxf(__fsub_rn(lo_z, c.z), __fsub_rn(c.z, hi_z)), 0.f);
+                    const float dist2 =
+                        __fadd_rn(__fadd_rn(__fmul_rn(bx, bx), __fmul_rn(by, by)), __fmul_rn(bz, bz));
+                    const bool accepted = dist2 > crit;
+                    const uint32_t mpresent = ~0u >> (32u - present);
+                    const uint32_t macc = __ballot_sync(kFullMask, accepted) & mpresent;
+                    uint32_t mfar = 0;
+                    bool far = false;
+                    if constexpr (kFar) {
+                        const float Dx = __fsub_rn(c.x, gcx), Dy = __fsub_rn(c.y, gcy),
+                                    Dz = __fsub_rn(c.z, gcz);
+                        const float D2 = __fadd_rn(__fmul_rn(Dx, Dx),
+                                                   __fadd_rn(__fmul_rn(Dy, Dy), __fmul_rn(Dz, Dz)));
+                        far = __fmul_rn(a.far2, D2) > rg2;
+                        mfar = __ballot_sync(kFullMask, far) & macc;
                     }
-                    const uint32_t rpre = rincl - run.y;
-                    const uint32_t rtotal = __shfl_sync(kFullMask, rincl, 31);
-                    for (uint32_t t0 = 0; t0 < rtotal; t0 += 32u) {
-                        const uint32_t pos = t0 + lane;
-                        uint32_t e = 0;
-#pragma unroll
-                        for (uint32_t step = 16; step > 0; step >>= 1) {
-                            const uint32_t cand = e + step;
-                            const uint32_t pc = __shfl_sync(kFullMask, rpre, cand & 31u);
-                            if (cand < nrun && pc <= pos) e = cand;
+                    const bool leaf = layer == 0 || r.w - r.z <= a.bucket;
+                    const uint32_t mleaf = __ballot_sync(kFullMask, leaf) & (mpresent & ~macc);
+                    // This lane's class: the lanes in it, its buffer's next
+                    // slot, and the item's words.
+                    const uint32_t mnear = macc & ~mfar, mopen = mpresent & ~macc & ~mleaf;
+                    const uint32_t mine = accepted ? (far ? mfar : mnear) : (leaf ? mleaf : mopen);
+                    const uint32_t slot = accepted ? (far ? kFarSlot + far_n : kCellSlot + cell_n)
+                                                   : (leaf ? kLeafSlot + leaf_n : kRunSlot + run_n);
+                    const uint2 item = make_uint2(accepted ? nd : (leaf ? r.z : r.x),
+                                                  leaf ? r.w : r.y - r.x);
+                    if (has) buf[slot + __popc(mine & lt)] = item;
+                    const uint32_t nacc = __popc(macc), nfar = __popc(mfar), nleaf = __popc(mleaf);
+                    far_n += nfar;
+                    cell_n += nacc - nfar;
+                    leaf_n += nleaf;
+                    run_n += present - nacc - nleaf;
+                    if (max(max(far_n, cell_n), 2u * max(leaf_n, run_n)) >= kListBlockWords) {
+                        if (kFar && far_n >= kListBlockWords) {
+                            write_ids(a, fars, bcache, buf + kFarSlot, lane, kListBlockWords);
+                            far_n -= kListBlockWords;
                         }
-                        const uint32_t first = __shfl_sync(kFullMask, run.x, e);
-                        const uint32_t estart = __shfl_sync(kFullMask, rpre, e);
-                        const bool has = pos < rtotal;
-                        const uint2 ch = test_nodes(has, has ? first + (pos - estart) : 0u, layer);
-                        const bool opn = ch.y > ch.x;
-                        const uint32_t bopen = __ballot_sync(kFullMask, opn);
-                        if (bopen) {
-                            if (nnext + __popc(bopen) <= run_cap) {
-                                if (opn) nxt[nnext + __popc(bopen & lt)] = make_uint2(ch.x, ch.y - ch.x);
-                                nnext += __popc(bopen);
-                            } else if (lane == 0) {
-                                atomicOr(a.err, kErrFrontier);
-                                atomicMax(a.frontier_need, 2u * (nnext + __popc(bopen)));
-                            }
+                        if (cell_n >= kListBlockWords) {
+                            write_ids(a, cells, bcache, buf + kCellSlot, lane, kListBlockWords);
+                            cell_n -= kListBlockWords;
+                        }
+                        if (leaf_n >= 32u) {
+                            write_ranges(a, leaves, bcache, buf + kLeafSlot, lane, 32u);
+                            leaf_n -= 32u;
+                        }
+                        if (run_n >= 32u) {
+                            nnext = write_runs(a, nxt, nnext, buf + kRunSlot, lane, 32u);
+                            run_n -= 32u;
                         }
                     }
                 }
-                __syncwarp();
+            }
+            stored = nnext > 0;
+            if (stored) {
+                if (run_n > 0) nnext = write_runs(a, nxt, nnext, buf + kRunSlot, lane, run_n);
+                ncur = nnext;
                 uint2* t = cur;
                 cur = nxt;
                 nxt = t;
-                ncur = nnext;
-                --layer;
+            } else {
+                ncur = run_n;
             }
-        } else {
-            // The frontier holds node indices, each opened node adding its
-            // children one by one.
-            uint32_t* cur = buf0;
-            uint32_t* nxt = buf1;
-            if (lane == 0) cur[0] = a.sys[sys].root;
-            uint32_t ncur = 1;
-            int layer = (int)a.lbits;
             __syncwarp();
-            while (ncur > 0) {
-                uint32_t nnext = 0;
-                for (uint32_t base = 0; base < ncur; base += 32u) {
-                    const uint32_t k = base + lane;
-                    const bool has = k < ncur;
-                    const uint2 ch = test_nodes(has, has ? cur[k] : 0u, layer);
-                    const uint32_t cnt = ch.y - ch.x;
-                    uint32_t incl = cnt;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
-                        if (lane >= (uint32_t)o) incl += y;
-                    }
-                    const uint32_t total = __shfl_sync(kFullMask, incl, 31);
-                    if (nnext + total <= a.frontier_cap) {
-                        const uint32_t o0 = nnext + incl - cnt;
-                        for (uint32_t j = 0; j < cnt; ++j) nxt[o0 + j] = ch.x + j;
-                        nnext += total;
-                    } else if (lane == 0) {
-                        atomicOr(a.err, kErrFrontier);
-                        atomicMax(a.frontier_need, nnext + total);
-                    }
-                }
-                __syncwarp();
-                uint32_t* t = cur;
-                cur = nxt;
-                nxt = t;
-                ncur = nnext;
-                --layer;
-            }
+            first_runs = lane < ncur ? buf[kRunSlot + lane] : make_uint2(0u, 0u);
+            __syncwarp();
+            --layer;
         }
+        if (far_n) write_ids(a, fars, bcache, buf + kFarSlot, lane, far_n);
+        if (cell_n) write_ids(a, cells, bcache, buf + kCellSlot, lane, cell_n);
+        if (leaf_n) write_ranges(a, leaves, bcache, buf + kLeafSlot, lane, leaf_n);
 
         // The group's descriptor (empty lists if the pool ran out).
-        if (failed) leaves.count = cells.count = fars.count = 0;
+        if (bcache.failed) leaves.done = cells.done = fars.done = 0;
         if (lane < 12) {
-            const uint32_t w[12] = {leaves.first, leaves.count, cells.first, cells.count,
-                                    fars.first, fars.count, __float_as_uint(gcx), __float_as_uint(gcy),
+            const uint32_t w[12] = {leaves.first, leaves.done, cells.first, cells.done,
+                                    fars.first, fars.done, __float_as_uint(gcx), __float_as_uint(gcy),
                                     __float_as_uint(gcz), 0u, 0u, 0u};
             uint32_t v = w[0];
 #pragma unroll
@@ -325,7 +360,7 @@ __global__ __launch_bounds__(kWalkWarps * 32, kWalkWarpsPerSm / kWalkWarps) void
         }
         // Per particle of the walk; one expansion per walk and far node.
         visits += (unsigned long long)wcount * tested;
-        far_nodes += fars.count;
+        far_nodes += fars.done;
     }
     if (lane == 0) {
         atomicAdd(&a.stats[1], visits);
@@ -459,7 +494,6 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 int g_sms[kMaxDevices] = {};
-int g_walk_per_sm[kMaxDevices] = {};
 std::mutex g_mutex;
 
 int device_index() {
@@ -479,21 +513,7 @@ int sm_count() {
     return g_sms[dev];
 }
 
-uint32_t walk_blocks() {
-    const int dev = device_index();
-    int per_sm = 0;
-    {
-        std::lock_guard<std::mutex> lock(g_mutex);
-        per_sm = g_walk_per_sm[dev];
-    }
-    if (per_sm == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, group_walk_kernel, kWalkWarps * 32, 0);
-        per_sm = std::max(1, per_sm);
-        std::lock_guard<std::mutex> lock(g_mutex);
-        g_walk_per_sm[dev] = per_sm;
-    }
-    return (uint32_t)per_sm * (uint32_t)sm_count();
-}
+uint32_t walk_blocks() { return (uint32_t)sm_count() * (kWalkWarpsPerSm / kWalkWarps); }
 
 }  // namespace
 
@@ -520,7 +540,9 @@ cudaError_t launch_traverse_groups(const TraverseArgs& a, const TraverseConfig& 
     e = cudaMemsetAsync(a.eval_queue, 0, 2 * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[0], st)) != cudaSuccess) return e;
-    group_walk_kernel<<<walk_blocks(), kWalkWarps * 32, 0, st>>>(a);
+    auto walk = a.delta ? (a.far2 > 0.f ? group_walk_kernel<true, true> : group_walk_kernel<true, false>)
+                        : (a.far2 > 0.f ? group_walk_kernel<false, true> : group_walk_kernel<false, false>);
+    walk<<<walk_blocks(), kWalkWarps * 32, 0, st>>>(a);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[1], st)) != cudaSuccess) return e;

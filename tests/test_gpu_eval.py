@@ -63,3 +63,24 @@ def test_small_softening(ag, oracle, eps):
     p = ag.default_params(L.PRESET_PHYSICAL, lbits=7, group_size=40, softening=eps, far_ratio=0.2)
     pm, vr = ic.plummer(3000, seed=8)
     _check(ag, oracle, p, pm, vr)
+
+
+@pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("far", [0.0, 0.3])
+@pytest.mark.parametrize("n,lbits,theta", [(1, 4, 0.7), (40, 2, 0.7), (6000, 10, 0.7), (3000, 5, 0.2)])
+def test_walk_variants_bit_exact(ag, oracle, delta, far, n, lbits, theta):
+    """The walk's four variants, with frontiers below and above the 32 runs
+    that stay on chip and lists that end inside and at a block: counts and
+    (in the exact form, which sums in list order) accelerations are equal."""
+    from astro_gb300 import ic
+    from test_gpu_parity import run_gpu
+
+    L = ag.layouts
+    flags = L.FLAG_IEEE_EXACT | L.FLAG_QUADRUPOLE | (L.FLAG_OPEN_DELTA if delta else 0)
+    p = ag.default_params(L.PRESET_PHYSICAL, lbits=lbits, theta=theta, far_ratio=far, flags=flags,
+                          bucket=4, group_size=24)
+    pm, vr = ic.plummer(n, seed=77)
+    out = run_gpu(ag, p, pm, vr, dt=1e-3, steps=1)
+    ref = oracle.phys_run(p, pm.copy(), vr.copy(), dt=1e-3, steps=1)
+    assert np.array_equal(out["acc4"], ref["acc4"])
+    assert out["interactions"] == ref["interactions"] and out["node_visits"] == ref["node_visits"]
