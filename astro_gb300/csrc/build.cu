@@ -11,6 +11,7 @@
 // are aggregated one launch each and the small top layers in one climbing
 // launch (aggregate_tree_kernel).
 #include <algorithm>
+#include <type_traits>
 
 #include "build_kernels.cuh"
 #include "common.cuh"
@@ -392,37 +393,48 @@ __device__ __forceinline__ float4 com_from_sums(double sx, double sy, double sz,
 // Slots for c groups of this thread: the active lanes of the warp add their
 // counts and one lane claims them with a single atomic (one atomic per warp
 // instead of one per group on the shared counter); lanes take their runs in
-// lane order.
+// lane order. Most calls have nothing to claim.
 __device__ __forceinline__ uint32_t reserve_groups(uint32_t* counter, uint32_t c) {
     const uint32_t mask = __activemask();
+    const uint32_t some = __ballot_sync(mask, c != 0u);
+    if (some == 0u) return 0u;
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t prefix = 0, total = 0;
-    for (uint32_t m = mask; m != 0u; m &= m - 1u) {
+    for (uint32_t m = some; m != 0u; m &= m - 1u) {
         const uint32_t l = (uint32_t)__ffs(m) - 1u;
         const uint32_t cl = __shfl_sync(mask, c, l);
         if (l < lane) prefix += cl;
         total += cl;
     }
-    const uint32_t leader = (uint32_t)__ffs(mask) - 1u;
+    const uint32_t leader = (uint32_t)__ffs(some) - 1u;
     uint32_t base = 0;
-    if (lane == leader && total != 0u) base = atomicAdd(counter, total);
+    if (lane == leader) base = atomicAdd(counter, total);
     return __shfl_sync(mask, base, leader) + prefix;
 }
 
-// Visits the particles [pb, pe) in order, loading four at a time so that
-// four loads are in flight (the sums stay in particle order).
+// Visits the particles [pb, pe) in order (the sums stay in particle order),
+// four at a time with the next four loaded ahead. One thread sums a leaf, so
+// a crowded leaf is a chain of load latencies: with one batch in flight the
+// leaf pass of a 524,288-body disk (leaves of up to about 70) took 47 us.
 template <typename F>
 __device__ __forceinline__ void for_particles(const float4* __restrict__ pos, uint32_t pb,
                                               uint32_t pe, F&& f) {
-    uint32_t i = pb;
-    for (; i + 4u <= pe; i += 4u) {
-        float4 q[4];
+    constexpr uint32_t kBatch = 4;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 next[kBatch];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) q[u] = __ldg(&pos[i + u]);
+    for (uint32_t u = 0; u < kBatch; ++u) next[u] = pb + u < pe ? __ldg(&pos[pb + u]) : zero;
+    for (uint32_t i = pb; i < pe; i += kBatch) {
+        float4 q[kBatch];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) f(q[u]);
+        for (uint32_t u = 0; u < kBatch; ++u) {
+            q[u] = next[u];
+            next[u] = i + kBatch + u < pe ? __ldg(&pos[i + kBatch + u]) : zero;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kBatch; ++u)
+            if (i + u < pe) f(q[u]);
     }
-    for (; i < pe; ++i) f(__ldg(&pos[i]));
 }
 
 // Mass moments of a leaf's particles about a point c (the cell's centre):
@@ -474,123 +486,47 @@ struct CellMoments {
     }
 };
 
-// aggregateLeafNodes (Octree.metal:53-117), one thread per leaf.
-// kMode 0 (REFERENCE): state in upload order, gathered through perm; FP32
-//   sums of m and x*m in sorted order; the last leaf sums [start, numUnique)
-//   as the reference does (Octree.metal:71).
-// kMode 1 (PHYSICAL plain): state already in sorted order; raw FP32 sums.
-// kMode 2 (PHYSICAL precision): FP64 sums of m and m*x over the FP32
-//   positions relative to the system origin.
-template <int kMode, bool kQuad>
-__device__ __forceinline__ void aggregate_leaf_node_q(const AggArgs& a, uint32_t j, uint32_t u0) {
+// REFERENCE: aggregateLeafNodes (Octree.metal:53-117), one thread per leaf.
+// State in upload order, gathered through perm; FP32 sums of m and x*m in
+// sorted order; the last leaf sums [start, numUnique) as the reference does
+// (Octree.metal:71).
+__device__ __forceinline__ void aggregate_ref_leaf(const AggArgs& a, uint32_t j, uint32_t u0) {
     const uint32_t pb = a.pbeg[j];
     const uint32_t pe = (j + 1 < u0) ? a.pbeg[j + 1] : a.n;
-    // PHYSICAL quadrupole in the same read of the particles as the sums:
-    // moments about the cell's centre, shifted to the centre of mass after.
-    uint64_t node_key = 0;
-    float4 box = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (kMode != 0 && (kQuad || a.want_delta)) node_key = a.node_key[j];
-    if (kQuad) box = cell_box(a, node_key, 0);
-    CellMoments mom;
+    const uint32_t sum_end = (j + 1 < u0) ? pe : u0;
     float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (kMode == 0) {
-        const uint32_t sum_end = (j + 1 < u0) ? pe : u0;
-        float m = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
-        // Stars (type 0): colours summed, positions averaged (Octree.metal:85-99).
-        float4 ec = make_float4(0.f, 0.f, 0.f, 0.f), en = ec;
-        uint32_t suns = 0;
-        for (uint32_t i = pb; i < sum_end; ++i) {
-            const uint32_t pi = a.perm[i];
-            const float4 q = a.pos[pi];
-            m = __fadd_rn(m, q.w);
-            sx = __fadd_rn(sx, __fmul_rn(q.x, q.w));
-            sy = __fadd_rn(sy, __fmul_rn(q.y, q.w));
-            sz = __fadd_rn(sz, __fmul_rn(q.z, q.w));
-            if (a.node_ecol && a.types[pi] == 0u) {
-                const float4 c = a.colors[pi];
-                ec = make_float4(__fadd_rn(ec.x, c.x), __fadd_rn(ec.y, c.y), __fadd_rn(ec.z, c.z),
-                                 __fadd_rn(ec.w, c.w));
-                en = make_float4(__fadd_rn(en.x, q.x), __fadd_rn(en.y, q.y), __fadd_rn(en.z, q.z), 0.f);
-                ++suns;
-            }
+    float m = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
+    // Stars (type 0): colours summed, positions averaged (Octree.metal:85-99).
+    float4 ec = make_float4(0.f, 0.f, 0.f, 0.f), en = ec;
+    uint32_t suns = 0;
+    for (uint32_t i = pb; i < sum_end; ++i) {
+        const uint32_t pi = a.perm[i];
+        const float4 q = a.pos[pi];
+        m = __fadd_rn(m, q.w);
+        sx = __fadd_rn(sx, __fmul_rn(q.x, q.w));
+        sy = __fadd_rn(sy, __fmul_rn(q.y, q.w));
+        sz = __fadd_rn(sz, __fmul_rn(q.z, q.w));
+        if (a.node_ecol && a.types[pi] == 0u) {
+            const float4 c = a.colors[pi];
+            ec = make_float4(__fadd_rn(ec.x, c.x), __fadd_rn(ec.y, c.y), __fadd_rn(ec.z, c.z),
+                             __fadd_rn(ec.w, c.w));
+            en = make_float4(__fadd_rn(en.x, q.x), __fadd_rn(en.y, q.y), __fadd_rn(en.z, q.z), 0.f);
+            ++suns;
         }
-        if (m > 0.f) cm = make_float4(__fdiv_rn(sx, m), __fdiv_rn(sy, m), __fdiv_rn(sz, m), m);
-        else cm.w = m;
-        if (a.node_ecol) {
-            const float ns = fmaxf((float)suns, 1e-9f);
-            a.node_ecol[j] = ec;
-            a.node_ecen[j] = make_float4(__fdiv_rn(en.x, ns), __fdiv_rn(en.y, ns), __fdiv_rn(en.z, ns), 0.f);
-        }
-    } else if (kMode == 1) {
-        float m = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
-        for_particles(a.pos, pb, pe, [&](const float4 q) {
-            m = __fadd_rn(m, q.w);
-            sx = __fadd_rn(sx, __fmul_rn(q.w, q.x));
-            sy = __fadd_rn(sy, __fmul_rn(q.w, q.y));
-            sz = __fadd_rn(sz, __fmul_rn(q.w, q.z));
-            if (kQuad) mom.add(q, box);
-        });
-        reinterpret_cast<float4*>(a.node_sum)[j] = make_float4(sx, sy, sz, m);
-        cm = com_from_sums(sx, sy, sz, m);
-    } else {
-        // FP64 sums of m * x over the FP32 positions relative to the system
-        // origin (written by the encode from the FP64 master copy): the
-        // product of two floats is exact in FP64, so each FMA rounds once,
-        // exactly as a multiply-then-add would.
-        double m = 0, sx = 0, sy = 0, sz = 0;
-        for_particles(a.pos, pb, pe, [&](const float4 q) {
-            const double mi = (double)q.w;
-            m = __dadd_rn(m, mi);
-            sx = __fma_rn(mi, (double)q.x, sx);
-            sy = __fma_rn(mi, (double)q.y, sy);
-            sz = __fma_rn(mi, (double)q.z, sz);
-            if (kQuad) mom.add(q, box);
-        });
-        reinterpret_cast<double4*>(a.node_sum)[j] = make_double4(sx, sy, sz, m);
-        if (pe - pb == 1 && m >= 1.17549435e-38) {
-            // One particle of normal FP32 mass: the sums are m*x exactly and
-            // the reciprocal is within 2^-47 of 1/m, so the FP32 centre of
-            // mass is x itself (+0 for -0, as the sums give).
-            const float4 q = a.pos[pb];
-            cm = make_float4(__fadd_rn(q.x, 0.f), __fadd_rn(q.y, 0.f), __fadd_rn(q.z, 0.f), q.w);
-        } else {
-            cm = com_from_sums(sx, sy, sz, m);
-        }
+    }
+    if (m > 0.f) cm = make_float4(__fdiv_rn(sx, m), __fdiv_rn(sy, m), __fdiv_rn(sz, m), m);
+    else cm.w = m;
+    if (a.node_ecol) {
+        const float ns = fmaxf((float)suns, 1e-9f);
+        a.node_ecol[j] = ec;
+        a.node_ecen[j] = make_float4(__fdiv_rn(en.x, ns), __fdiv_rn(en.y, ns), __fdiv_rn(en.z, ns), 0.f);
     }
     a.node_cm[j] = cm;
     a.node_rng[j] = make_uint4(0u, 0u, pb, pe);
-    if (kMode != 0) {
-        if (kQuad) {
-            float q[5];
-            mom.quadrupole(cm, box, q);
-            a.node_q[j] = make_float4(q[0], q[1], q[2], q[3]);
-            a.node_qyz[j] = q[4];
-        }
-        if (a.want_delta) a.node_crit2[j] = node_crit2(a, node_key, 0, cm);
-        // A leaf holding more than one group is cut into group-sized chunks.
-        const uint32_t gs = a.group_size;
-        const uint32_t c = pe - pb > gs ? (pe - pb + gs - 1u) / gs : 0u;
-        const uint32_t slot = reserve_groups(a.group_count, c);
-        for (uint32_t i = 0; i < c; ++i)
-            a.groups[slot + i] = make_uint4(pb + i * gs, min(pb + (i + 1u) * gs, pe), pe, i);
-    }
 }
 
-template <int kMode>
-__device__ __forceinline__ void aggregate_leaf_node(const AggArgs& a, uint32_t j, uint32_t u0) {
-    if (kMode != 0 && a.want_quad) aggregate_leaf_node_q<kMode, true>(a, j, u0);
-    else aggregate_leaf_node_q<kMode, false>(a, j, u0);
-}
-
-// aggregateNodes (Octree.metal:120-202) for node j of layer l (one thread).
-// Children are the contiguous run of layer l-1 nodes sharing code >> 3 (at
-// most 8). Each thread first loads all its children's records together
-// (one memory latency instead of one per child), then sums them in child
-// order with the same roundings as a sequential loop.
-// kMode 0 sums child centre of mass times child mass (the reference's
-// formula); kModes 1 and 2 add the children's raw sums.
-// Children are read through L2 (ld.global.cg): the climbing kernel below
-// reads records that other blocks wrote in the same launch.
+// Children are read through L2 (ld.global.cg): the climbing kernels below
+// read records that other blocks wrote in the same launch.
 __device__ __forceinline__ float4 ld_l2(const float4* p) { return __ldcg(p); }
 __device__ __forceinline__ float ld_l2(const float* p) { return __ldcg(p); }
 __device__ __forceinline__ uint4 ld_l2(const uint4* p) { return __ldcg(p); }
@@ -600,9 +536,12 @@ __device__ __forceinline__ double4 ld_l2(const double4* p) {
     return make_double4(lo.x, lo.y, hi.x, hi.y);
 }
 
-template <int kMode>
-__device__ __forceinline__ void aggregate_internal_node(const AggArgs& a, uint32_t l, uint32_t j,
-                                                        uint32_t u) {
+// REFERENCE: aggregateNodes (Octree.metal:120-202) for node j of layer l (one
+// thread): child centre of mass times child mass, summed in child order.
+// Children are the contiguous run of layer l-1 nodes sharing code >> 3 (at
+// most 8); their records are loaded together.
+__device__ __forceinline__ void aggregate_ref_internal(const AggArgs& a, uint32_t l, uint32_t j,
+                                                       uint32_t u) {
     const uint32_t off = a.offset[l], off_below = a.offset[l - 1];
     const uint32_t node = off + j;
     const uint32_t cb = a.node_cbeg[node];
@@ -612,212 +551,432 @@ __device__ __forceinline__ void aggregate_internal_node(const AggArgs& a, uint32
     if (ce - cb > 8u) atomicOr(a.err, kErrBadLayer);
     const uint32_t nch = min(ce - cb, 8u);
     float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 ccm[8];  // children's centres of mass (modes 0 and quadrupoles)
-    const bool need_ccm = kMode == 0 || (kMode != 0 && a.want_quad);
-    if (need_ccm) {
+    float4 ccm[8];
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k)
-            ccm[k] = k < nch ? ld_l2(a.node_cm + cb + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t k = 0; k < 8; ++k)
+        ccm[k] = k < nch ? ld_l2(a.node_cm + cb + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float m = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+        if (k < nch) {
+            const float4 q = ccm[k];
+            m = __fadd_rn(m, q.w);
+            sx = __fadd_rn(sx, __fmul_rn(q.x, q.w));
+            sy = __fadd_rn(sy, __fmul_rn(q.y, q.w));
+            sz = __fadd_rn(sz, __fmul_rn(q.z, q.w));
+        }
     }
-    if (kMode == 0) {
-        float m = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
+    if (m > 0.f) cm = make_float4(__fdiv_rn(sx, m), __fdiv_rn(sy, m), __fdiv_rn(sz, m), m);
+    else cm.w = m;
+    if (a.node_ecol) {
+        // Children whose emitted colour has alpha > 0: colours summed,
+        // centres averaged over those children (Octree.metal:155-178).
+        float4 ec = make_float4(0.f, 0.f, 0.f, 0.f), en = ec;
+        uint32_t suns = 0;
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k) {
             if (k < nch) {
-                const float4 q = ccm[k];
-                m = __fadd_rn(m, q.w);
-                sx = __fadd_rn(sx, __fmul_rn(q.x, q.w));
-                sy = __fadd_rn(sy, __fmul_rn(q.y, q.w));
-                sz = __fadd_rn(sz, __fmul_rn(q.z, q.w));
-            }
-        }
-        if (m > 0.f) cm = make_float4(__fdiv_rn(sx, m), __fdiv_rn(sy, m), __fdiv_rn(sz, m), m);
-        else cm.w = m;
-        if (a.node_ecol) {
-            // Children whose emitted colour has alpha > 0: colours summed,
-            // centres averaged over those children (Octree.metal:155-178).
-            float4 ec = make_float4(0.f, 0.f, 0.f, 0.f), en = ec;
-            uint32_t suns = 0;
-#pragma unroll
-            for (uint32_t k = 0; k < 8; ++k) {
-                if (k < nch) {
-                    const float4 c = ld_l2(a.node_ecol + cb + k);
-                    if (c.w > 0.f) {
-                        const float4 e = ld_l2(a.node_ecen + cb + k);
-                        ec = make_float4(__fadd_rn(ec.x, c.x), __fadd_rn(ec.y, c.y),
-                                         __fadd_rn(ec.z, c.z), __fadd_rn(ec.w, c.w));
-                        en = make_float4(__fadd_rn(en.x, e.x), __fadd_rn(en.y, e.y),
-                                         __fadd_rn(en.z, e.z), 0.f);
-                        ++suns;
-                    }
+                const float4 c = ld_l2(a.node_ecol + cb + k);
+                if (c.w > 0.f) {
+                    const float4 e = ld_l2(a.node_ecen + cb + k);
+                    ec = make_float4(__fadd_rn(ec.x, c.x), __fadd_rn(ec.y, c.y),
+                                     __fadd_rn(ec.z, c.z), __fadd_rn(ec.w, c.w));
+                    en = make_float4(__fadd_rn(en.x, e.x), __fadd_rn(en.y, e.y),
+                                     __fadd_rn(en.z, e.z), 0.f);
+                    ++suns;
                 }
             }
-            if (suns > 0) {
-                const float ns = (float)suns;
-                en = make_float4(__fdiv_rn(en.x, ns), __fdiv_rn(en.y, ns), __fdiv_rn(en.z, ns), 0.f);
-            }
-            a.node_ecol[node] = ec;
-            a.node_ecen[node] = en;
         }
-    } else if (nch == 1) {
-        // One child (most nodes of the lower layers): every sum is the
-        // child's (0 + s is exact, and no sum is -0 since all start at +0),
-        // so the sums, the centre of mass and the moments equal the child's;
-        // copying them is what the arithmetic below would produce.
-        if (kMode == 1)
-            reinterpret_cast<float4*>(a.node_sum)[node] = ld_l2(reinterpret_cast<const float4*>(a.node_sum) + cb);
-        else
-            reinterpret_cast<double4*>(a.node_sum)[node] = ld_l2(reinterpret_cast<const double4*>(a.node_sum) + cb);
-        cm = need_ccm ? ccm[0] : ld_l2(a.node_cm + cb);
-    } else if (kMode == 1) {
-        const float4* sum = reinterpret_cast<const float4*>(a.node_sum);
-        float4 cs[8];
-#pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) cs[k] = k < nch ? ld_l2(sum + cb + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        float m = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
-#pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) {
-            if (k < nch) {
-                sx = __fadd_rn(sx, cs[k].x);
-                sy = __fadd_rn(sy, cs[k].y);
-                sz = __fadd_rn(sz, cs[k].z);
-                m = __fadd_rn(m, cs[k].w);
-            }
+        if (suns > 0) {
+            const float ns = (float)suns;
+            en = make_float4(__fdiv_rn(en.x, ns), __fdiv_rn(en.y, ns), __fdiv_rn(en.z, ns), 0.f);
         }
-        reinterpret_cast<float4*>(a.node_sum)[node] = make_float4(sx, sy, sz, m);
-        cm = com_from_sums(sx, sy, sz, m);
-    } else {
-        const double4* sum = reinterpret_cast<const double4*>(a.node_sum);
-        double4 cs[8];
-#pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) cs[k] = k < nch ? ld_l2(sum + cb + k) : make_double4(0.0, 0.0, 0.0, 0.0);
-        double m = 0, sx = 0, sy = 0, sz = 0;
-#pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) {
-            if (k < nch) {
-                sx = __dadd_rn(sx, cs[k].x);
-                sy = __dadd_rn(sy, cs[k].y);
-                sz = __dadd_rn(sz, cs[k].z);
-                m = __dadd_rn(m, cs[k].w);
-            }
-        }
-        reinterpret_cast<double4*>(a.node_sum)[node] = make_double4(sx, sy, sz, m);
-        cm = com_from_sums(sx, sy, sz, m);
+        a.node_ecol[node] = ec;
+        a.node_ecen[node] = en;
     }
     a.node_cm[node] = cm;
     a.node_rng[node] = make_uint4(cb, ce, pb, pe);
-    if (kMode != 0) {
-        if (a.want_quad && nch == 1) {
-            a.node_q[node] = ld_l2(a.node_q + cb);
-            a.node_qyz[node] = ld_l2(a.node_qyz + cb);
-        } else if (a.want_quad) {
-            float4 qc[8];
-            float qyz[8];
+}
+
+// ---- PHYSICAL ----
+
+// A node's record as the climbing thread holds it: raw sums (FP32 in the
+// plain form, FP64 in the precision form), centre of mass and mass,
+// quadrupole, particles and key.
+template <bool kPrec>
+struct NodeRec {
+    using Sum = typename std::conditional<kPrec, double4, float4>::type;
+    Sum sum;
+    float4 cm;
+    float q[5];
+    uint32_t pb, pe;
+    uint64_t key;
+};
+
+// Writes node's record but for its sums.
+template <bool kPrec, bool kQuad>
+__device__ __forceinline__ void store_node(const AggArgs& a, uint32_t node, uint32_t l, uint32_t cb,
+                                           uint32_t ce, const NodeRec<kPrec>& r) {
+    a.node_cm[node] = r.cm;
+    a.node_rng[node] = make_uint4(cb, ce, r.pb, r.pe);
+    if (kQuad) {
+        a.node_q[node] = make_float4(r.q[0], r.q[1], r.q[2], r.q[3]);
+        a.node_qyz[node] = r.q[4];
+    }
+    if (a.want_delta) a.node_crit2[node] = node_crit2(a, r.key, l, r.cm);
+}
+
+// aggregateLeafNodes (Octree.metal:53-117), state already in sorted order.
+// Plain: raw FP32 sums of m and m*x. Precision: FP64 sums over the FP32
+// positions relative to the system origin. The quadrupole comes from the same
+// read: moments about the cell's centre, shifted to the centre of mass after.
+template <bool kPrec, bool kQuad>
+__device__ __forceinline__ NodeRec<kPrec> aggregate_leaf(const AggArgs& a, uint32_t j, uint32_t u0) {
+    NodeRec<kPrec> r;
+    r.pb = a.pbeg[j];
+    r.pe = (j + 1 < u0) ? a.pbeg[j + 1] : a.n;
+    r.key = a.node_key[j];
+    const float4 box = kQuad ? cell_box(a, r.key, 0) : make_float4(0.f, 0.f, 0.f, 0.f);
+    CellMoments mom;
+    if constexpr (!kPrec) {
+        float m = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
+        for_particles(a.pos, r.pb, r.pe, [&](const float4 q) {
+            m = __fadd_rn(m, q.w);
+            sx = __fadd_rn(sx, __fmul_rn(q.w, q.x));
+            sy = __fadd_rn(sy, __fmul_rn(q.w, q.y));
+            sz = __fadd_rn(sz, __fmul_rn(q.w, q.z));
+            if (kQuad) mom.add(q, box);
+        });
+        r.sum = make_float4(sx, sy, sz, m);
+        r.cm = com_from_sums(sx, sy, sz, m);
+    } else {
+        // The product of two floats is exact in FP64, so each FMA rounds
+        // once, exactly as a multiply-then-add would.
+        double m = 0, sx = 0, sy = 0, sz = 0;
+        for_particles(a.pos, r.pb, r.pe, [&](const float4 q) {
+            const double mi = (double)q.w;
+            m = __dadd_rn(m, mi);
+            sx = __fma_rn(mi, (double)q.x, sx);
+            sy = __fma_rn(mi, (double)q.y, sy);
+            sz = __fma_rn(mi, (double)q.z, sz);
+            if (kQuad) mom.add(q, box);
+        });
+        r.sum = make_double4(sx, sy, sz, m);
+        if (r.pe - r.pb == 1 && m >= 1.17549435e-38) {
+            // One particle of normal FP32 mass: the sums are m*x exactly and
+            // the reciprocal is within 2^-47 of 1/m, so the FP32 centre of
+            // mass is x itself (+0 for -0, as the sums give).
+            const float4 q = a.pos[r.pb];
+            r.cm = make_float4(__fadd_rn(q.x, 0.f), __fadd_rn(q.y, 0.f), __fadd_rn(q.z, 0.f), q.w);
+        } else {
+            r.cm = com_from_sums(sx, sy, sz, m);
+        }
+    }
+    if (kQuad) mom.quadrupole(r.cm, box, r.q);
+    store_node<kPrec, kQuad>(a, j, 0, 0u, 0u, r);
+    // A leaf holding more than one group is cut into group-sized chunks.
+    const uint32_t gs = a.group_size;
+    const uint32_t c = r.pe - r.pb > gs ? (r.pe - r.pb + gs - 1u) / gs : 0u;
+    const uint32_t slot = reserve_groups(a.group_count, c);
+    for (uint32_t i = 0; i < c; ++i)
+        a.groups[slot + i] = make_uint4(r.pb + i * gs, min(r.pb + (i + 1u) * gs, r.pe), r.pe, i);
+    return r;
+}
+
+// aggregateNodes (Octree.metal:120-202) for a node with several children (at
+// most 8): their records loaded together, sums and quadrupoles added in child
+// order with the roundings of a sequential loop.
+template <bool kPrec, bool kQuad>
+__device__ __forceinline__ void aggregate_internal(const AggArgs& a, uint32_t l, uint32_t node,
+                                                   uint32_t cb, uint32_t ce, NodeRec<kPrec>& r) {
+    using Sum = typename NodeRec<kPrec>::Sum;
+    if (ce - cb > 8u) atomicOr(a.err, kErrBadLayer);
+    const uint32_t nch = min(ce - cb, 8u);
+    const Sum* sum = reinterpret_cast<const Sum*>(a.node_sum);
+    {
+        Sum cs[8];
 #pragma unroll
-            for (uint32_t k = 0; k < 8; ++k) {
-                qc[k] = k < nch ? ld_l2(a.node_q + cb + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-                qyz[k] = k < nch ? ld_l2(a.node_qyz + cb + k) : 0.f;
-            }
-            float q[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+        for (uint32_t k = 0; k < 8; ++k) cs[k] = k < nch ? ld_l2(sum + cb + k) : Sum{};
+        Sum t{};
 #pragma unroll
-            for (uint32_t k = 0; k < 8; ++k) {
-                if (k < nch) {
-                    const float4 cc = ccm[k];
-                    quad_add(q, cc.w, __fsub_rn(cc.x, cm.x), __fsub_rn(cc.y, cm.y), __fsub_rn(cc.z, cm.z));
-                    q[0] = __fadd_rn(q[0], qc[k].x);
-                    q[1] = __fadd_rn(q[1], qc[k].y);
-                    q[2] = __fadd_rn(q[2], qc[k].z);
-                    q[3] = __fadd_rn(q[3], qc[k].w);
-                    q[4] = __fadd_rn(q[4], qyz[k]);
+        for (uint32_t k = 0; k < 8; ++k) {
+            if (k < nch) {
+                if constexpr (kPrec) {
+                    t.x = __dadd_rn(t.x, cs[k].x);
+                    t.y = __dadd_rn(t.y, cs[k].y);
+                    t.z = __dadd_rn(t.z, cs[k].z);
+                    t.w = __dadd_rn(t.w, cs[k].w);
+                } else {
+                    t.x = __fadd_rn(t.x, cs[k].x);
+                    t.y = __fadd_rn(t.y, cs[k].y);
+                    t.z = __fadd_rn(t.z, cs[k].z);
+                    t.w = __fadd_rn(t.w, cs[k].w);
                 }
             }
-            a.node_q[node] = make_float4(q[0], q[1], q[2], q[3]);
-            a.node_qyz[node] = q[4];
         }
-        if (a.want_delta) a.node_crit2[node] = node_crit2(a, a.node_key[node], l, cm);
-        // Groups: a node over the group size packs runs of consecutive
-        // small children (greedy, in child order); a small top-layer node is
-        // a group by itself.
-        const uint32_t gs = a.group_size;
+        r.sum = t;
+        r.cm = com_from_sums(t.x, t.y, t.z, t.w);
+    }
+    if constexpr (kQuad) {
+        float4 ccm[8], qc[8];
+        float qyz[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            ccm[k] = k < nch ? ld_l2(a.node_cm + cb + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            qc[k] = k < nch ? ld_l2(a.node_q + cb + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            qyz[k] = k < nch ? ld_l2(a.node_qyz + cb + k) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 5; ++i) r.q[i] = 0.f;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            if (k < nch) {
+                const float4 cc = ccm[k];
+                quad_add(r.q, cc.w, __fsub_rn(cc.x, r.cm.x), __fsub_rn(cc.y, r.cm.y),
+                         __fsub_rn(cc.z, r.cm.z));
+                r.q[0] = __fadd_rn(r.q[0], qc[k].x);
+                r.q[1] = __fadd_rn(r.q[1], qc[k].y);
+                r.q[2] = __fadd_rn(r.q[2], qc[k].z);
+                r.q[3] = __fadd_rn(r.q[3], qc[k].w);
+                r.q[4] = __fadd_rn(r.q[4], qyz[k]);
+            }
+        }
+    }
+    // Groups: a node over the group size packs runs of consecutive small
+    // children (greedy, in child order). The packing runs twice: to count the
+    // groups, then to write them into the slots reserved for this node.
+    const uint32_t gs = a.group_size;
+    if (r.pe - r.pb > gs) {
         uint2 cr[8];
-        const bool split = pe - pb > gs;
-        if (split) {
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            const uint4 rng = k < nch ? ld_l2(a.node_rng + cb + k) : make_uint4(0u, 0u, 0u, 0u);
+            cr[k] = make_uint2(rng.z, rng.w);
+        }
+        auto pack = [&](auto&& emit) {
+            uint32_t gb = 0, ge = 0;
 #pragma unroll
             for (uint32_t k = 0; k < 8; ++k) {
-                const uint4 rng = k < nch ? ld_l2(a.node_rng + cb + k) : make_uint4(0u, 0u, 0u, 0u);
-                cr[k] = make_uint2(rng.z, rng.w);
-            }
-        }
-        // The packing runs twice: to count the groups, then to write them
-        // into the slots reserved for this node.
-        auto pack = [&](auto&& emit) {
-            if (split) {
-                uint32_t gb = 0, ge = 0;
-#pragma unroll
-                for (uint32_t k = 0; k < 8; ++k) {
-                    if (k >= nch) break;
-                    const uint32_t cc = cr[k].y - cr[k].x;
-                    if (cc <= gs) {
-                        if (ge == gb) {
-                            gb = cr[k].x;
-                            ge = cr[k].y;
-                        } else if ((ge - gb) + cc <= gs) {
-                            ge = cr[k].y;
-                        } else {
-                            emit(gb, ge);
-                            gb = cr[k].x;
-                            ge = cr[k].y;
-                        }
-                    } else if (ge != gb) {
+                if (k >= nch) break;
+                const uint32_t cc = cr[k].y - cr[k].x;
+                if (cc <= gs) {
+                    if (ge == gb) {
+                        gb = cr[k].x;
+                        ge = cr[k].y;
+                    } else if ((ge - gb) + cc <= gs) {
+                        ge = cr[k].y;
+                    } else {
                         emit(gb, ge);
-                        gb = ge = 0;
+                        gb = cr[k].x;
+                        ge = cr[k].y;
                     }
+                } else if (ge != gb) {
+                    emit(gb, ge);
+                    gb = ge = 0;
                 }
-                if (ge != gb) emit(gb, ge);
-            } else if (l == a.lbits) {
-                emit(pb, pe);
             }
+            if (ge != gb) emit(gb, ge);
         };
         uint32_t c = 0;
         pack([&](uint32_t, uint32_t) { ++c; });
         uint32_t slot = reserve_groups(a.group_count, c);
         pack([&](uint32_t b, uint32_t e) { a.groups[slot++] = make_uint4(b, e, e, 0u); });
     }
+    store_node<kPrec, kQuad>(a, node, l, cb, ce, r);
 }
 
-// Bottom-up aggregation. Layers of at least kClimbMinNodes nodes (capacity)
-// run one launch each, a thread per node with coalesced records; the rest
-// of the tree runs in one launch that climbs: a thread per node of the
-// first small layer aggregates its node, then makes the records visible
-// (fence) and counts itself in at the parent; the thread that brings the
-// parent's count to its number of children aggregates the parent (reading
-// the children through L2) and climbs on; the others stop. Every node is
-// aggregated once, after all its children, with the arithmetic of the
-// per-node functions above; no thread waits on another. The small top
-// layers thus cost one launch instead of one each.
+// The bottom-up aggregation. Layers of at least kClimbMinNodes nodes (capacity)
+// run one launch each, a thread per node with coalesced records; the rest of
+// the tree runs in one climbing launch.
+//
+// A parent with one child takes the child's sums, centre of mass and
+// quadrupole as they are (each sum is 0 + the child's, and no sum is -0), so
+// the thread that made the child writes the parent from its registers, and so
+// on up the single-child chain; a layer's own launch only takes the nodes with
+// several children: from a work list in layers of at least kWorkMinNodes nodes
+// (capacity), by looking at every node in smaller ones, where the list's
+// atomics and indirection cost more than the idle threads.
+//
+// What bounds it: the record stores (56 bytes a node of a chain), in the
+// precision form the FP64 pipe (64 cycles an instruction and warp), and in
+// small trees the launches and load latencies. Aggregation before and after
+// (one launch a layer, each re-reading its children): 6,000,007-body cube at 21
+// bits 4.55 -> 1.83 ms, two Plummer spheres of 4,194,304 in the precision form
+// 481 -> 356 us, 256 systems 590 -> 422 us, 524,288-body disk 146 -> 120 us.
+// Work lists in every layer: disk 134 us; in none: merger 420 us, 21 bits
+// 2.56 ms; the whole tree in one climbing launch: merger 594 us, disk 124 us.
 constexpr uint32_t kClimbMinNodes = 32768;
-template <int kMode>
-__global__ __launch_bounds__(128) void aggregate_leaf_kernel(AggArgs a) {
+constexpr uint32_t kWorkMinNodes = 1u << 20;
+
+// The children [cb, ce) of node jp of layer l (u nodes there, `below` nodes
+// one layer down).
+struct Children {
+    uint32_t cb, ce;
+};
+__device__ __forceinline__ Children children_of(const AggArgs& a, uint32_t p, uint32_t jp, uint32_t u,
+                                                uint32_t l, uint32_t below) {
+    return {a.node_cbeg[p], (jp + 1 < u) ? a.node_cbeg[p + 1] : a.offset[l - 1] + below};
+}
+
+// Writes the single-child chain above node (of layer l) in the layers below
+// `top`, then the sums of the chain's last node, which its parent adds. A
+// parent with several children in a layer below `work_top` goes to its layer's
+// work list, once: by the thread that ends the chain of its first child.
+template <bool kPrec, bool kQuad>
+__device__ __forceinline__ void climb_chain(const AggArgs& a, uint32_t l, uint32_t node, uint32_t top,
+                                            uint32_t work_top, NodeRec<kPrec>& r) {
+    uint32_t work = kNoParent, k = l + 1;
+    for (; k < top; ++k) {
+        const uint32_t p = a.parent[node];
+        const uint32_t u = a.layer_count[k], jp = p - a.offset[k];
+        if (jp >= u) {
+            atomicOr(a.err, kErrBadLayer);
+            return;
+        }
+        const Children c = children_of(a, p, jp, u, k, a.layer_count[k - 1]);
+        if (c.ce - c.cb != 1u) {
+            if (c.cb == node && k < work_top) work = p;
+            break;
+        }
+        r.key >>= 3;
+        store_node<kPrec, kQuad>(a, p, k, c.cb, c.ce, r);
+        node = p;
+    }
+    reinterpret_cast<typename NodeRec<kPrec>::Sum*>(a.node_sum)[node] = r.sum;
+    // One atomic per layer and warp for the slots of the list.
+    const uint32_t mask = __activemask();
+    const uint32_t peers = __match_any_sync(mask, work != kNoParent ? k : 0xFFFFu);
+    if (work == kNoParent) return;
+    const uint32_t lane = threadIdx.x & 31u, leader = (uint32_t)__ffs(peers) - 1u;
+    uint32_t slot = 0;
+    if (lane == leader) slot = atomicAdd(&a.work_count[k], (uint32_t)__popc(peers));
+    slot = __shfl_sync(peers, slot, leader) + __popc(peers & lanemask_lt());
+    a.work[a.offset[k] + slot] = work;
+}
+
+template <bool kPrec, bool kQuad>
+__global__ __launch_bounds__(128) void aggregate_leaf_kernel(AggArgs a, uint32_t top, uint32_t work_top) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t u0 = a.layer_count[0];
-    if (j < u0) aggregate_leaf_node<kMode>(a, j, u0);
+    if (j >= u0) return;
+    NodeRec<kPrec> r = aggregate_leaf<kPrec, kQuad>(a, j, u0);
+    climb_chain<kPrec, kQuad>(a, 0, j, top, work_top, r);
 }
 
-template <int kMode>
-__global__ __launch_bounds__(128) void aggregate_internal_kernel(AggArgs a, uint32_t l) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t u = a.layer_count[l];
-    if (j < u) aggregate_internal_node<kMode>(a, l, j, u);
+// The nodes of layer l with several children: the layer's work list (kWork;
+// the blocks stride over it), or all nodes, the others left out.
+template <bool kPrec, bool kQuad, bool kWork>
+__global__ __launch_bounds__(128) void aggregate_internal_kernel(AggArgs a, uint32_t l, uint32_t top,
+                                                                 uint32_t work_top) {
+    const uint32_t u = a.layer_count[l], count = kWork ? a.work_count[l] : u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const uint32_t node = kWork ? a.work[a.offset[l] + i] : a.offset[l] + i, j = node - a.offset[l];
+        const Children c = children_of(a, node, j, u, l, a.layer_count[l - 1]);
+        if (!kWork && c.ce - c.cb == 1u) continue;
+        NodeRec<kPrec> r;
+        r.pb = a.pbeg[node];
+        r.pe = (j + 1 < u) ? a.pbeg[node + 1] : a.n;
+        r.key = a.node_key[node];
+        aggregate_internal<kPrec, kQuad>(a, l, node, c.cb, c.ce, r);
+        climb_chain<kPrec, kQuad>(a, l, node, top, work_top, r);
+    }
 }
 
-// Layers l0 and up in one launch: one thread per node of layer l0.
-template <int kMode>
-__global__ __launch_bounds__(128) void aggregate_tree_kernel(AggArgs a, uint32_t l0) {
+// Layers l0 and up in one launch: a thread per node of layer l0 makes its
+// record and climbs. At a parent with several children it stores its node's
+// sums, makes its records visible (fence) and counts itself in; the thread
+// that completes the count aggregates the parent (reading the children
+// through L2), sets the count back to zero for the next build and climbs on;
+// the others stop. Every node is aggregated once, after all its children; no
+// thread waits on another. A small tree takes a chain of fences and dependent
+// loads up its layers; the parent's own links are loaded before the fence.
+template <bool kPrec, bool kQuad>
+__global__ __launch_bounds__(128) void aggregate_climb_kernel(AggArgs a, uint32_t l0) {
+    using Sum = typename NodeRec<kPrec>::Sum;
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t u0 = a.layer_count[l0];
     if (j >= u0) return;
-    if (l0 == 0) aggregate_leaf_node<kMode>(a, j, u0);
-    else aggregate_internal_node<kMode>(a, l0, j, u0);
+    uint32_t node = a.offset[l0] + j;
+    uint32_t p = a.parent[node];
+    NodeRec<kPrec> r;
+    if (l0 == 0) {
+        r = aggregate_leaf<kPrec, kQuad>(a, j, u0);
+    } else {
+        const Children c = children_of(a, node, j, u0, l0, a.layer_count[l0 - 1]);
+        r.pb = a.pbeg[node];
+        r.pe = (j + 1 < u0) ? a.pbeg[node + 1] : a.n;
+        r.key = a.node_key[node];
+        if (c.ce - c.cb == 1u) {
+            r.sum = ld_l2(reinterpret_cast<const Sum*>(a.node_sum) + c.cb);
+            r.cm = ld_l2(a.node_cm + c.cb);
+            if (kQuad) {
+                const float4 q = ld_l2(a.node_q + c.cb);
+                r.q[0] = q.x, r.q[1] = q.y, r.q[2] = q.z, r.q[3] = q.w;
+                r.q[4] = ld_l2(a.node_qyz + c.cb);
+            }
+            store_node<kPrec, kQuad>(a, node, l0, c.cb, c.ce, r);
+        } else {
+            aggregate_internal<kPrec, kQuad>(a, l0, node, c.cb, c.ce, r);
+        }
+    }
+    uint32_t below = u0;
+    for (uint32_t l = l0 + 1; l <= a.lbits; ++l) {
+        if (p == kNoParent) return;
+        const uint32_t u = a.layer_count[l];
+        const uint32_t jp = p - a.offset[l];
+        if (jp >= u) {
+            atomicOr(a.err, kErrBadLayer);
+            return;
+        }
+        const Children c = children_of(a, p, jp, u, l, below);
+        const uint32_t above = a.parent[p];
+        r.key >>= 3;
+        if (c.ce - c.cb > 1u) {
+            const uint32_t pb = a.pbeg[p], pe = (jp + 1 < u) ? a.pbeg[p + 1] : a.n;
+            reinterpret_cast<Sum*>(a.node_sum)[node] = r.sum;
+            __threadfence();
+            if (atomicAdd(&a.arrive[p], 1u) != c.ce - c.cb - 1u) return;
+            __threadfence();
+            a.arrive[p] = 0u;
+            r.pb = pb;
+            r.pe = pe;
+            aggregate_internal<kPrec, kQuad>(a, l, p, c.cb, c.ce, r);
+        } else {
+            store_node<kPrec, kQuad>(a, p, l, c.cb, c.ce, r);
+        }
+        node = p;
+        p = above;
+        below = u;
+    }
+    // The root of a system no larger than a group is a group by itself.
+    if (r.pe - r.pb <= a.group_size) {
+        const uint32_t slot = reserve_groups(a.group_count, 1u);
+        a.groups[slot] = make_uint4(r.pb, r.pe, r.pe, 0u);
+    }
+}
+
+// ---- REFERENCE ----
+
+// One launch per large layer, the rest of the tree climbing, as above.
+__global__ __launch_bounds__(128) void aggregate_ref_leaf_kernel(AggArgs a) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t u0 = a.layer_count[0];
+    if (j < u0) aggregate_ref_leaf(a, j, u0);
+}
+
+__global__ __launch_bounds__(128) void aggregate_ref_internal_kernel(AggArgs a, uint32_t l) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t u = a.layer_count[l];
+    if (j < u) aggregate_ref_internal(a, l, j, u);
+}
+
+// Layers l0 and up in one launch: one thread per node of layer l0.
+__global__ __launch_bounds__(128) void aggregate_ref_tree_kernel(AggArgs a, uint32_t l0) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t u0 = a.layer_count[l0];
+    if (j >= u0) return;
+    if (l0 == 0) aggregate_ref_leaf(a, j, u0);
+    else aggregate_ref_internal(a, l0, j, u0);
     uint32_t node = a.offset[l0] + j;
     for (uint32_t l = l0 + 1; l <= a.lbits; ++l) {
         const uint32_t p = a.parent[node];
@@ -834,8 +993,9 @@ __global__ __launch_bounds__(128) void aggregate_tree_kernel(AggArgs a, uint32_t
             __threadfence();
             if (atomicAdd(&a.arrive[p], 1u) != ce - cb - 1u) return;
             __threadfence();
+            a.arrive[p] = 0u;
         }
-        aggregate_internal_node<kMode>(a, l, jp, u);
+        aggregate_ref_internal(a, l, jp, u);
         node = p;
     }
 }
@@ -1220,31 +1380,44 @@ cudaError_t launch_topology(const TopoArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+namespace {
 uint32_t climb_first_layer(const LayerTable& t) {
     uint32_t l0 = 0;
     while (l0 + 1 < t.n_layers && t.size[l0] >= kClimbMinNodes) ++l0;
     return l0;
 }
 
+constexpr uint32_t kWorkBlocks = 152 * 16;  // several waves at any register count
+
+template <bool kPrec, bool kQuad>
+cudaError_t launch_physical(const AggArgs& a, const LayerTable& t, cudaStream_t st) {
+    const uint32_t t0 = 128, l0 = climb_first_layer(t);
+    uint32_t lw = 0;  // layers below lw have work lists (sizes fall with the layer)
+    while (lw < l0 && t.size[lw] >= kWorkMinNodes) ++lw;
+    for (uint32_t l = 0; l < l0; ++l) {
+        const uint32_t g = blocks_for(t.size[l], t0);
+        if (l == 0) aggregate_leaf_kernel<kPrec, kQuad><<<g, t0, 0, st>>>(a, l0, lw);
+        else if (l < lw)
+            aggregate_internal_kernel<kPrec, kQuad, true><<<std::min(g, kWorkBlocks), t0, 0, st>>>(a, l, l0, lw);
+        else
+            aggregate_internal_kernel<kPrec, kQuad, false><<<g, t0, 0, st>>>(a, l, l0, lw);
+    }
+    aggregate_climb_kernel<kPrec, kQuad><<<blocks_for(t.size[l0], t0), t0, 0, st>>>(a, l0);
+    return cudaGetLastError();
+}
+}  // namespace
+
 cudaError_t launch_aggregate(int mode, const AggArgs& a, const LayerTable& t, cudaStream_t st) {
     const uint32_t t0 = 128;
+    if (mode == 1) return a.want_quad ? launch_physical<false, true>(a, t, st) : launch_physical<false, false>(a, t, st);
+    if (mode == 2) return a.want_quad ? launch_physical<true, true>(a, t, st) : launch_physical<true, false>(a, t, st);
     const uint32_t l0 = climb_first_layer(t);
     for (uint32_t l = 0; l < l0; ++l) {
         const uint32_t g = blocks_for(t.size[l], t0);
-        if (l == 0) {
-            if (mode == 0) aggregate_leaf_kernel<0><<<g, t0, 0, st>>>(a);
-            else if (mode == 1) aggregate_leaf_kernel<1><<<g, t0, 0, st>>>(a);
-            else aggregate_leaf_kernel<2><<<g, t0, 0, st>>>(a);
-        } else {
-            if (mode == 0) aggregate_internal_kernel<0><<<g, t0, 0, st>>>(a, l);
-            else if (mode == 1) aggregate_internal_kernel<1><<<g, t0, 0, st>>>(a, l);
-            else aggregate_internal_kernel<2><<<g, t0, 0, st>>>(a, l);
-        }
+        if (l == 0) aggregate_ref_leaf_kernel<<<g, t0, 0, st>>>(a);
+        else aggregate_ref_internal_kernel<<<g, t0, 0, st>>>(a, l);
     }
-    const uint32_t g = blocks_for(t.size[l0], t0);
-    if (mode == 0) aggregate_tree_kernel<0><<<g, t0, 0, st>>>(a, l0);
-    else if (mode == 1) aggregate_tree_kernel<1><<<g, t0, 0, st>>>(a, l0);
-    else aggregate_tree_kernel<2><<<g, t0, 0, st>>>(a, l0);
+    aggregate_ref_tree_kernel<<<blocks_for(t.size[l0], t0), t0, 0, st>>>(a, l0);
     return cudaGetLastError();
 }
 

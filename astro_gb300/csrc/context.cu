@@ -239,6 +239,9 @@ int check_device(astro_ctx* ctx) {
     }
     if (err) {
         CK(cudaMemset(ctx->err, 0, sizeof(uint32_t)));
+        // A build that went wrong may have left arrival counts behind.
+        if (ctx->node_arrive)
+            CK(cudaMemsetAsync(ctx->node_arrive, 0, ctx->tree_capacity * sizeof(uint32_t), ctx->stream));
         if (err & astro::kErrLookbackTimeout)
             return fail(ctx, ASTRO_ERR_DEVICE_TIMEOUT, "a decoupled look-back wait gave up");
         if (err & astro::kErrFrontier)
@@ -386,6 +389,8 @@ int stage_build(astro_ctx* ctx) {
     a.node_qyz = ctx->node_qyz;
     a.groups = ctx->groups;
     a.group_count = ctx->counters + 2;
+    a.work = ctx->node_arrive;
+    a.work_count = ctx->counters + 16;
     if (!is_phys(ctx)) {
         a.colors = ctx->colors;
         a.types = ctx->types;
@@ -401,13 +406,7 @@ int stage_build(astro_ctx* ctx) {
     a.group_size = ctx->p.group_size ? ctx->p.group_size : astro::kDefaultGroupSize;
     a.err = ctx->err;
     CK(cudaMemsetAsync(ctx->counters + 2, 0, sizeof(uint32_t), st));
-    const uint32_t l0 = astro::climb_first_layer(ctx->layers);
-    if (l0 < ctx->lbits) {
-        // Arrival counters of the layers the aggregation climbs into.
-        const uint64_t first = ctx->layers.offset[l0 + 1];
-        const uint64_t end = (uint64_t)ctx->layers.offset[ctx->lbits] + ctx->layers.size[ctx->lbits];
-        CK(cudaMemsetAsync(ctx->node_arrive + first, 0, (end - first) * sizeof(uint32_t), st));
-    }
+    CK(cudaMemsetAsync(ctx->counters + 16, 0, ASTRO_MAX_LAYERS * sizeof(uint32_t), st));
     const int mode = !is_phys(ctx) ? 0 : (is_prec(ctx) ? 2 : 1);
     CK(astro::launch_aggregate(mode, a, ctx->layers, st));
     ctx->tree_valid = true;
@@ -726,7 +725,7 @@ int astro_create(const astro_params* params, uint32_t max_n, uint32_t max_system
     CKC(cudaMalloc(&ctx->sort_temp, ctx->sort_temp_bytes));
     ctx->topo_lookback_words = (size_t)astro::topology_tiles(max_n) * 32 + 32;
     CKC(dev_alloc(&ctx->topo_lookback, ctx->topo_lookback_words));
-    CKC(dev_alloc(&ctx->counters, 16));
+    CKC(dev_alloc(&ctx->counters, 64));
     CKC(dev_alloc(&ctx->groups, max_n));
     CKC(dev_alloc(&ctx->err, 1));
     CKC(dev_alloc(&ctx->stats, kNumStats));
@@ -887,6 +886,9 @@ static int upload_common(astro_ctx* ctx, const PositionMass* pm, const VelocityR
     layer_table(sizes, ctx->lbits, &ctx->layers, &ctx->capacity);
     int r = ensure_tree(ctx, ctx->capacity);
     if (r != ASTRO_OK) return r;
+    // Arrival counts are zero between builds, but the large layers' part holds
+    // work lists, and the layers have moved.
+    CK(cudaMemsetAsync(ctx->node_arrive, 0, ctx->tree_capacity * sizeof(uint32_t), st));
     if ((r = ensure_frontier(ctx)) != ASTRO_OK) return r;
     if (prec && (r = ensure_x64(ctx)) != ASTRO_OK) return r;
     // Systems and chunks.
