@@ -256,7 +256,15 @@ struct TraverseConfig {
     int warps;        // warps per block (2, 4 or 8)
     bool quad;        // quadrupole terms (group walk template switch)
 };
-cudaError_t launch_traverse_ref(const TraverseArgs& a, cudaStream_t st);
+// REFERENCE: the tree's layers (first node of each, live nodes on the device)
+// and its capacity in nodes.
+struct RefTree {
+    const uint32_t* layer_count;
+    uint32_t offset[ASTRO_MAX_LAYERS];
+    uint32_t capacity;
+};
+cudaError_t traverse_init();
+cudaError_t launch_traverse_ref(const TraverseArgs& a, const RefTree& t, cudaStream_t st);
 cudaError_t launch_traverse_phys(const TraverseArgs& a, const TraverseConfig& c, cudaStream_t st);
 // Group walk: warps of the persistent walk launch (each owns two frontier
 // buffers of frontier_cap words), the list pool size in blocks for n

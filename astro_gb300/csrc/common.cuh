@@ -76,6 +76,18 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
+// Minimum and maximum over the warp (NaNs lose, as with fminf / fmaxf).
+__device__ __forceinline__ float warp_min_f32(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max_f32(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // Device-side error word bits, read back by the host after a stream sync.
 enum DeviceError : uint32_t {
     kErrLookbackTimeout = 1u << 0,  // a decoupled look-back wait gave up

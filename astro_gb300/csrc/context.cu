@@ -487,7 +487,11 @@ int stage_traverse(astro_ctx* ctx, float dt, bool integrate) {
             return ASTRO_OK;
         }
         if (!ctx->tree_valid) return fail(ctx, ASTRO_ERR_STATE, "traverse called before build");
-        CK(astro::launch_traverse_ref(traverse_args(ctx, 0.0f, false), st));
+        astro::RefTree t{};
+        t.layer_count = ctx->layer_count;
+        for (uint32_t l = 0; l <= ctx->lbits; ++l) t.offset[l] = ctx->layers.offset[l];
+        t.capacity = (uint32_t)std::min<uint64_t>(ctx->capacity, 0xFFFFFFFFull);
+        CK(astro::launch_traverse_ref(traverse_args(ctx, 0.0f, false), t, st));
         return ASTRO_OK;
     }
     if (!ctx->state_in_b || !ctx->tree_valid)
@@ -704,6 +708,7 @@ int astro_create(const astro_params* params, uint32_t max_n, uint32_t max_system
     } while (0)
     CKC(cudaGetDevice(&ctx->device));
     CKC(astro::sort_init());
+    CKC(astro::traverse_init());
     CKC(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     for (int b = 0; b < 2; ++b) {
         CKC(dev_alloc(&ctx->pos[b], max_n));

@@ -144,18 +144,6 @@ __device__ __forceinline__ uint32_t shl_clamped(uint32_t v, uint32_t n) {
     return r;
 }
 
-// Minimum and maximum over the warp (NaNs lose, as with fminf / fmaxf).
-__device__ __forceinline__ float warp_min_f32(float v) {
-    float r;
-    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
-__device__ __forceinline__ float warp_max_f32(float v) {
-    float r;
-    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
-
 }  // namespace
 
 // ------------------------------------------------------------------ walk --
