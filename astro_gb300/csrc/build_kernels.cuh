@@ -235,7 +235,8 @@ struct SplatArgs {
     float clear_depth;
     float4* prim;            // per particle: window x, y, depth, size / radius (pixels)
     uint32_t* kind;          // 0 culled, 1 disc, 2 point
-    uint64_t* keys;          // fragments (pixel << 32 | particle)
+    uint64_t* keys;          // fragments (pixel << id_bits | particle)
+    uint32_t id_bits;        // bits that a particle's index needs
     uint32_t cap;
     uint32_t* cursor;
     float4* image;           // width * height, row 0 = top

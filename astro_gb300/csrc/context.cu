@@ -1389,6 +1389,7 @@ int astro_splat(astro_ctx* ctx, const astro_camera* camera, uint32_t width, uint
     a.prim = ctx->splat_prim;
     a.kind = ctx->splat_kind;
     a.cursor = ctx->splat_kind + ctx->max_n;
+    a.id_bits = std::max(1u, bits_for(ctx->n));
     a.image = ctx->splat_image;
     a.depth = ctx->splat_depth;
     CK(astro::launch_splat_project(a, st));
@@ -1422,7 +1423,7 @@ int astro_splat(astro_ctx* ctx, const astro_camera* camera, uint32_t width, uint
     uint32_t pixel_bits = 0;
     while ((1ull << pixel_bits) < pixels) ++pixel_bits;
     CK(astro::sort_pairs(ctx->frag_keys, nullptr, ctx->frag_sorted, ctx->frag_vals, count, nullptr,
-                         32u + pixel_bits, ctx->frag_temp, ctx->frag_temp_bytes, st, ctx->err));
+                         a.id_bits + pixel_bits, ctx->frag_temp, ctx->frag_temp_bytes, st, ctx->err));
     CK(astro::launch_splat_clear(a, st));
     CK(astro::launch_splat_fold(a, ctx->frag_sorted, count, st));
     CK(cudaMemcpyAsync(rgba, ctx->splat_image, 16ull * pixels, cudaMemcpyDeviceToHost, st));

@@ -8,7 +8,7 @@
 // scaled by the radius: world radius radius/2); here each is a disc of that
 // projected radius at its centre's depth, drawn opaque. Dust (type 2) is a
 // point sprite of `radius` pixels, blended with source alpha. Fragments are
-// keyed (pixel, particle), sorted with the library's radix sort, and every
+// keyed (pixel, particle) in as few bits as both need, sorted with the library's radix sort, and every
 // pixel folds its fragments in particle order — the reference's draw order
 // (stars, planets, dust by instance) — with the depth test "less", depth
 // writes on, and the colour rounded to half precision after every write (the
@@ -91,28 +91,80 @@ __device__ __forceinline__ bool covers(uint32_t kind, float4 q, int px, int py) 
     return __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) < __fmul_rn(q.w, q.w);
 }
 
-// One warp per primitive: its lanes stride over the covered box and append
-// (pixel << 32 | particle) keys; writes past cap are counted, not stored.
-__global__ void splat_emit_kernel(SplatArgs a) {
-    const uint32_t lane = threadIdx.x & 31u;
+// Fragments of 32 primitives per warp and round. A lane draws its own small
+// primitive (a box of at most kLaneCells pixels: dust points) - it counts the
+// pixels covered, the warp claims the slots of all its lanes with one atomic,
+// and the lane writes its keys; larger ones (discs) are then drawn one after
+// the other by the whole warp, one atomic for 32 pixels. Keys are
+// pixel << id_bits | particle; writes past cap are counted, not stored.
+// One atomic per fragment on the one cursor took 185 us for 500,205 particles
+// (about two million fragments); one per 32 primitives 32 us.
+constexpr uint32_t kLaneCells = 64;
+
+__global__ __launch_bounds__(256) void splat_emit_kernel(SplatArgs a) {
+    const uint32_t lane = threadIdx.x & 31u, lt = lanemask_lt();
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < a.n; i += warps) {
-        const uint32_t kind = a.kind[i];
-        if (kind == 0u) continue;
-        const float4 q = a.prim[i];
+    const uint32_t chunks = (a.n + 31u) / 32u;
+    for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < chunks; c += warps) {
+        const uint32_t i = c * 32u + lane;
+        uint32_t kind = i < a.n ? a.kind[i] : 0u;
+        const float4 q = kind ? a.prim[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         const float h = kind == 2u ? __fmul_rn(q.w, 0.5f) : q.w;
-        int x0, x1, y0, y1;
-        span(q.x, h, a.width, x0, x1);
-        span(q.y, h, a.height, y0, y1);
-        if (x1 < x0 || y1 < y0) continue;
-        const uint32_t bw = (uint32_t)(x1 - x0 + 1);
-        const uint64_t cells = (uint64_t)bw * (uint32_t)(y1 - y0 + 1);
-        for (uint64_t k = lane; k < cells; k += 32u) {
-            const int px = x0 + (int)(k % bw), py = y0 + (int)(k / bw);
-            if (!covers(kind, q, px, py)) continue;
-            const uint32_t slot = atomicAdd(a.cursor, 1u);
-            if (slot < a.cap)
-                a.keys[slot] = ((uint64_t)((uint32_t)py * a.width + (uint32_t)px) << 32) | i;
+        int x0 = 0, x1 = -1, y0 = 0, y1 = -1;
+        if (kind) {
+            span(q.x, h, a.width, x0, x1);
+            span(q.y, h, a.height, y0, y1);
+        }
+        if (x1 < x0 || y1 < y0) kind = 0u;
+        const uint64_t cells = kind ? (uint64_t)(uint32_t)(x1 - x0 + 1) * (uint32_t)(y1 - y0 + 1) : 0ull;
+        const bool small = cells <= kLaneCells;
+        uint32_t count = 0;
+        if (kind && small)
+            for (int py = y0; py <= y1; ++py)
+                for (int px = x0; px <= x1; ++px) count += covers(kind, q, px, py) ? 1u : 0u;
+        uint32_t incl = count;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        const uint32_t total = __shfl_sync(kFullMask, incl, 31);
+        if (total > 0u) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(a.cursor, total);
+            uint32_t slot = __shfl_sync(kFullMask, base, 0) + incl - count;
+            if (count)
+                for (int py = y0; py <= y1; ++py)
+                    for (int px = x0; px <= x1; ++px) {
+                        if (!covers(kind, q, px, py)) continue;
+                        if (slot < a.cap)
+                            a.keys[slot] =
+                                ((uint64_t)((uint32_t)py * a.width + (uint32_t)px) << a.id_bits) | i;
+                        ++slot;
+                    }
+        }
+        for (uint32_t big = __ballot_sync(kFullMask, !small); big; big &= big - 1u) {
+            const uint32_t src = (uint32_t)__ffs(big) - 1u;
+            const uint32_t bkind = __shfl_sync(kFullMask, kind, src);
+            const float4 bq = make_float4(
+                __shfl_sync(kFullMask, q.x, src), __shfl_sync(kFullMask, q.y, src),
+                __shfl_sync(kFullMask, q.z, src), __shfl_sync(kFullMask, q.w, src));
+            const int bx = __shfl_sync(kFullMask, x0, src), by = __shfl_sync(kFullMask, y0, src);
+            const uint32_t bw = (uint32_t)(__shfl_sync(kFullMask, x1, src) - bx + 1);
+            const uint64_t bcells = __shfl_sync(kFullMask, cells, src);
+            for (uint64_t k0 = 0; k0 < bcells; k0 += 32u) {
+                const uint64_t k = k0 + lane;
+                const int px = bx + (int)(k % bw), py = by + (int)(k / bw);
+                const bool in = k < bcells && covers(bkind, bq, px, py);
+                const uint32_t m = __ballot_sync(kFullMask, in);
+                if (m == 0u) continue;
+                uint32_t base = 0;
+                if (lane == 0) base = atomicAdd(a.cursor, (uint32_t)__popc(m));
+                const uint32_t slot = __shfl_sync(kFullMask, base, 0) + __popc(m & lt);
+                if (in && slot < a.cap)
+                    a.keys[slot] = ((uint64_t)((uint32_t)py * a.width + (uint32_t)px) << a.id_bits) |
+                                   (c * 32u + src);
+            }
         }
     }
 }
@@ -130,12 +182,13 @@ __global__ void splat_clear_kernel(SplatArgs a) {
 __global__ void splat_fold_kernel(SplatArgs a, const uint64_t* __restrict__ keys, uint32_t count) {
     const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= count) return;
-    const uint32_t pix = (uint32_t)(keys[f] >> 32);
-    if (f > 0 && (uint32_t)(keys[f - 1] >> 32) == pix) return;
+    const uint32_t pix = (uint32_t)(keys[f] >> a.id_bits);
+    if (f > 0 && (uint32_t)(keys[f - 1] >> a.id_bits) == pix) return;
+    const uint64_t id_mask = (1ull << a.id_bits) - 1ull;
     float4 dst = a.image[pix];
     float z = a.depth[pix];
-    for (uint32_t g = f; g < count && (uint32_t)(keys[g] >> 32) == pix; ++g) {
-        const uint32_t i = (uint32_t)(keys[g] & 0xFFFFFFFFull);
+    for (uint32_t g = f; g < count && (uint32_t)(keys[g] >> a.id_bits) == pix; ++g) {
+        const uint32_t i = (uint32_t)(keys[g] & id_mask);
         const float zf = a.prim[i].z;
         if (!(zf < z)) continue;
         const float4 src = a.colors[i];
@@ -164,7 +217,7 @@ cudaError_t launch_splat_project(const SplatArgs& a, cudaStream_t st) {
 
 cudaError_t launch_splat_emit(const SplatArgs& a, cudaStream_t st) {
     if (a.n == 0) return cudaSuccess;
-    const uint32_t blocks = (uint32_t)std::min<uint64_t>(((uint64_t)a.n * 32 + 255) / 256, 152u * 64u);
+    const uint32_t blocks = (uint32_t)std::min<uint64_t>(((uint64_t)a.n + 255) / 256, 152u * 64u);
     splat_emit_kernel<<<blocks, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
