@@ -21,7 +21,7 @@ OBJ_DIR = PKG / "_build"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
               "--expt-relaxed-constexpr", "-Xptxas", "-warn-spills"]
-SOURCES = ["sort.cu", "sort_noalloc.cu", "build.cu", "traverse.cu", "traverse_group.cu", "group_eval.cu",
+SOURCES = ["sort.cu", "sort_small.cu", "sort_noalloc.cu", "build.cu", "traverse.cu", "traverse_group.cu", "group_eval.cu",
            "splat.cu",
            "context.cu", "tune.cu", "ic.cpp"]
 

@@ -59,6 +59,14 @@ cudaError_t sort_pairs(const uint64_t* keys_in, const uint32_t* vals_in, uint64_
                        uint32_t key_bits, void* temp, size_t temp_bytes, cudaStream_t st,
                        uint32_t* err, uint32_t variant = 0);
 uint32_t sort_variant_count();
+// The one-launch sort of up to sort_small_max(device) pairs (sort_small.cu);
+// clear_err: a word to zero, or NULL.
+cudaError_t sort_small_init(int dev);
+uint32_t sort_small_max(int dev);
+cudaError_t sort_small(const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out,
+                       uint32_t* vals_out, uint64_t* keys_tmp, uint32_t* vals_tmp, uint32_t n_est,
+                       const uint32_t* d_count, uint32_t key_bits, int dev, cudaStream_t st,
+                       uint32_t* clear_err);
 // Test hook: a one-pass sort (key_bits <= 8) whose tile 0 is never
 // processed, so the look-back waits of the later tiles give up after
 // spin_limit polls and set the error word of `temp`.

@@ -13,6 +13,7 @@
 //      tile in sorted order in shared memory, obtains the counts of all
 //      earlier tiles by decoupled look-back (bounded waits), and writes each
 //      digit's run of the tile with contiguous stores.
+// Few pairs are sorted in one launch instead (sort_small.cu).
 // A stable LSD sort yields the one stable permutation, so the result equals
 // the reference's bit by bit, including the order of equal keys.
 #include <algorithm>
@@ -603,6 +604,7 @@ cudaError_t sort_init() {
     }
     e = cudaFuncSetAttribute(sort_histogram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(kWarps * kMaxPasses * kRadix * sizeof(uint32_t)));
+    if (e == cudaSuccess) e = sort_small_init(dev);
     if (e == cudaSuccess) g_init_done[dev] = true;
     return e;
 }
@@ -654,6 +656,13 @@ cudaError_t sort_launch(const uint64_t* keys_in, const uint32_t* vals_in, uint64
     if (stall_first_tile && plan.passes != 1) return cudaErrorInvalidValue;
     cudaError_t e0 = sort_init();
     if (e0 != cudaSuccess) return e0;
+    if (!stall_first_tile && n_est <= sort_small_max(current_device())) {
+        char* t = static_cast<char*>(temp);
+        uint32_t* own = err ? nullptr : reinterpret_cast<uint32_t*>(t + plan.counters) + kErrWord;
+        return sort_small(keys_in, vals_in, keys_out, vals_out, reinterpret_cast<uint64_t*>(t + plan.keys_tmp),
+                          reinterpret_cast<uint32_t*>(t + plan.vals_tmp), n_est, d_count, key_bits,
+                          current_device(), st, own);
+    }
     int vi = variant == 0 ? g_variant : (int)variant - 1;
     // Bulk copies need 16-byte aligned sources; the temporaries always are.
     // The stalled test pass needs one block per tile (no persistent blocks).
