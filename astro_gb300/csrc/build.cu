@@ -11,11 +11,16 @@
 // are aggregated one launch each and the small top layers in one climbing
 // launch (aggregate_tree_kernel).
 #include <algorithm>
+#include <mutex>
 #include <type_traits>
+
+#include <cooperative_groups.h>
 
 #include "build_kernels.cuh"
 #include "common.cuh"
 #include "internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace astro {
 
@@ -390,36 +395,34 @@ __device__ __forceinline__ float4 com_from_sums(double sx, double sy, double sz,
                        __double2float_rn(__dmul_rn(sz, inv)), __double2float_rn(m));
 }
 
-// Slots for c groups of this thread: the active lanes of the warp add their
-// counts and one lane claims them with a single atomic (one atomic per warp
-// instead of one per group on the shared counter); lanes take their runs in
-// lane order. Most calls have nothing to claim.
+// Slots for c groups of this thread: the warp's lanes (all of them call) add
+// their counts and one lane claims the slots with a single atomic (instead of
+// one per group on the shared counter); lanes take their runs in lane order.
+// Most calls have nothing to claim.
 __device__ __forceinline__ uint32_t reserve_groups(uint32_t* counter, uint32_t c) {
-    const uint32_t mask = __activemask();
-    const uint32_t some = __ballot_sync(mask, c != 0u);
-    if (some == 0u) return 0u;
+    if (__ballot_sync(kFullMask, c != 0u) == 0u) return 0u;
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t prefix = 0, total = 0;
-    for (uint32_t m = some; m != 0u; m &= m - 1u) {
-        const uint32_t l = (uint32_t)__ffs(m) - 1u;
-        const uint32_t cl = __shfl_sync(mask, c, l);
-        if (l < lane) prefix += cl;
-        total += cl;
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
     }
-    const uint32_t leader = (uint32_t)__ffs(some) - 1u;
     uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(counter, total);
-    return __shfl_sync(mask, base, leader) + prefix;
+    if (lane == 31u) base = atomicAdd(counter, incl);
+    return __shfl_sync(kFullMask, base, 31) + incl - c;
 }
 
 // Visits the particles [pb, pe) in order (the sums stay in particle order),
-// four at a time with the next four loaded ahead. One thread sums a leaf, so
-// a crowded leaf is a chain of load latencies: with one batch in flight the
-// leaf pass of a 524,288-body disk (leaves of up to about 70) took 47 us.
-template <typename F>
+// kBatch at a time with the next batch loaded ahead. One thread sums a leaf, so
+// a crowded leaf is a serial chain: with the next batch not loaded ahead the leaf
+// pass of a 524,288-body disk (leaves of up to about 70) took 47 us; 35 us in
+// batches of four, 28 us of eight (two or three batches ahead: 34 us). The
+// precision form, bound by the FP64 pipe, runs best at four (174 us against 217
+// for 4,194,304 bodies).
+template <uint32_t kBatch, typename F>
 __device__ __forceinline__ void for_particles(const float4* __restrict__ pos, uint32_t pb,
                                               uint32_t pe, F&& f) {
-    constexpr uint32_t kBatch = 4;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 next[kBatch];
 #pragma unroll
@@ -525,7 +528,7 @@ __device__ __forceinline__ void aggregate_ref_leaf(const AggArgs& a, uint32_t j,
     a.node_rng[j] = make_uint4(0u, 0u, pb, pe);
 }
 
-// Children are read through L2 (ld.global.cg): the climbing kernels below
+// Children are read through L2 (ld.global.cg): the cluster kernels below
 // read records that other blocks wrote in the same launch.
 __device__ __forceinline__ float4 ld_l2(const float4* p) { return __ldcg(p); }
 __device__ __forceinline__ float ld_l2(const float* p) { return __ldcg(p); }
@@ -640,7 +643,7 @@ __device__ __forceinline__ NodeRec<kPrec> aggregate_leaf(const AggArgs& a, uint3
     CellMoments mom;
     if constexpr (!kPrec) {
         float m = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
-        for_particles(a.pos, r.pb, r.pe, [&](const float4 q) {
+        for_particles<8>(a.pos, r.pb, r.pe, [&](const float4 q) {
             m = __fadd_rn(m, q.w);
             sx = __fadd_rn(sx, __fmul_rn(q.w, q.x));
             sy = __fadd_rn(sy, __fmul_rn(q.w, q.y));
@@ -653,7 +656,7 @@ __device__ __forceinline__ NodeRec<kPrec> aggregate_leaf(const AggArgs& a, uint3
         // The product of two floats is exact in FP64, so each FMA rounds
         // once, exactly as a multiply-then-add would.
         double m = 0, sx = 0, sy = 0, sz = 0;
-        for_particles(a.pos, r.pb, r.pe, [&](const float4 q) {
+        for_particles<4>(a.pos, r.pb, r.pe, [&](const float4 q) {
             const double mi = (double)q.w;
             m = __dadd_rn(m, mi);
             sx = __fma_rn(mi, (double)q.x, sx);
@@ -674,13 +677,62 @@ __device__ __forceinline__ NodeRec<kPrec> aggregate_leaf(const AggArgs& a, uint3
     }
     if (kQuad) mom.quadrupole(r.cm, box, r.q);
     store_node<kPrec, kQuad>(a, j, 0, 0u, 0u, r);
-    // A leaf holding more than one group is cut into group-sized chunks.
+    return r;
+}
+
+// A leaf holding more than one group is cut into group-sized chunks (all lanes
+// of the warp call; those without a leaf pass pe = pb).
+__device__ __forceinline__ void emit_chunks(const AggArgs& a, uint32_t pb, uint32_t pe) {
     const uint32_t gs = a.group_size;
-    const uint32_t c = r.pe - r.pb > gs ? (r.pe - r.pb + gs - 1u) / gs : 0u;
+    const uint32_t c = pe - pb > gs ? (pe - pb + gs - 1u) / gs : 0u;
     const uint32_t slot = reserve_groups(a.group_count, c);
     for (uint32_t i = 0; i < c; ++i)
-        a.groups[slot + i] = make_uint4(r.pb + i * gs, min(r.pb + (i + 1u) * gs, r.pe), r.pe, i);
-    return r;
+        a.groups[slot + i] = make_uint4(pb + i * gs, min(pb + (i + 1u) * gs, pe), pe, i);
+}
+
+// Groups of a node with several children that holds more particles than a
+// group: runs of consecutive small children (greedy, in child order). The
+// packing runs twice: to count the groups, then to write them into the slots
+// reserved for this node. All lanes of the warp call; those without such a node
+// pass ce = cb, and `root` marks a group [pb, pe) of its own.
+__device__ __forceinline__ void emit_groups(const AggArgs& a, uint32_t cb, uint32_t ce,
+                                            bool root = false, uint32_t pb = 0, uint32_t pe = 0) {
+    const uint32_t gs = a.group_size, nch = min(ce - cb, 8u);
+    uint2 cr[8];
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+        const uint4 rng = k < nch ? ld_l2(a.node_rng + cb + k) : make_uint4(0u, 0u, 0u, 0u);
+        cr[k] = make_uint2(rng.z, rng.w);
+    }
+    auto pack = [&](auto&& emit) {
+        uint32_t gb = 0, ge = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            if (k >= nch) break;
+            const uint32_t cc = cr[k].y - cr[k].x;
+            if (cc <= gs) {
+                if (ge == gb) {
+                    gb = cr[k].x;
+                    ge = cr[k].y;
+                } else if ((ge - gb) + cc <= gs) {
+                    ge = cr[k].y;
+                } else {
+                    emit(gb, ge);
+                    gb = cr[k].x;
+                    ge = cr[k].y;
+                }
+            } else if (ge != gb) {
+                emit(gb, ge);
+                gb = ge = 0;
+            }
+        }
+        if (ge != gb) emit(gb, ge);
+        if (root) emit(pb, pe);
+    };
+    uint32_t c = 0;
+    pack([&](uint32_t, uint32_t) { ++c; });
+    uint32_t slot = reserve_groups(a.group_count, c);
+    pack([&](uint32_t b, uint32_t e) { a.groups[slot++] = make_uint4(b, e, e, 0u); });
 }
 
 // aggregateNodes (Octree.metal:120-202) for a node with several children (at
@@ -742,52 +794,12 @@ __device__ __forceinline__ void aggregate_internal(const AggArgs& a, uint32_t l,
             }
         }
     }
-    // Groups: a node over the group size packs runs of consecutive small
-    // children (greedy, in child order). The packing runs twice: to count the
-    // groups, then to write them into the slots reserved for this node.
-    const uint32_t gs = a.group_size;
-    if (r.pe - r.pb > gs) {
-        uint2 cr[8];
-#pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) {
-            const uint4 rng = k < nch ? ld_l2(a.node_rng + cb + k) : make_uint4(0u, 0u, 0u, 0u);
-            cr[k] = make_uint2(rng.z, rng.w);
-        }
-        auto pack = [&](auto&& emit) {
-            uint32_t gb = 0, ge = 0;
-#pragma unroll
-            for (uint32_t k = 0; k < 8; ++k) {
-                if (k >= nch) break;
-                const uint32_t cc = cr[k].y - cr[k].x;
-                if (cc <= gs) {
-                    if (ge == gb) {
-                        gb = cr[k].x;
-                        ge = cr[k].y;
-                    } else if ((ge - gb) + cc <= gs) {
-                        ge = cr[k].y;
-                    } else {
-                        emit(gb, ge);
-                        gb = cr[k].x;
-                        ge = cr[k].y;
-                    }
-                } else if (ge != gb) {
-                    emit(gb, ge);
-                    gb = ge = 0;
-                }
-            }
-            if (ge != gb) emit(gb, ge);
-        };
-        uint32_t c = 0;
-        pack([&](uint32_t, uint32_t) { ++c; });
-        uint32_t slot = reserve_groups(a.group_count, c);
-        pack([&](uint32_t b, uint32_t e) { a.groups[slot++] = make_uint4(b, e, e, 0u); });
-    }
     store_node<kPrec, kQuad>(a, node, l, cb, ce, r);
 }
 
-// The bottom-up aggregation. Layers of at least kClimbMinNodes nodes (capacity)
+// The bottom-up aggregation. Layers of at least kLayerMinNodes nodes (capacity)
 // run one launch each, a thread per node with coalesced records; the rest of
-// the tree runs in one climbing launch.
+// the tree runs in one launch (aggregate_top_kernel).
 //
 // A parent with one child takes the child's sums, centre of mass and
 // quadrupole as they are (each sum is 0 + the child's, and no sum is -0), so
@@ -802,10 +814,10 @@ __device__ __forceinline__ void aggregate_internal(const AggArgs& a, uint32_t l,
 // small trees the launches and load latencies. Aggregation before and after
 // (one launch a layer, each re-reading its children): 6,000,007-body cube at 21
 // bits 4.55 -> 1.83 ms, two Plummer spheres of 4,194,304 in the precision form
-// 481 -> 356 us, 256 systems 590 -> 422 us, 524,288-body disk 146 -> 120 us.
-// Work lists in every layer: disk 134 us; in none: merger 420 us, 21 bits
-// 2.56 ms; the whole tree in one climbing launch: merger 594 us, disk 124 us.
-constexpr uint32_t kClimbMinNodes = 32768;
+// 481 -> 342 us, 256 systems 590 -> 424 us, 524,288-body disk 146 -> 105 us.
+// Work lists in every layer: disk 14 us more; in none: merger 64 us, 21 bits
+// 0.7 ms more; the whole tree in one climbing launch: merger 594 us, disk 124 us.
+constexpr uint32_t kLayerMinNodes = 32768;
 constexpr uint32_t kWorkMinNodes = 1u << 20;
 
 // The children [cb, ce) of node jp of layer l (u nodes there, `below` nodes
@@ -858,9 +870,11 @@ template <bool kPrec, bool kQuad>
 __global__ __launch_bounds__(128) void aggregate_leaf_kernel(AggArgs a, uint32_t top, uint32_t work_top) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t u0 = a.layer_count[0];
-    if (j >= u0) return;
-    NodeRec<kPrec> r = aggregate_leaf<kPrec, kQuad>(a, j, u0);
-    climb_chain<kPrec, kQuad>(a, 0, j, top, work_top, r);
+    NodeRec<kPrec> r;
+    r.pb = r.pe = 0;
+    if (j < u0) r = aggregate_leaf<kPrec, kQuad>(a, j, u0);
+    emit_chunks(a, r.pb, r.pe);
+    if (j < u0) climb_chain<kPrec, kQuad>(a, 0, j, top, work_top, r);
 }
 
 // The nodes of layer l with several children: the layer's work list (kWork;
@@ -869,95 +883,204 @@ template <bool kPrec, bool kQuad, bool kWork>
 __global__ __launch_bounds__(128) void aggregate_internal_kernel(AggArgs a, uint32_t l, uint32_t top,
                                                                  uint32_t work_top) {
     const uint32_t u = a.layer_count[l], count = kWork ? a.work_count[l] : u;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const uint32_t node = kWork ? a.work[a.offset[l] + i] : a.offset[l] + i, j = node - a.offset[l];
-        const Children c = children_of(a, node, j, u, l, a.layer_count[l - 1]);
-        if (!kWork && c.ce - c.cb == 1u) continue;
+    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < count; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + threadIdx.x;
+        uint32_t node = 0;
+        Children c{0u, 0u};
         NodeRec<kPrec> r;
-        r.pb = a.pbeg[node];
-        r.pe = (j + 1 < u) ? a.pbeg[node + 1] : a.n;
-        r.key = a.node_key[node];
-        aggregate_internal<kPrec, kQuad>(a, l, node, c.cb, c.ce, r);
-        climb_chain<kPrec, kQuad>(a, l, node, top, work_top, r);
+        r.pb = r.pe = 0;
+        bool several = false;
+        if (i < count) {
+            node = kWork ? a.work[a.offset[l] + i] : a.offset[l] + i;
+            const uint32_t j = node - a.offset[l];
+            c = children_of(a, node, j, u, l, a.layer_count[l - 1]);
+            several = kWork || c.ce - c.cb != 1u;
+            if (several) {
+                r.pb = a.pbeg[node];
+                r.pe = (j + 1 < u) ? a.pbeg[node + 1] : a.n;
+                r.key = a.node_key[node];
+                aggregate_internal<kPrec, kQuad>(a, l, node, c.cb, c.ce, r);
+            }
+        }
+        if (__any_sync(kFullMask, r.pe - r.pb > a.group_size))
+            emit_groups(a, c.cb, r.pe - r.pb > a.group_size ? c.ce : c.cb);
+        if (several) climb_chain<kPrec, kQuad>(a, l, node, top, work_top, r);
     }
 }
 
-// Layers l0 and up in one launch: a thread per node of layer l0 makes its
-// record and climbs. At a parent with several children it stores its node's
-// sums, makes its records visible (fence) and counts itself in; the thread
-// that completes the count aggregates the parent (reading the children
-// through L2), sets the count back to zero for the next build and climbs on;
-// the others stop. Every node is aggregated once, after all its children; no
-// thread waits on another. A small tree takes a chain of fences and dependent
-// loads up its layers; the parent's own links are loaded before the fence.
+// A node's links from the topology pass.
+struct Links {
+    uint32_t cb, ce, pb, pe;
+    uint64_t key;
+};
+__device__ __forceinline__ Links load_links(const AggArgs& a, uint32_t l, uint32_t j, uint32_t u,
+                                            uint32_t below) {
+    Links k{0u, 0u, 0u, 0u, 0ull};
+    if (j >= u) return k;
+    const uint32_t node = a.offset[l] + j;
+    const Children c = children_of(a, node, j, u, l, below);
+    k.cb = c.cb;
+    k.ce = c.ce;
+    k.pb = a.pbeg[node];
+    k.pe = (j + 1 < u) ? a.pbeg[node + 1] : a.n;
+    k.key = a.node_key[node];
+    return k;
+}
+
+// A node by eight lanes (all lanes of the warp call; `live`: the lane's group
+// has a node): every record of its children loaded at once, then lane c adds
+// component c of the sums and of the quadrupole, in child order. The same
+// roundings as aggregate_internal, an eighth of its serial work.
 template <bool kPrec, bool kQuad>
-__global__ __launch_bounds__(128) void aggregate_climb_kernel(AggArgs a, uint32_t l0) {
-    using Sum = typename NodeRec<kPrec>::Sum;
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t u0 = a.layer_count[l0];
-    if (j >= u0) return;
-    uint32_t node = a.offset[l0] + j;
-    uint32_t p = a.parent[node];
-    NodeRec<kPrec> r;
-    if (l0 == 0) {
-        r = aggregate_leaf<kPrec, kQuad>(a, j, u0);
-    } else {
-        const Children c = children_of(a, node, j, u0, l0, a.layer_count[l0 - 1]);
-        r.pb = a.pbeg[node];
-        r.pe = (j + 1 < u0) ? a.pbeg[node + 1] : a.n;
-        r.key = a.node_key[node];
-        if (c.ce - c.cb == 1u) {
-            r.sum = ld_l2(reinterpret_cast<const Sum*>(a.node_sum) + c.cb);
-            r.cm = ld_l2(a.node_cm + c.cb);
-            if (kQuad) {
-                const float4 q = ld_l2(a.node_q + c.cb);
-                r.q[0] = q.x, r.q[1] = q.y, r.q[2] = q.z, r.q[3] = q.w;
-                r.q[4] = ld_l2(a.node_qyz + c.cb);
+__device__ __forceinline__ void aggregate_wide(const AggArgs& a, uint32_t l, uint32_t node, bool live,
+                                               const Links& k) {
+    using Comp = typename std::conditional<kPrec, double, float>::type;
+    const uint32_t c = threadIdx.x & 7u;
+    if (live && k.ce - k.cb > 8u) atomicOr(a.err, kErrBadLayer);
+    const uint32_t nch = live ? min(k.ce - k.cb, 8u) : 0u;
+    Comp* const sums = reinterpret_cast<Comp*>(a.node_sum);
+    float* const quads = reinterpret_cast<float*>(a.node_q);
+    Comp sv[8];
+    float qv[8];
+    float4 ccm[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+        sv[i] = c < 4u && i < nch ? __ldcg(sums + 4ull * (k.cb + i) + c) : Comp(0);
+        ccm[i] = i < nch ? ld_l2(a.node_cm + k.cb + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        qv[i] = 0.f;
+        if (kQuad && i < nch && c < 5u)
+            qv[i] = __ldcg(c < 4u ? quads + 4ull * (k.cb + i) + c : a.node_qyz + k.cb + i);
+    }
+    Comp sum = Comp(0);
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i)
+        if (i < nch) {
+            if constexpr (kPrec) sum = __dadd_rn(sum, sv[i]);
+            else sum = __fadd_rn(sum, sv[i]);
+        }
+    const Comp m = __shfl_sync(kFullMask, sum, 3, 8);
+    const float4 com = com_from_sums(sum, sum, sum, m);  // this lane's component in x
+    float4 cm = make_float4(__shfl_sync(kFullMask, com.x, 0, 8), __shfl_sync(kFullMask, com.x, 1, 8),
+                            __shfl_sync(kFullMask, com.x, 2, 8), com.w);
+    float q = 0.f;
+    if (nch == 1u) {
+        cm = ccm[0];
+        q = qv[0];
+    } else if (kQuad) {
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i)
+            if (i < nch) {
+                const float dx = __fsub_rn(ccm[i].x, cm.x), dy = __fsub_rn(ccm[i].y, cm.y),
+                            dz = __fsub_rn(ccm[i].z, cm.z);
+                const float r2 =
+                    __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                // xx: tx dx - r2, yy: ty dy - r2, xy: tx dy, xz: tx dz, yz: ty dz.
+                const float t = __fmul_rn(3.0f, c == 1u || c == 4u ? dy : dx);
+                float v = __fmul_rn(t, c == 0u ? dx : (c < 3u ? dy : dz));
+                if (c < 2u) v = __fsub_rn(v, r2);
+                q = __fadd_rn(__fadd_rn(q, __fmul_rn(ccm[i].w, v)), qv[i]);
             }
-            store_node<kPrec, kQuad>(a, node, l0, c.cb, c.ce, r);
-        } else {
-            aggregate_internal<kPrec, kQuad>(a, l0, node, c.cb, c.ce, r);
-        }
     }
-    uint32_t below = u0;
-    for (uint32_t l = l0 + 1; l <= a.lbits; ++l) {
-        if (p == kNoParent) return;
-        const uint32_t u = a.layer_count[l];
-        const uint32_t jp = p - a.offset[l];
-        if (jp >= u) {
-            atomicOr(a.err, kErrBadLayer);
-            return;
+    if (!live) return;
+    if (c < 4u) sums[4ull * node + c] = sum;
+    if (kQuad && c < 5u) *(c < 4u ? quads + 4ull * node + c : a.node_qyz + node) = q;
+    if (c == 5u) a.node_cm[node] = cm;
+    if (c == 6u) a.node_rng[node] = make_uint4(k.cb, k.ce, k.pb, k.pe);
+    if (c == 7u && a.want_delta) a.node_crit2[node] = node_crit2(a, k.key, l, cm);
+}
+
+// Layers l0 and up in one launch of one thread-block cluster: a layer's nodes
+// are spread over its blocks, and the cluster barrier (which makes the blocks'
+// records visible to each other) ends the layer. The next layer's links, which
+// the topology pass wrote, are loaded while the barrier completes; the groups
+// are written after the last layer. Layers of few nodes give a node eight lanes.
+// What bounds it: the chain up the layers, each a barrier (about 1,000 cycles
+// until the stores have landed), the children's records and the arithmetic. A
+// tree of 9 layers: 26 us with 1,024 bodies, 34 us with 16,384. Climbing with an
+// arrival count per parent (fences, an atomic, one thread a node): 36 and 44 us;
+// this kernel with one thread a node and the groups written layer by layer: 37
+// and 49 us (3,500 to 4,600 cycles a node, 4,400 to 5,800 a layer of groups).
+constexpr uint32_t kTopThreads = 512;
+template <bool kPrec, bool kQuad>
+__global__ __launch_bounds__(kTopThreads, 1) void aggregate_top_kernel(AggArgs a, uint32_t l0) {
+    using Sum = typename NodeRec<kPrec>::Sum;
+    cg::cluster_group cluster = cg::this_cluster();
+    // Consecutive warps of nodes go to different blocks.
+    const uint32_t first = ((threadIdx.x >> 5) * cluster.num_blocks() + cluster.block_rank()) * 32u +
+                           (threadIdx.x & 31u);
+    const uint32_t stride = cluster.num_blocks() * kTopThreads;
+    Sum* const sums = reinterpret_cast<Sum*>(a.node_sum);
+    uint32_t u = a.layer_count[l0], below = l0 > 0 ? a.layer_count[l0 - 1] : 0u;
+    // Layers of few nodes give each node eight lanes.
+    const auto wide = [&](uint32_t l, uint32_t nodes) { return l > 0 && nodes <= stride / 4u; };
+    Links links{0u, 0u, 0u, 0u, 0ull};
+    if (l0 > 0) links = load_links(a, l0, wide(l0, u) ? first / 8u : first, u, below);
+    for (uint32_t l = l0; l <= a.lbits; ++l) {
+        const bool by_eight = wide(l, u);
+        const uint32_t warp_node = first / 32u * 4u;  // of the warp's first eight lanes
+        for (uint32_t j0 = by_eight ? warp_node : u; j0 < u; j0 += stride / 8u) {
+            const uint32_t j = j0 + (threadIdx.x & 31u) / 8u;
+            const Links k = j0 == warp_node ? links : load_links(a, l, j, u, below);
+            aggregate_wide<kPrec, kQuad>(a, l, a.offset[l] + j, j < u, k);
         }
-        const Children c = children_of(a, p, jp, u, l, below);
-        const uint32_t above = a.parent[p];
-        r.key >>= 3;
-        if (c.ce - c.cb > 1u) {
-            const uint32_t pb = a.pbeg[p], pe = (jp + 1 < u) ? a.pbeg[p + 1] : a.n;
-            reinterpret_cast<Sum*>(a.node_sum)[node] = r.sum;
-            __threadfence();
-            if (atomicAdd(&a.arrive[p], 1u) != c.ce - c.cb - 1u) return;
-            __threadfence();
-            a.arrive[p] = 0u;
-            r.pb = pb;
-            r.pe = pe;
-            aggregate_internal<kPrec, kQuad>(a, l, p, c.cb, c.ce, r);
-        } else {
-            store_node<kPrec, kQuad>(a, p, l, c.cb, c.ce, r);
+        for (uint32_t j = by_eight ? u : first; j < u; j += stride) {
+            const uint32_t node = a.offset[l] + j;
+            if (l == 0) {
+                const NodeRec<kPrec> r = aggregate_leaf<kPrec, kQuad>(a, j, u);
+                sums[node] = r.sum;
+                continue;
+            }
+            const Links k = j == first ? links : load_links(a, l, j, u, below);
+            NodeRec<kPrec> r;
+            r.pb = k.pb;
+            r.pe = k.pe;
+            r.key = k.key;
+            if (k.ce - k.cb == 1u) {
+                r.sum = ld_l2(sums + k.cb);
+                r.cm = ld_l2(a.node_cm + k.cb);
+                if (kQuad) {
+                    const float4 q = ld_l2(a.node_q + k.cb);
+                    r.q[0] = q.x, r.q[1] = q.y, r.q[2] = q.z, r.q[3] = q.w;
+                    r.q[4] = ld_l2(a.node_qyz + k.cb);
+                }
+                store_node<kPrec, kQuad>(a, node, l, k.cb, k.ce, r);
+            } else {
+                aggregate_internal<kPrec, kQuad>(a, l, node, k.cb, k.ce, r);
+            }
+            sums[node] = r.sum;
         }
-        node = p;
-        p = above;
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        const uint32_t above = l < a.lbits ? a.layer_count[l + 1] : 0u;
+        if (l < a.lbits) links = load_links(a, l + 1u, wide(l + 1u, above) ? first / 8u : first, above, u);
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
         below = u;
+        u = above;
     }
-    // The root of a system no larger than a group is a group by itself.
-    if (r.pe - r.pb <= a.group_size) {
-        const uint32_t slot = reserve_groups(a.group_count, 1u);
-        a.groups[slot] = make_uint4(r.pb, r.pe, r.pe, 0u);
+    // The groups of all these layers together (nothing above waits for them).
+    uint32_t total = 0;
+    for (uint32_t l = l0; l <= a.lbits; ++l) total += a.layer_count[l];
+    for (uint32_t t0 = first - (threadIdx.x & 31u); t0 < total; t0 += stride) {
+        uint32_t j = t0 + (threadIdx.x & 31u), l = l0;
+        const bool some = j < total;
+        while (some && j >= a.layer_count[l]) j -= a.layer_count[l++];
+        Links k{0u, 0u, 0u, 0u, 0ull};
+        if (some && l > 0) k = load_links(a, l, j, a.layer_count[l], a.layer_count[l - 1]);
+        if (some && l == 0) {
+            k.pb = a.pbeg[j];
+            k.pe = j + 1 < a.layer_count[0] ? a.pbeg[j + 1] : a.n;
+        }
+        const bool large = k.pe - k.pb > a.group_size;
+        if (l0 == 0) emit_chunks(a, k.pb, some && l == 0 ? k.pe : k.pb);
+        // The root of a system no larger than a group is a group by itself.
+        const bool root = some && l == a.lbits && !large;
+        if (__any_sync(kFullMask, root || (large && l > 0)))
+            emit_groups(a, k.cb, large && k.ce - k.cb > 1u ? k.ce : k.cb, root, k.pb, k.pe);
     }
 }
 
 // ---- REFERENCE ----
 
-// One launch per large layer, the rest of the tree climbing, as above.
+// One launch per large layer, the rest of the tree in one cluster.
 __global__ __launch_bounds__(128) void aggregate_ref_leaf_kernel(AggArgs a) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t u0 = a.layer_count[0];
@@ -970,33 +1093,19 @@ __global__ __launch_bounds__(128) void aggregate_ref_internal_kernel(AggArgs a, 
     if (j < u) aggregate_ref_internal(a, l, j, u);
 }
 
-// Layers l0 and up in one launch: one thread per node of layer l0.
-__global__ __launch_bounds__(128) void aggregate_ref_tree_kernel(AggArgs a, uint32_t l0) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t u0 = a.layer_count[l0];
-    if (j >= u0) return;
-    if (l0 == 0) aggregate_ref_leaf(a, j, u0);
-    else aggregate_ref_internal(a, l0, j, u0);
-    uint32_t node = a.offset[l0] + j;
-    for (uint32_t l = l0 + 1; l <= a.lbits; ++l) {
-        const uint32_t p = a.parent[node];
-        if (p == kNoParent) return;
+// Layers l0 and up in one launch of one cluster, as above.
+__global__ __launch_bounds__(kTopThreads, 1) void aggregate_ref_top_kernel(AggArgs a, uint32_t l0) {
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t first = ((threadIdx.x >> 5) * cluster.num_blocks() + cluster.block_rank()) * 32u +
+                           (threadIdx.x & 31u);
+    const uint32_t stride = cluster.num_blocks() * kTopThreads;
+    for (uint32_t l = l0; l <= a.lbits; ++l) {
         const uint32_t u = a.layer_count[l];
-        const uint32_t jp = p - a.offset[l];
-        if (jp >= u) {
-            atomicOr(a.err, kErrBadLayer);
-            return;
+        for (uint32_t j = first; j < u; j += stride) {
+            if (l == 0) aggregate_ref_leaf(a, j, u);
+            else aggregate_ref_internal(a, l, j, u);
         }
-        const uint32_t cb = a.node_cbeg[p];
-        const uint32_t ce = (jp + 1 < u) ? a.node_cbeg[p + 1] : a.offset[l - 1] + a.layer_count[l - 1];
-        if (ce - cb > 1u) {
-            __threadfence();
-            if (atomicAdd(&a.arrive[p], 1u) != ce - cb - 1u) return;
-            __threadfence();
-            a.arrive[p] = 0u;
-        }
-        aggregate_ref_internal(a, l, jp, u);
-        node = p;
+        cluster.sync();
     }
 }
 
@@ -1381,17 +1490,55 @@ cudaError_t launch_topology(const TopoArgs& a, cudaStream_t st) {
 }
 
 namespace {
-uint32_t climb_first_layer(const LayerTable& t) {
+uint32_t top_first_layer(const LayerTable& t) {
     uint32_t l0 = 0;
-    while (l0 + 1 < t.n_layers && t.size[l0] >= kClimbMinNodes) ++l0;
+    while (l0 + 1 < t.n_layers && t.size[l0] >= kLayerMinNodes) ++l0;
     return l0;
+}
+
+// Blocks of the cluster that a device runs (0: not asked yet), for every
+// cluster kernel.
+constexpr int kMaxDevices = 64;
+uint32_t g_top_blocks[kMaxDevices] = {};
+std::mutex g_top_mutex;
+using TopKernel = void (*)(AggArgs, uint32_t);
+const TopKernel kTopKernels[] = {aggregate_top_kernel<false, false>, aggregate_top_kernel<false, true>,
+                                 aggregate_top_kernel<true, false>, aggregate_top_kernel<true, true>,
+                                 aggregate_ref_top_kernel};
+
+void cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, uint32_t blocks, cudaStream_t st) {
+    *cfg = cudaLaunchConfig_t{};
+    cfg->gridDim = dim3(blocks);
+    cfg->blockDim = dim3(kTopThreads);
+    cfg->stream = st;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = blocks;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg->attrs = attr;
+    cfg->numAttrs = 1;
+}
+
+cudaError_t launch_cluster(TopKernel kernel, const AggArgs& a, uint32_t l0, cudaStream_t st) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    uint32_t blocks = 0;
+    {
+        std::lock_guard<std::mutex> lock(g_top_mutex);
+        if (dev >= 0 && dev < kMaxDevices) blocks = g_top_blocks[dev];
+    }
+    if (blocks == 0) return cudaErrorInvalidDevice;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    cluster_config(&cfg, &attr, blocks, st);
+    return cudaLaunchKernelEx(&cfg, kernel, a, l0);
 }
 
 constexpr uint32_t kWorkBlocks = 152 * 16;  // several waves at any register count
 
 template <bool kPrec, bool kQuad>
 cudaError_t launch_physical(const AggArgs& a, const LayerTable& t, cudaStream_t st) {
-    const uint32_t t0 = 128, l0 = climb_first_layer(t);
+    const uint32_t t0 = 128, l0 = top_first_layer(t);
     uint32_t lw = 0;  // layers below lw have work lists (sizes fall with the layer)
     while (lw < l0 && t.size[lw] >= kWorkMinNodes) ++lw;
     for (uint32_t l = 0; l < l0; ++l) {
@@ -1402,23 +1549,47 @@ cudaError_t launch_physical(const AggArgs& a, const LayerTable& t, cudaStream_t 
         else
             aggregate_internal_kernel<kPrec, kQuad, false><<<g, t0, 0, st>>>(a, l, l0, lw);
     }
-    aggregate_climb_kernel<kPrec, kQuad><<<blocks_for(t.size[l0], t0), t0, 0, st>>>(a, l0);
-    return cudaGetLastError();
+    return launch_cluster(aggregate_top_kernel<kPrec, kQuad>, a, l0, st);
 }
 }  // namespace
+
+// Cluster kernels: their attributes and the largest cluster, once per device;
+// called before any stream capture.
+cudaError_t build_init() {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lock(g_top_mutex);
+    if (g_top_blocks[dev]) return cudaSuccess;
+    uint32_t blocks = 16;
+    for (TopKernel k : kTopKernels) {
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+        for (; blocks > 1; blocks /= 2) {
+            cudaLaunchConfig_t cfg;
+            cudaLaunchAttribute attr;
+            cluster_config(&cfg, &attr, blocks, nullptr);
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) == cudaSuccess && clusters > 0) break;
+            (void)cudaGetLastError();
+        }
+    }
+    g_top_blocks[dev] = blocks;
+    return cudaSuccess;
+}
 
 cudaError_t launch_aggregate(int mode, const AggArgs& a, const LayerTable& t, cudaStream_t st) {
     const uint32_t t0 = 128;
     if (mode == 1) return a.want_quad ? launch_physical<false, true>(a, t, st) : launch_physical<false, false>(a, t, st);
     if (mode == 2) return a.want_quad ? launch_physical<true, true>(a, t, st) : launch_physical<true, false>(a, t, st);
-    const uint32_t l0 = climb_first_layer(t);
+    const uint32_t l0 = top_first_layer(t);
     for (uint32_t l = 0; l < l0; ++l) {
         const uint32_t g = blocks_for(t.size[l], t0);
         if (l == 0) aggregate_ref_leaf_kernel<<<g, t0, 0, st>>>(a);
         else aggregate_ref_internal_kernel<<<g, t0, 0, st>>>(a, l);
     }
-    aggregate_ref_tree_kernel<<<blocks_for(t.size[l0], t0), t0, 0, st>>>(a, l0);
-    return cudaGetLastError();
+    return launch_cluster(aggregate_ref_top_kernel, a, l0, st);
 }
 
 cudaError_t launch_integrate_ref(float4* pos, float4* vel, const float4* acc, const uint32_t* types,

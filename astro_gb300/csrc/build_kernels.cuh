@@ -32,11 +32,7 @@ struct AggArgs {
     const uint32_t* pbeg;
     const uint32_t* node_cbeg;
     const uint32_t* parent;    // per node: its parent (kNoParent at the top layer)
-    uint32_t* arrive;          // per internal node: children aggregated so far (zero between builds,
-                               // for the layers that climb)
-    uint32_t* work;            // per large layer, from its offset: its nodes with several
-                               // children (the storage of `arrive`, which only the
-                               // layers above them use)
+    uint32_t* work;            // per large layer, from its offset: its nodes with several children
     uint32_t* work_count;      // entries of each layer's work list (zeroed per build)
     const uint32_t* layer_count;
     uint32_t offset[ASTRO_MAX_LAYERS];  // first node of each layer
@@ -182,6 +178,7 @@ cudaError_t launch_reorder(bool prec, const uint32_t* perm, const float4* pos_a,
                            uint32_t* id_b, double* x_b, uint32_t n, cudaStream_t st);
 uint32_t topology_tiles(uint32_t n);
 cudaError_t launch_topology(const TopoArgs& a, cudaStream_t st);
+cudaError_t build_init();
 cudaError_t launch_aggregate(int mode, const AggArgs& a, const LayerTable& t, cudaStream_t st);
 cudaError_t launch_integrate_ref(float4* pos, float4* vel, const float4* acc, const uint32_t* types,
                                  uint32_t n, float dt, const astro_params& p, cudaStream_t st);

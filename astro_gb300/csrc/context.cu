@@ -133,7 +133,7 @@ int ensure_tree(astro_ctx* ctx, uint64_t capacity) {
     dev_free(ctx->node_pbeg);
     dev_free(ctx->node_cbeg);
     dev_free(ctx->node_parent);
-    dev_free(ctx->node_arrive);
+    dev_free(ctx->node_work);
     dev_free(ctx->node_crit2);
     dev_free(ctx->node_ecol);
     dev_free(ctx->node_ecen);
@@ -155,7 +155,7 @@ int ensure_tree(astro_ctx* ctx, uint64_t capacity) {
     CK(dev_alloc(&ctx->node_pbeg, cap + 1));
     CK(dev_alloc(&ctx->node_cbeg, cap + 1));
     CK(dev_alloc(&ctx->node_parent, cap));
-    CK(dev_alloc(&ctx->node_arrive, cap));
+    CK(dev_alloc(&ctx->node_work, cap));
     ctx->tree_capacity = cap;
     return ASTRO_OK;
 }
@@ -239,9 +239,6 @@ int check_device(astro_ctx* ctx) {
     }
     if (err) {
         CK(cudaMemset(ctx->err, 0, sizeof(uint32_t)));
-        // A build that went wrong may have left arrival counts behind.
-        if (ctx->node_arrive)
-            CK(cudaMemsetAsync(ctx->node_arrive, 0, ctx->tree_capacity * sizeof(uint32_t), ctx->stream));
         if (err & astro::kErrLookbackTimeout)
             return fail(ctx, ASTRO_ERR_DEVICE_TIMEOUT, "a decoupled look-back wait gave up");
         if (err & astro::kErrFrontier)
@@ -377,7 +374,6 @@ int stage_build(astro_ctx* ctx) {
     a.pbeg = ctx->node_pbeg;
     a.node_cbeg = ctx->node_cbeg;
     a.parent = ctx->node_parent;
-    a.arrive = ctx->node_arrive;
     a.layer_count = ctx->layer_count;
     for (uint32_t l = 0; l <= ctx->lbits; ++l) a.offset[l] = ctx->layers.offset[l];
     a.node_cm = ctx->node_cm;
@@ -389,7 +385,7 @@ int stage_build(astro_ctx* ctx) {
     a.node_qyz = ctx->node_qyz;
     a.groups = ctx->groups;
     a.group_count = ctx->counters + 2;
-    a.work = ctx->node_arrive;
+    a.work = ctx->node_work;
     a.work_count = ctx->counters + 16;
     if (!is_phys(ctx)) {
         a.colors = ctx->colors;
@@ -709,6 +705,7 @@ int astro_create(const astro_params* params, uint32_t max_n, uint32_t max_system
     CKC(cudaGetDevice(&ctx->device));
     CKC(astro::sort_init());
     CKC(astro::traverse_init());
+    CKC(astro::build_init());
     CKC(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     for (int b = 0; b < 2; ++b) {
         CKC(dev_alloc(&ctx->pos[b], max_n));
@@ -806,7 +803,7 @@ int astro_destroy(astro_ctx* ctx) {
     dev_free(ctx->node_pbeg);
     dev_free(ctx->node_cbeg);
     dev_free(ctx->node_parent);
-    dev_free(ctx->node_arrive);
+    dev_free(ctx->node_work);
     dev_free(ctx->node_crit2);
     dev_free(ctx->node_ecol);
     dev_free(ctx->node_ecen);
@@ -891,9 +888,6 @@ static int upload_common(astro_ctx* ctx, const PositionMass* pm, const VelocityR
     layer_table(sizes, ctx->lbits, &ctx->layers, &ctx->capacity);
     int r = ensure_tree(ctx, ctx->capacity);
     if (r != ASTRO_OK) return r;
-    // Arrival counts are zero between builds, but the large layers' part holds
-    // work lists, and the layers have moved.
-    CK(cudaMemsetAsync(ctx->node_arrive, 0, ctx->tree_capacity * sizeof(uint32_t), st));
     if ((r = ensure_frontier(ctx)) != ASTRO_OK) return r;
     if (prec && (r = ensure_x64(ctx)) != ASTRO_OK) return r;
     // Systems and chunks.

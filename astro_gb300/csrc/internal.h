@@ -154,7 +154,7 @@ struct astro_ctx {
     uint32_t* node_pbeg = nullptr;
     uint32_t* node_cbeg = nullptr;
     uint32_t* node_parent = nullptr;
-    uint32_t* node_arrive = nullptr;
+    uint32_t* node_work = nullptr;    // aggregation: work lists of the large layers
     float* node_crit2 = nullptr;      // opening radius^2 per node
     float4* node_ecol = nullptr;      // REFERENCE: emittedColor per node
     float4* node_ecen = nullptr;      // REFERENCE: emittedColorCenter per node
