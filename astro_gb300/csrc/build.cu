@@ -26,10 +26,21 @@ namespace astro {
 
 // ------------------------------------------------------------- encode ----
 
+// Zeroes what the next build and traversal count in. One memset for each of
+// these small buffers cost a step seven launches of 1 us and their gaps.
+__device__ __forceinline__ void clear_scratch(const ClearArgs& c) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+    for (uint32_t k = i; k < c.lookback_words; k += threads) c.lookback[k] = 0u;
+    for (uint32_t k = i; k < kCounterWords; k += threads)
+        if (k < kClearedWords || k >= kWorkCounts) c.counters[k] = 0u;
+    for (uint32_t k = i; k < c.num_stats; k += threads) c.stats[k] = 0ull;
+}
+
 // generateMortonCodes with the reference quantiser (u32)(p + 1e6): the
 // float-to-uint conversion saturates and rounds toward zero.
 __global__ void encode_ref_kernel(const float4* __restrict__ pos, uint64_t* __restrict__ codes,
-                                  uint32_t n_tree, uint32_t unused_bits, float offset) {
+                                  uint32_t n_tree, uint32_t unused_bits, float offset, ClearArgs clear) {
+    clear_scratch(clear);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_tree) return;
     const float4 q = pos[i];
@@ -206,7 +217,8 @@ __global__ void reorder_kernel(const uint32_t* __restrict__ perm, const float4* 
                                const float4* __restrict__ vel_a, const uint32_t* __restrict__ id_a,
                                const double* __restrict__ x_a, float4* __restrict__ pos_b,
                                float4* __restrict__ vel_b, uint32_t* __restrict__ id_b,
-                               double* __restrict__ x_b, uint32_t n) {
+                               double* __restrict__ x_b, uint32_t n, ClearArgs clear) {
+    clear_scratch(clear);
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const uint32_t s = perm[j];
@@ -224,8 +236,13 @@ __global__ void reorder_kernel(const uint32_t* __restrict__ perm, const float4* 
 
 constexpr int kTopoThreads = 256;
 constexpr int kTopoWarps = kTopoThreads / 32;
-constexpr int kTopoItems = 8;
-constexpr int kTopoTile = kTopoThreads * kTopoItems;
+
+// Keys per thread: few where the array is small, so that the tiles spread over
+// the chip and the serial loops over keys and layers are short (16,384 bodies,
+// two keys: 6.6 us, eight keys: 15.4; 524,288 bodies, four keys: 18 us, eight:
+// 24); eight where the look-back over many tiles would cost more.
+constexpr uint32_t kTopoSmall = 1u << 17, kTopoMedium = 1u << 20;
+constexpr uint32_t topo_items(uint32_t n) { return n <= kTopoSmall ? 2u : (n <= kTopoMedium ? 4u : 8u); }
 
 // One pass over the sorted keys finds the nodes of every layer. Position i
 // starts a node at layer l when its key differs from key i-1 above bit 3l,
@@ -238,7 +255,9 @@ constexpr int kTopoTile = kTopoThreads * kTopoItems;
 // for all layers without re-sorting or re-scanning per layer. Each node
 // below the top layer also gets its parent: the node one layer up that
 // holds its first particle (the bottom-up aggregation climbs these links).
+template <int kTopoItems>
 __global__ __launch_bounds__(kTopoThreads) void topology_kernel(TopoArgs a) {
+    constexpr int kTopoTile = kTopoThreads * kTopoItems;
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_off[ASTRO_MAX_LAYERS];
     __shared__ uint32_t s_wcnt[kTopoWarps][32];
@@ -1432,10 +1451,10 @@ inline uint32_t blocks_for(uint64_t n, uint32_t t) { return (uint32_t)((n + t - 
 }  // namespace
 
 cudaError_t launch_encode_ref(const float4* pos, uint64_t* codes, uint32_t n_tree, uint32_t lbits,
-                              float offset, cudaStream_t st) {
+                              float offset, const ClearArgs& clear, cudaStream_t st) {
     if (n_tree == 0) return cudaSuccess;
     encode_ref_kernel<<<blocks_for(n_tree, 256), 256, 0, st>>>(pos, codes, n_tree, 63u - 3u * lbits,
-                                                               offset);
+                                                               offset, clear);
     return cudaGetLastError();
 }
 
@@ -1471,21 +1490,31 @@ cudaError_t launch_setup(bool prec, SysInfo* sys, uint32_t nsys, uint32_t* bb32,
 
 cudaError_t launch_reorder(bool prec, const uint32_t* perm, const float4* pos_a, const float4* vel_a,
                            const uint32_t* id_a, const double* x_a, float4* pos_b, float4* vel_b,
-                           uint32_t* id_b, double* x_b, uint32_t n, cudaStream_t st) {
+                           uint32_t* id_b, double* x_b, uint32_t n, const ClearArgs& clear,
+                           cudaStream_t st) {
     if (prec)
-        reorder_kernel<true><<<blocks_for(n, 256), 256, 0, st>>>(perm, pos_a, vel_a, id_a, x_a,
-                                                                 pos_b, vel_b, id_b, x_b, n);
+        reorder_kernel<true><<<blocks_for(n, 256), 256, 0, st>>>(perm, pos_a, vel_a, id_a, x_a, pos_b,
+                                                                 vel_b, id_b, x_b, n, clear);
     else
-        reorder_kernel<false><<<blocks_for(n, 256), 256, 0, st>>>(perm, pos_a, vel_a, id_a, x_a,
-                                                                  pos_b, vel_b, id_b, x_b, n);
+        reorder_kernel<false><<<blocks_for(n, 256), 256, 0, st>>>(perm, pos_a, vel_a, id_a, x_a, pos_b,
+                                                                  vel_b, id_b, x_b, n, clear);
     return cudaGetLastError();
 }
 
-uint32_t topology_tiles(uint32_t n) { return blocks_for(n, kTopoTile); }
+uint32_t topology_tiles(uint32_t n) { return blocks_for(n, kTopoThreads * topo_items(n)); }
+// Of any count up to max_n (the tiles grow with the count).
+uint32_t topology_tiles_max(uint32_t max_n) {
+    return std::max(topology_tiles(max_n),
+                    std::max(topology_tiles(std::min(max_n, kTopoSmall)), topology_tiles(std::min(max_n, kTopoMedium))));
+}
 
 cudaError_t launch_topology(const TopoArgs& a, cudaStream_t st) {
     if (a.n == 0) return cudaSuccess;
-    topology_kernel<<<a.ntiles, kTopoThreads, 0, st>>>(a);
+    switch (topo_items(a.n)) {
+        case 2: topology_kernel<2><<<a.ntiles, kTopoThreads, 0, st>>>(a); break;
+        case 4: topology_kernel<4><<<a.ntiles, kTopoThreads, 0, st>>>(a); break;
+        default: topology_kernel<8><<<a.ntiles, kTopoThreads, 0, st>>>(a); break;
+    }
     return cudaGetLastError();
 }
 

@@ -73,6 +73,21 @@ constexpr uint32_t kGroupSize = 64;     // largest group of the group walk (two 
 constexpr uint32_t kDefaultGroupSize = 32;  // group_size 0
 constexpr uint32_t kNoParent = 0xFFFFFFFFu;
 
+// Words of the context's counter array: [0] topology tiles, [1] walk queue,
+// [2] groups, [3] evaluation queue, [4] list pool, all zero when a build and its
+// traversal begin; [5] frontier wanted and [6] evaluations run, kept; from
+// kWorkCounts on the work lists' counts, zero when a build begins.
+constexpr uint32_t kClearedWords = 5;
+constexpr uint32_t kWorkCounts = 16;
+constexpr uint32_t kCounterWords = kWorkCounts + ASTRO_MAX_LAYERS;
+struct ClearArgs {
+    uint32_t* lookback;       // topology look-back words
+    uint32_t lookback_words;  // (0: nothing to clear there)
+    uint32_t* counters;
+    unsigned long long* stats;
+    uint32_t num_stats;
+};
+
 struct DirectArgs {
     const float4* pos;
     const double* x64;
@@ -163,7 +178,7 @@ struct TraverseArgs {
 };
 
 cudaError_t launch_encode_ref(const float4* pos, uint64_t* codes, uint32_t n_tree, uint32_t lbits,
-                              float offset, cudaStream_t st);
+                              float offset, const ClearArgs& clear, cudaStream_t st);
 cudaError_t launch_encode_phys(bool prec, const Chunk* chunks, uint32_t nchunks, const SysInfo* sys,
                                float4* pos, const double* x64, uint64_t* codes, uint32_t n,
                                uint32_t lbits, cudaStream_t st);
@@ -175,8 +190,10 @@ cudaError_t launch_setup(bool prec, SysInfo* sys, uint32_t nsys, uint32_t* bb32,
                          cudaStream_t st);
 cudaError_t launch_reorder(bool prec, const uint32_t* perm, const float4* pos_a, const float4* vel_a,
                            const uint32_t* id_a, const double* x_a, float4* pos_b, float4* vel_b,
-                           uint32_t* id_b, double* x_b, uint32_t n, cudaStream_t st);
+                           uint32_t* id_b, double* x_b, uint32_t n, const ClearArgs& clear,
+                           cudaStream_t st);
 uint32_t topology_tiles(uint32_t n);
+uint32_t topology_tiles_max(uint32_t max_n);
 cudaError_t launch_topology(const TopoArgs& a, cudaStream_t st);
 cudaError_t build_init();
 cudaError_t launch_aggregate(int mode, const AggArgs& a, const LayerTable& t, cudaStream_t st);
@@ -272,7 +289,8 @@ uint32_t group_walk_warps();
 size_t group_list_blocks(uint32_t n, uint32_t group_size);
 // ev (optional, three events): recorded before the walk, between the walk
 // and the evaluation, and after it.
-cudaError_t launch_traverse_groups(const TraverseArgs& a, const TraverseConfig& c, cudaStream_t st,
-                                   cudaEvent_t* ev = nullptr);
+// clean: the queues and the list pool's counter are already zero.
+cudaError_t launch_traverse_groups(const TraverseArgs& a, const TraverseConfig& c, bool clean,
+                                   cudaStream_t st, cudaEvent_t* ev = nullptr);
 
 }  // namespace astro

@@ -311,11 +311,20 @@ int ensure_frontier(astro_ctx* ctx) {
 
 // --------------------------------------------------------------- stages --
 
+// What a build and a traversal count in, zeroed by a kernel that runs before
+// them (the statistics only inside a whole step: between stage calls they are
+// the last traversal's until the next one).
+astro::ClearArgs clear_args(astro_ctx* ctx, uint32_t count) {
+    return astro::ClearArgs{ctx->topo_lookback, astro::topology_tiles(count) * 32u, ctx->counters,
+                            ctx->stats, ctx->whole_step ? (uint32_t)kNumStats : 0u};
+}
+
 int stage_encode(astro_ctx* ctx) {
     cudaStream_t st = ctx->stream;
     if (!is_phys(ctx)) {
-        CK(astro::launch_encode_ref(ctx->pos[0], ctx->codes, ctx->n_tree, ctx->lbits,
-                                    ctx->p.quant_offset, st));
+        CK(astro::launch_encode_ref(ctx->pos[0], ctx->codes, ctx->n_tree, ctx->lbits, ctx->p.quant_offset,
+                                    clear_args(ctx, ctx->n_tree), st));
+        ctx->build_clean = ctx->walk_clean = ctx->n_tree > 0;
         return ASTRO_OK;
     }
     if (ctx->state_in_b) return fail(ctx, ASTRO_ERR_STATE, "encode called between sort and traverse");
@@ -339,8 +348,9 @@ int stage_sort(astro_ctx* ctx) {
         if (ctx->state_in_b) return fail(ctx, ASTRO_ERR_STATE, "sort called twice without traverse");
         CK(astro::launch_reorder(is_prec(ctx), ctx->perm, ctx->pos[0], ctx->vel[0], ctx->ids[0],
                                  ctx->x64[0], ctx->pos[1], ctx->vel[1], ctx->ids[1], ctx->x64[1],
-                                 ctx->n, st));
+                                 ctx->n, clear_args(ctx, ctx->n), st));
         ctx->state_in_b = true;
+        ctx->build_clean = ctx->walk_clean = true;
     }
     return ASTRO_OK;
 }
@@ -364,8 +374,13 @@ int stage_build(astro_ctx* ctx) {
     t.lookback = ctx->topo_lookback;
     t.tile_counter = ctx->counters;
     t.err = ctx->err;
-    CK(cudaMemsetAsync(ctx->topo_lookback, 0, (size_t)t.ntiles * 32 * sizeof(uint32_t), st));
-    CK(cudaMemsetAsync(ctx->counters, 0, sizeof(uint32_t), st));
+    if (!ctx->build_clean) {
+        CK(cudaMemsetAsync(ctx->topo_lookback, 0, (size_t)t.ntiles * 32 * sizeof(uint32_t), st));
+        CK(cudaMemsetAsync(ctx->counters, 0, sizeof(uint32_t), st));
+        CK(cudaMemsetAsync(ctx->counters + 2, 0, sizeof(uint32_t), st));
+        CK(cudaMemsetAsync(ctx->counters + astro::kWorkCounts, 0, ASTRO_MAX_LAYERS * sizeof(uint32_t), st));
+    }
+    ctx->build_clean = false;
     CK(astro::launch_topology(t, st));
     astro::AggArgs a{};
     a.perm = ctx->perm;
@@ -386,7 +401,7 @@ int stage_build(astro_ctx* ctx) {
     a.groups = ctx->groups;
     a.group_count = ctx->counters + 2;
     a.work = ctx->node_work;
-    a.work_count = ctx->counters + 16;
+    a.work_count = ctx->counters + astro::kWorkCounts;
     if (!is_phys(ctx)) {
         a.colors = ctx->colors;
         a.types = ctx->types;
@@ -401,8 +416,6 @@ int stage_build(astro_ctx* ctx) {
     a.delta_weight = ctx->p.open_delta_weight;
     a.group_size = ctx->p.group_size ? ctx->p.group_size : astro::kDefaultGroupSize;
     a.err = ctx->err;
-    CK(cudaMemsetAsync(ctx->counters + 2, 0, sizeof(uint32_t), st));
-    CK(cudaMemsetAsync(ctx->counters + 16, 0, ASTRO_MAX_LAYERS * sizeof(uint32_t), st));
     const int mode = !is_phys(ctx) ? 0 : (is_prec(ctx) ? 2 : 1);
     CK(astro::launch_aggregate(mode, a, ctx->layers, st));
     ctx->tree_valid = true;
@@ -476,7 +489,11 @@ astro::TraverseArgs traverse_args(astro_ctx* ctx, float dt, bool integrate) {
 // evaluates forces (the state is copied back to A unchanged).
 int stage_traverse(astro_ctx* ctx, float dt, bool integrate) {
     cudaStream_t st = ctx->stream;
-    CK(cudaMemsetAsync(ctx->stats, 0, kNumStats * sizeof(unsigned long long), st));
+    // A whole step has zeroed the statistics and the queues before.
+    const bool clean = ctx->walk_clean;
+    if (!(clean && ctx->whole_step))
+        CK(cudaMemsetAsync(ctx->stats, 0, kNumStats * sizeof(unsigned long long), st));
+    ctx->walk_clean = false;
     if (!is_phys(ctx)) {
         if (ctx->n_tree == 0) {
             CK(cudaMemsetAsync(ctx->acc, 0, sizeof(float4) * ctx->n, st));
@@ -500,7 +517,7 @@ int stage_traverse(astro_ctx* ctx, float dt, bool integrate) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         CK(cudaStreamIsCapturing(st, &cap));
         const bool timed = cap == cudaStreamCaptureStatusNone;
-        CK(astro::launch_traverse_groups(traverse_args(ctx, dt, integrate), traverse_config(ctx), st,
+        CK(astro::launch_traverse_groups(traverse_args(ctx, dt, integrate), traverse_config(ctx), clean, st,
                                          timed ? ctx->trav_ev : nullptr));
         ctx->trav_timed = timed;
     } else {
@@ -522,7 +539,7 @@ int stage_integrate(astro_ctx* ctx, float dt) {
     return ASTRO_OK;
 }
 
-int run_step(astro_ctx* ctx, float dt) {
+int run_stages(astro_ctx* ctx, float dt) {
     int r;
     if ((r = stage_encode(ctx)) != ASTRO_OK) return r;
     if ((r = stage_sort(ctx)) != ASTRO_OK) return r;
@@ -534,6 +551,13 @@ int run_step(astro_ctx* ctx, float dt) {
         CK(astro::launch_lighting(ctx->pos[0], ctx->types, ctx->colors, ctx->lights, ctx->n,
                                   ctx->p.light_sources, ctx->stream));
     return stage_integrate(ctx, dt);
+}
+
+int run_step(astro_ctx* ctx, float dt) {
+    ctx->whole_step = true;
+    const int r = run_stages(ctx, dt);
+    ctx->whole_step = false;
+    return r;
 }
 
 void drop_graph(astro_ctx* ctx) {
@@ -580,6 +604,7 @@ int launch_steps(astro_ctx* ctx, float dt, uint32_t nsteps) {
     if ((r = ensure_frontier(ctx)) != ASTRO_OK) return r;
     if (!(ctx->graph_valid && ctx->graph_dt == dt))
         if ((r = capture_step(ctx, dt)) != ASTRO_OK) return r;
+    ctx->build_clean = ctx->walk_clean = false;  // the steps count in them
     for (uint32_t s = 0; s < nsteps; ++s) CK(cudaGraphLaunch(ctx->graph, ctx->stream));
     ctx->tree_valid = true;
     return ASTRO_OK;
@@ -725,9 +750,10 @@ int astro_create(const astro_params* params, uint32_t max_n, uint32_t max_system
     CKC(cudaMalloc(&ctx->staging, ctx->staging_bytes));
     ctx->sort_temp_bytes = astro::sort_plan(max_n, 64).total;
     CKC(cudaMalloc(&ctx->sort_temp, ctx->sort_temp_bytes));
-    ctx->topo_lookback_words = (size_t)astro::topology_tiles(max_n) * 32 + 32;
+    ctx->topo_lookback_words = (size_t)astro::topology_tiles_max(max_n) * 32 + 32;
     CKC(dev_alloc(&ctx->topo_lookback, ctx->topo_lookback_words));
-    CKC(dev_alloc(&ctx->counters, 64));
+    CKC(dev_alloc(&ctx->counters, astro::kCounterWords));
+    CKC(cudaMemset(ctx->counters, 0, astro::kCounterWords * sizeof(uint32_t)));
     CKC(dev_alloc(&ctx->groups, max_n));
     CKC(dev_alloc(&ctx->err, 1));
     CKC(dev_alloc(&ctx->stats, kNumStats));
@@ -736,7 +762,7 @@ int astro_create(const astro_params* params, uint32_t max_n, uint32_t max_system
     CKC(dev_alloc(&ctx->sys, max_systems));
     CKC(dev_alloc(&ctx->bbox32, 6ull * max_systems));
     CKC(dev_alloc(&ctx->bbox64, 6ull * max_systems));
-    ctx->chunk_capacity = max_n / astro::kChunkParticles + max_systems + 1;
+    ctx->chunk_capacity = max_n / astro::kChunkParticles + 1300 + max_systems;  // see chunk_particles
     CKC(dev_alloc(&ctx->chunks, ctx->chunk_capacity));
     CKC(cudaMemset(ctx->err, 0, sizeof(uint32_t)));
     CKC(cudaMemset(ctx->layer_count, 0, sizeof(uint32_t) * ASTRO_MAX_LAYERS));
@@ -879,6 +905,7 @@ static int upload_common(astro_ctx* ctx, const PositionMass* pm, const VelocityR
     ctx->uploaded = false;
     ctx->n = n;
     ctx->n_tree = n_tree;
+    ctx->build_clean = ctx->walk_clean = false;  // cleared for another count
     ctx->nsys = (uint32_t)sizes.size();
     ctx->lbits = ctx->p.lbits;
     ctx->sysbits = ctx->nsys > 1 ? bits_for(ctx->nsys) : 0;
@@ -893,14 +920,15 @@ static int upload_common(astro_ctx* ctx, const PositionMass* pm, const VelocityR
     // Systems and chunks.
     std::vector<SysInfo> sys(ctx->nsys);
     std::vector<Chunk> chunks;
+    const uint32_t chunk = astro::chunk_particles(n);
     uint32_t off = 0;
     for (uint32_t s = 0; s < ctx->nsys; ++s) {
         std::memset(&sys[s], 0, sizeof(SysInfo));
         sys[s].begin = off;
         sys[s].end = off + sizes[s];
         sys[s].root = ctx->layers.offset[ctx->lbits] + s;
-        for (uint32_t b = off; b < off + sizes[s]; b += astro::kChunkParticles)
-            chunks.push_back(Chunk{s, b, std::min(b + astro::kChunkParticles, off + sizes[s]), 0});
+        for (uint32_t b = off; b < off + sizes[s]; b += chunk)
+            chunks.push_back(Chunk{s, b, std::min(b + chunk, off + sizes[s]), 0});
         off += sizes[s];
     }
     if (chunks.size() > ctx->chunk_capacity) return fail(ctx, ASTRO_ERR_CAPACITY, "too many chunks");

@@ -31,7 +31,14 @@ struct SysInfo {
 struct Chunk {
     uint32_t sys, begin, end, _pad;
 };
-constexpr uint32_t kChunkParticles = 4096;
+constexpr uint32_t kChunkParticles = 4096;  // at most
+// Small systems are cut finer, so that about 600 blocks share the particles
+// (4,096 a block left 16,384 bodies to four blocks: bbox and encode 6 us each).
+inline uint32_t chunk_particles(uint32_t n) {
+    uint32_t c = 256;
+    while (c < kChunkParticles && c * 608u < n) c *= 2u;
+    return c;
+}
 
 struct LayerTable {
     uint32_t n_layers;
@@ -187,7 +194,10 @@ struct astro_ctx {
     size_t sort_temp_bytes = 0;
     uint32_t* topo_lookback = nullptr;
     size_t topo_lookback_words = 0;
-    uint32_t* counters = nullptr;             // [0] topology tiles, [1] traversal queue, [2] groups
+    uint32_t* counters = nullptr;             // kCounterWords words, see ClearArgs
+    bool build_clean = false;                 // the sort (encode, REFERENCE) zeroed the build's ...
+    bool walk_clean = false;                  // ... and the traversal's counters since they ran
+    bool whole_step = false;                  // run_step is launching the stages
     uint32_t* err = nullptr;                  // device error word
     cudaEvent_t trav_ev[3] = {nullptr, nullptr, nullptr};  // traversal stage call: before,
                                               // between walk and evaluation, after

@@ -519,14 +519,15 @@ size_t group_list_blocks(uint32_t n, uint32_t group_size) {
     return std::min<size_t>(blocks, 0xFFFFFF00ull);
 }
 
-cudaError_t launch_traverse_groups(const TraverseArgs& a, const TraverseConfig& c, cudaStream_t st,
-                                   cudaEvent_t* ev) {
+cudaError_t launch_traverse_groups(const TraverseArgs& a, const TraverseConfig& c, bool clean,
+                                   cudaStream_t st, cudaEvent_t* ev) {
     if (a.n == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
-    // Evaluation queue and list pool counter (adjacent words).
-    e = cudaMemsetAsync(a.eval_queue, 0, 2 * sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
+    if (!clean) {
+        if ((e = cudaMemsetAsync(a.queue, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
+        // Evaluation queue and list pool counter (adjacent words).
+        if ((e = cudaMemsetAsync(a.eval_queue, 0, 2 * sizeof(uint32_t), st)) != cudaSuccess) return e;
+    }
     if (ev && (e = cudaEventRecord(ev[0], st)) != cudaSuccess) return e;
     auto walk = a.delta ? (a.far2 > 0.f ? group_walk_kernel<true, true> : group_walk_kernel<true, false>)
                         : (a.far2 > 0.f ? group_walk_kernel<false, true> : group_walk_kernel<false, false>);
