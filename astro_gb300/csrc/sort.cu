@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "internal.h"
@@ -60,15 +61,41 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
     return r;
 }
 
-// Lanes of the warp whose digit equals this lane's digit, among `valid`.
-__device__ __forceinline__ uint32_t peer_mask(uint32_t digit, uint32_t bits, uint32_t valid) {
+// The digit of a pass. Passes start at multiples of 8 bits, so a digit lies in
+// one word of the key.
+__device__ __forceinline__ uint32_t digit_of(uint64_t key, uint32_t shift, uint32_t dmask) {
+    const uint32_t w = (shift & 32u) ? (uint32_t)(key >> 32) : (uint32_t)key;
+    return (w >> (shift & 31u)) & dmask;
+}
+
+// Lanes of the warp whose digit equals this lane's digit, among `valid`. All
+// eight bits are compared, also where the last digit has fewer: the loop has to
+// be unrolled (over the run-time width, with the checks that whole tiles
+// do not need it cost a pass 187 instructions for 32 keys, and 16.7 M pairs 156
+// us a pass against 135).
+__device__ __forceinline__ uint32_t peer_mask(uint32_t digit, uint32_t valid) {
     uint32_t peers = valid;
-    for (uint32_t b = 0; b < bits; ++b) {
-        uint32_t bit = (digit >> b) & 1u;
-        uint32_t ballot = __ballot_sync(kFullMask, bit);
+#pragma unroll
+    for (uint32_t b = 0; b < 8; ++b) {
+        const bool bit = (digit & (1u << b)) != 0u;
+        const uint32_t ballot = __ballot_sync(kFullMask, bit);
         peers &= bit ? ballot : ~ballot;
     }
     return peers;
+}
+
+// Stable rank of this lane's key among the keys of its digit that the warp has
+// ranked so far; counts the warp's keys in `hist`.
+__device__ __forceinline__ uint32_t warp_rank(uint32_t* hist, uint32_t digit, bool valid, uint32_t valid_mask,
+                                              uint32_t lane, uint32_t lt) {
+    const uint32_t peers = peer_mask(digit, valid_mask);
+    uint32_t rank = __popc(peers & lt);
+    if (valid) rank += hist[digit];
+    __syncwarp();
+    // The last lane of the digit has the highest rank.
+    if (valid && (peers & ~lt) == (1u << lane)) hist[digit] = rank + 1u;
+    __syncwarp();
+    return rank;
 }
 
 // All digit histograms in one read of the keys. Each warp counts into its own
@@ -88,6 +115,7 @@ __global__ __launch_bounds__(kThreads) void sort_histogram_kernel(
     for (uint32_t i = tid; i < kWarps * per_warp; i += kThreads) s_hist[i] = 0;
     __syncthreads();
     uint32_t* my_hist = s_hist + warp * per_warp;
+    const uint32_t last_mask = key_bits == 0 ? 0u : (1u << (key_bits - 8u * (passes - 1u))) - 1u;
     // Each thread takes kHistKeys keys per round (independent loads in flight).
     constexpr int kHistKeys = 4;
     const uint64_t stride = (uint64_t)gridDim.x * kThreads * kHistKeys;
@@ -102,14 +130,18 @@ __global__ __launch_bounds__(kThreads) void sort_histogram_kernel(
         }
 #pragma unroll
         for (int k = 0; k < kHistKeys; ++k) {
+            // Bits in which the warp's keys differ.
+            const uint64_t x = key[k] ^ __shfl_sync(kFullMask, key[k], 0);
             const bool full = __all_sync(kFullMask, valid[k]);
-            for (uint32_t p = 0; p < passes; ++p) {
-                const uint32_t shift = 8u * p;
-                const uint32_t bits = min(8u, key_bits - shift);
-                const uint32_t digit = (uint32_t)(key[k] >> shift) & ((1u << bits) - 1u);
-                const bool same =
-                    full && __all_sync(kFullMask, digit == __shfl_sync(kFullMask, digit, 0));
-                if (same) {
+            const uint32_t dlo = __reduce_or_sync(kFullMask, full ? (uint32_t)x : ~0u);
+            const uint32_t dhi = __reduce_or_sync(kFullMask, full ? (uint32_t)(x >> 32) : ~0u);
+#pragma unroll
+            for (uint32_t p = 0; p < kMaxPasses; ++p) {
+                if (p >= passes) break;
+                const uint32_t dmask = p + 1 == passes ? last_mask : 0xFFu;
+                const uint32_t digit = digit_of(key[k], 8u * p, dmask);
+                const uint32_t diff = digit_of((uint64_t)dhi << 32 | dlo, 8u * p, dmask);
+                if (diff == 0u) {
                     if (lane == 0) atomicAdd(&my_hist[p * kRadix + digit], 32u);
                 } else if (valid[k]) {
                     atomicAdd(&my_hist[p * kRadix + digit], 1u);
@@ -137,179 +169,224 @@ __global__ __launch_bounds__(kThreads) void sort_histogram_kernel(
 
 // The tile in sorted order for the scatter: keys with their values, or
 // (lean passes) keys with the tile-local index of their value.
-template <int kItems, bool kLean>
+template <int kTile, bool kLean>
 struct StageArrays {
-    uint64_t keys[kThreads * kItems];
-    uint32_t vals[kThreads * kItems];
+    uint64_t keys[kTile];
+    uint32_t vals[kTile];
 };
-template <int kItems>
-struct StageArrays<kItems, true> {
-    uint64_t keys[kThreads * kItems];
-    uint16_t src[kThreads * kItems];
+template <int kTile>
+struct StageArrays<kTile, true> {
+    uint64_t keys[kTile];
+    uint16_t src[kTile];
 };
 
-template <int kItems, bool kLean = false>
+template <int kBlock, int kItems, bool kLean = false>
 struct PassSmem {
-    static constexpr int kTile = kThreads * kItems;
-    union {
-        uint32_t warp_hist[kWarps][kRadix];  // ranking: per-warp digit counters
-        StageArrays<kItems, kLean> stage;    // scatter: the tile in sorted order
-    } u;
-    uint32_t tile_start[kRadix];   // first slot of each digit inside the tile
-    uint32_t global_base[kRadix];  // first output slot of each digit of this tile
-    uint32_t scan_tmp[kWarps];
-    uint32_t tile_id;
+    static constexpr int kTile = kBlock * kItems;
+    StageArrays<kTile, kLean> stage;            // the tile in sorted order
+    uint32_t warp_hist[kBlock / 32][kRadix];    // per-warp digit counts, then the next slot of each
+    uint32_t out_base[kRadix];  // first output slot of each digit less its first slot in the tile
+    uint32_t warp_sum[kWarps];
+    uint32_t next_tile;
 };
 
 __device__ __forceinline__ void prefetch_l2(const void* p) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
-// One onesweep pass. kItems pairs per thread; kMatch ranks with
-// __match_any_sync and one shared atomic per distinct digit, otherwise with
-// per-bit ballots and per-warp counters. kLean keeps no value in registers:
+// One onesweep pass. kItems pairs per thread, ranked with per-bit ballots and
+// per-warp counters. kLean keeps no value in registers:
 // the tile's values are prefetched into L2 when the keys are loaded and
 // gathered by their tile-local index (staged as 16 bits beside the key) in
 // the scatter, so fewer registers and less shared memory let more blocks
 // share an SM.
-template <int kItems, int kMinBlocks, bool kMatch, bool kLean = false>
-__global__ __launch_bounds__(kThreads, kMinBlocks) void sort_pass_kernel(
+//
+// A pass is a chain of latencies, not of bytes (384 MB at 16.7 M pairs are 59
+// us): the ticket, the loads, the ranking, the wait for the earlier tiles'
+// counts, the scatter. So the blocks stay (grid: what fits on the chip), and
+//  - the next tile's ticket is taken before the look-back and its keys are
+//    asked for before the scatter, so both arrive behind other work;
+//  - the digits are counted (one shared atomic a key) and published before the
+//    ranking, so that no look-back waits for another tile's ranking;
+//  - the ranking then yields final slots of the sorted tile, and the values are
+//    asked for behind it, to arrive during the look-back.
+// Tickets are taken in order and each block works on its lowest first: a
+// look-back only waits for tiles that running blocks hold and reach.
+// 16.7 M pairs of 63-bit keys: 156 us a pass -> 124 (20 keys a thread); 524,288:
+// 12.0 -> 10.2. What is left is spread over the phases: a warp's 32 keys cost an
+// SM about 26 cycles of ranking (the ballots' logic runs at half rate), 22 of
+// scattering and 8 of counting and staging, and the look-back 5,000 cycles a
+// tile. Tried: wider windows and a look-back inside the ranking (the words to
+// add up are the same, it only moves), blocks of 384 to 1,024 threads with
+// larger tiles (their warps rank at once and scatter at once: 130-150 us).
+template <int kBlock, int kItems, int kMinBlocks, bool kLean = false>
+__global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(
     const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
     uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
     const uint32_t* __restrict__ d_count, uint32_t n_est, const uint32_t* __restrict__ excl,
     uint32_t* __restrict__ lookback, uint32_t* __restrict__ tile_counter, uint32_t shift,
     uint32_t digit_bits, uint32_t* __restrict__ err, uint32_t spin_limit) {
-    using Smem = PassSmem<kItems, kLean>;
+    using Smem = PassSmem<kBlock, kItems, kLean>;
+    constexpr int kBlockWarps = kBlock / 32;
     constexpr int kTile = Smem::kTile;
     static_assert(kTile <= 65536, "tile-local indices fit 16 bits");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t n = d_count ? min(*d_count, n_est) : n_est;
-    if (tid == 0) sm.tile_id = atomicAdd(tile_counter, 1u);
-    for (uint32_t i = tid; i < kWarps * kRadix; i += kThreads) (&sm.u.warp_hist[0][0])[i] = 0;
-    __syncthreads();
-    const uint32_t tile = sm.tile_id;
-    const uint64_t tile_base = (uint64_t)tile * kTile;
-    if (tile_base >= n) return;
+    const uint32_t ntiles = n / kTile + (n % kTile != 0 ? 1u : 0u);
     const uint32_t dmask = (1u << digit_bits) - 1u;
     const uint32_t lt = lanemask_lt();
+    // Warp-striped: warp w owns a contiguous 32*kItems slice of a tile, item k of
+    // lane j sits at slice + 32k + j, so processing k in order keeps the ranking
+    // stable.
+    const uint32_t first = warp * 32u * kItems + lane;
+    uint32_t* my_hist = sm.warp_hist[warp];
 
-    // Warp-striped load: warp w owns a contiguous 32*kItems slice, item k of
-    // lane j sits at slice + 32k + j, so processing k in order keeps the
-    // ranking stable.
     uint64_t key[kItems];
-    uint32_t val[kLean ? 1 : kItems], pos[kItems];
-    const uint64_t warp_base = tile_base + (uint64_t)warp * 32 * kItems;
+    auto tile_len = [&](uint32_t t) { return min((uint32_t)kTile, n - t * (uint32_t)kTile); };
+    auto load_keys = [&](uint32_t t) {
+        const uint64_t* src = keys_in + (size_t)t * kTile;
+        const uint32_t len = tile_len(t);
+        if (len == (uint32_t)kTile) {
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const uint64_t i = warp_base + 32ull * k + lane;
-        const bool valid = i < n;
-        key[k] = valid ? __ldcs(keys_in + i) : ~0ull;
+            for (int k = 0; k < kItems; ++k) key[k] = __ldcs(src + first + 32 * k);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) key[k] = first + 32u * k < len ? __ldcs(src + first + 32 * k) : ~0ull;
+        }
         if constexpr (kLean) {
-            // One prefetch per 32 values (a 128-byte line) of this item.
-            if (vals_in && lane == 0 && valid) prefetch_l2(vals_in + i);
-        } else {
-            val[k] = valid ? (vals_in ? __ldcs(vals_in + i) : (uint32_t)i) : 0u;
+            // One prefetch per 32 values (a 128-byte line) of each item.
+            if (vals_in && lane == 0)
+                for (int k = 0; k < kItems; ++k)
+                    if (first + 32u * k < len) prefetch_l2(vals_in + (size_t)t * kTile + first + 32 * k);
         }
-    }
+    };
+    // Whole tiles (all but the last) take a copy of the code without checks.
+    auto pass = [&](uint32_t tile, auto whole) {
+        constexpr bool kWhole = decltype(whole)::value;
+        const uint32_t tile_n = tile_len(tile), tile_base = tile * (uint32_t)kTile;
+        const uint32_t* tile_vals = vals_in ? vals_in + tile_base : nullptr;
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const uint64_t i = warp_base + 32ull * k + lane;
-        const bool valid = i < n;
-        const uint32_t digit = (uint32_t)(key[k] >> shift) & dmask;
-        if (kMatch) {
-            const uint32_t peers = __match_any_sync(kFullMask, valid ? digit : (256u + lane));
-            const uint32_t leader = 31u - __clz(peers);
-            uint32_t old = 0;
-            if (valid && lane == leader) old = atomicAdd(&sm.u.warp_hist[warp][digit], __popc(peers));
-            old = __shfl_sync(kFullMask, old, leader);
-            pos[k] = old + __popc(peers & lt);
-        } else {
-            const uint32_t peers = peer_mask(digit, digit_bits, __ballot_sync(kFullMask, valid));
-            const uint32_t lower = __popc(peers & lt), cnt = __popc(peers);
-            uint32_t old = 0;
-            if (valid) old = sm.u.warp_hist[warp][digit];
-            __syncwarp();
-            if (valid && lower + 1 == cnt) sm.u.warp_hist[warp][digit] = old + cnt;
-            __syncwarp();
-            pos[k] = old + lower;
-        }
-    }
-    __syncthreads();
+        for (int k = 0; k < kItems; ++k)
+            if (kWhole || first + 32u * k < tile_n) atomicAdd(&my_hist[digit_of(key[k], shift, dmask)], 1u);
+        __syncthreads();
 
-    // Thread d owns digit d: per-warp exclusive offsets and the tile count.
-    uint32_t tile_cnt = 0;
+        // Thread d < 256 owns digit d: the tile's count, then the first slot of
+        // each warp's keys of the digit inside the sorted tile.
+        uint32_t* my_word = lookback + (size_t)tile * kRadix + tid;
+        uint32_t tile_cnt = 0, tile_start = 0;
+        if (tid < kRadix) {
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-        uint32_t c = sm.u.warp_hist[w][tid];
-        sm.u.warp_hist[w][tid] = tile_cnt;
-        tile_cnt += c;
-    }
-    uint32_t* my_word = lookback + (size_t)tile * kRadix + tid;
-    st_relaxed_u32(my_word, (tile == 0 ? kLbInclusive : kLbAggregate) | tile_cnt);
-    const uint32_t tile_start = block_exclusive_scan(tile_cnt, sm.scan_tmp);
-    sm.tile_start[tid] = tile_start;
-    __syncthreads();
-
-    // The tile is staged in sorted order before the look-back: staging needs
-    // only tile-local offsets, and the time it takes is slack in which the
-    // earlier tiles publish their counts.
+            for (int w = 0; w < kBlockWarps; ++w) tile_cnt += sm.warp_hist[w][tid];
+            st_relaxed_u32(my_word, (tile == 0 ? kLbInclusive : kLbAggregate) | tile_cnt);
+            tile_start = tile_cnt;
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const uint32_t digit = (uint32_t)(key[k] >> shift) & dmask;
-        pos[k] += sm.tile_start[digit] + sm.u.warp_hist[warp][digit];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const uint64_t i = warp_base + 32ull * k + lane;
-        if (i < n) {
-            sm.u.stage.keys[pos[k]] = key[k];
-            if constexpr (kLean)
-                sm.u.stage.src[pos[k]] = (uint16_t)(warp * 32u * kItems + 32u * k + lane);
-            else
-                sm.u.stage.vals[pos[k]] = val[k];
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFullMask, tile_start, o);
+                if (lane >= (uint32_t)o) tile_start += y;
+            }
+            if (lane == 31) sm.warp_sum[warp] = tile_start;
+            tile_start -= tile_cnt;
         }
-    }
-    uint32_t prefix = 0;
-    if (tile > 0) {
-        prefix = lookback_window(lookback, tile, tid, err, kRadix, spin_limit);
-        st_relaxed_u32(my_word, kLbInclusive | (prefix + tile_cnt));
-    }
-    sm.global_base[tid] = excl[tid] + prefix;
-    __syncthreads();
-    const uint32_t tile_n = (uint32_t)min((uint64_t)kTile, (uint64_t)n - tile_base);
-    if constexpr (kLean) {
-        // Gather every value of this thread's slots first (independent
-        // loads in flight), then store.
-        uint32_t v[kItems];
+        __syncthreads();
+        if (tid < kRadix) {
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const uint32_t i = tid + (uint32_t)k * kThreads;
-            const uint32_t sidx = i < tile_n ? (uint32_t)sm.u.stage.src[i] : 0u;
-            v[k] = i < tile_n ? (vals_in ? __ldcs(vals_in + tile_base + sidx) : (uint32_t)(tile_base + sidx))
-                              : 0u;
-        }
+            for (int w = 0; w < kWarps; ++w) tile_start += w < (int)warp ? sm.warp_sum[w] : 0u;
+            uint32_t run = tile_start;
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const uint32_t i = tid + (uint32_t)k * kThreads;
-            if (i < tile_n) {
-                const uint64_t key_i = sm.u.stage.keys[i];
-                const uint32_t digit = (uint32_t)(key_i >> shift) & dmask;
-                const uint32_t o = sm.global_base[digit] + (i - sm.tile_start[digit]);
-                keys_out[o] = key_i;
-                vals_out[o] = v[k];
+            for (int w = 0; w < kBlockWarps; ++w) {
+                const uint32_t c = sm.warp_hist[w][tid];
+                sm.warp_hist[w][tid] = run;
+                run += c;
             }
         }
-    } else {
-        for (uint32_t i = tid; i < tile_n; i += kThreads) {
-            const uint64_t k = sm.u.stage.keys[i];
-            const uint32_t digit = (uint32_t)(k >> shift) & dmask;
-            const uint32_t o = sm.global_base[digit] + (i - sm.tile_start[digit]);
-            keys_out[o] = k;
-            vals_out[o] = sm.u.stage.vals[i];
+        __syncthreads();
+
+        uint32_t val[kLean ? 1 : kItems], pos[kItems];
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            const bool valid = kWhole || first + 32u * k < tile_n;
+            const uint32_t vmask = kWhole ? kFullMask : __ballot_sync(kFullMask, valid);
+            pos[k] = warp_rank(my_hist, digit_of(key[k], shift, dmask), valid, vmask, lane, lt);
         }
+        if constexpr (!kLean) {
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) {
+                const uint32_t i = first + 32u * k;
+                val[k] = (kWhole || i < tile_n) ? (tile_vals ? __ldcs(tile_vals + i) : tile_base + i) : 0u;
+            }
+        }
+        if (tid < kRadix) {
+            uint32_t prefix = 0;
+            if (tile > 0) {
+                prefix = lookback_window(lookback, tile, tid, err, kRadix, spin_limit);
+                st_relaxed_u32(my_word, kLbInclusive | (prefix + tile_cnt));
+            }
+            // Slot i of the tile goes to out_base[its digit] + i (modulo 2^32).
+            sm.out_base[tid] = excl[tid] + prefix - tile_start;
+        }
+        if (tid == 0) sm.next_tile = atomicAdd(tile_counter, 1u);
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            if (kWhole || first + 32u * k < tile_n) {
+                sm.stage.keys[pos[k]] = key[k];
+                if constexpr (kLean) sm.stage.src[pos[k]] = (uint16_t)(first + 32u * k);
+                else sm.stage.vals[pos[k]] = val[k];
+            }
+        }
+        __syncthreads();
+        const uint32_t next = sm.next_tile;
+        if (next < ntiles) load_keys(next);
+        if constexpr (kLean) {
+            // Gather every value of this thread's slots first (independent
+            // loads in flight), then store.
+            uint32_t v[kItems];
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) {
+                const uint32_t i = tid + (uint32_t)k * kBlock;
+                v[k] = 0u;
+                if (kWhole || i < tile_n) {
+                    const uint32_t src = sm.stage.src[i];
+                    v[k] = tile_vals ? __ldcs(tile_vals + src) : tile_base + src;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) {
+                const uint32_t i = tid + (uint32_t)k * kBlock;
+                if (kWhole || i < tile_n) {
+                    const uint64_t key_i = sm.stage.keys[i];
+                    const uint32_t o = sm.out_base[digit_of(key_i, shift, dmask)] + i;
+                    keys_out[o] = key_i;
+                    vals_out[o] = v[k];
+                }
+            }
+        } else {
+#pragma unroll(kWhole ? kItems : 1)
+            for (int k = 0; k < kItems; ++k) {
+                const uint32_t i = tid + (uint32_t)k * kBlock;
+                if (kWhole || i < tile_n) {
+                    const uint64_t key_i = sm.stage.keys[i];
+                    const uint32_t o = sm.out_base[digit_of(key_i, shift, dmask)] + i;
+                    keys_out[o] = key_i;
+                    vals_out[o] = sm.stage.vals[i];
+                }
+            }
+        }
+        return next;
+    };
+
+    if (tid == 0) sm.next_tile = atomicAdd(tile_counter, 1u);
+    __syncthreads();
+    uint32_t tile = sm.next_tile;
+    if (tile >= ntiles) return;
+    load_keys(tile);
+    while (true) {
+#pragma unroll
+        for (int w = 0; w < 8; ++w) my_hist[32 * w + lane] = 0;
+        __syncthreads();  // the stage and the counters are free
+        tile = tile_len(tile) == (uint32_t)kTile ? pass(tile, std::true_type{}) : pass(tile, std::false_type{});
+        if (tile >= ntiles) return;
     }
 }
 
@@ -457,17 +534,9 @@ __global__ __launch_bounds__(kThreads, kMinBlocks) void sort_pass_pipelined_kern
         // Ranking with per-bit ballots, in item order (stable).
 #pragma unroll
         for (int k = 0; k < kItems; ++k) {
-            const uint64_t i = tile_base + warp_off + 32ull * k + lane;
-            const bool valid = i < n;
-            const uint32_t digit = (uint32_t)(key[k] >> shift) & dmask;
-            const uint32_t peers = peer_mask(digit, digit_bits, __ballot_sync(kFullMask, valid));
-            const uint32_t lower = __popc(peers & lt), cnt = __popc(peers);
-            uint32_t old = 0;
-            if (valid) old = sm.warp_hist[warp][digit];
-            __syncwarp();
-            if (valid && lower + 1 == cnt) sm.warp_hist[warp][digit] = old + cnt;
-            __syncwarp();
-            pos[k] = old + lower;
+            const bool valid = tile_base + warp_off + 32ull * k + lane < n;
+            pos[k] = warp_rank(sm.warp_hist[warp], digit_of(key[k], shift, dmask), valid,
+                                      __ballot_sync(kFullMask, valid), lane, lt);
         }
         __syncthreads();
         uint32_t tile_cnt = 0;
@@ -490,7 +559,7 @@ __global__ __launch_bounds__(kThreads, kMinBlocks) void sort_pass_pipelined_kern
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < kItems; ++k) {
-            const uint32_t digit = (uint32_t)(key[k] >> shift) & dmask;
+            const uint32_t digit = digit_of(key[k], shift, dmask);
             pos[k] += sm.tile_start[digit] + sm.warp_hist[warp][digit];
         }
         // The current buffer is free (its contents are in registers): stage
@@ -507,7 +576,7 @@ __global__ __launch_bounds__(kThreads, kMinBlocks) void sort_pass_pipelined_kern
         const uint32_t tile_n = (uint32_t)min((uint64_t)kTile, (uint64_t)n - tile_base);
         for (uint32_t i = tid; i < tile_n; i += kThreads) {
             const uint64_t kk = sm.keys[b][i];
-            const uint32_t digit = (uint32_t)(kk >> shift) & dmask;
+            const uint32_t digit = digit_of(kk, shift, dmask);
             const uint32_t o = sm.global_base[digit] + (i - sm.tile_start[digit]);
             keys_out[o] = kk;
             vals_out[o] = sm.vals[b][i];
@@ -523,40 +592,46 @@ __global__ __launch_bounds__(kThreads, kMinBlocks) void sort_pass_pipelined_kern
         if ((pending >> k) & 1u) mbar_wait(&sm.bar[k], (phase >> k) & 1u, err, spin_limit);
 }
 
-// Pass-kernel variants (items per thread, blocks per SM, ranking; the
-// pipelined ones run persistent blocks and need 16-byte aligned inputs).
+// Pass-kernel variants (threads, items per thread, blocks per SM; the pipelined
+// ones copy the next tile in bulk and need 16-byte aligned inputs).
 struct PassVariant {
-    int items;
+    int threads, items;
     void (*kernel)(const uint64_t*, const uint32_t*, uint64_t*, uint32_t*, const uint32_t*, uint32_t,
                    const uint32_t*, uint32_t*, uint32_t*, uint32_t, uint32_t, uint32_t*, uint32_t);
     size_t smem;
     bool pipelined;
 };
 const PassVariant kVariants[] = {
-    {16, sort_pass_kernel<16, 2, false>, sizeof(PassSmem<16>), false},
-    {16, sort_pass_kernel<16, 2, true>, sizeof(PassSmem<16>), false},
-    {12, sort_pass_kernel<12, 3, true>, sizeof(PassSmem<12>), false},
-    {8, sort_pass_kernel<8, 4, true>, sizeof(PassSmem<8>), false},
-    {20, sort_pass_kernel<20, 2, true>, sizeof(PassSmem<20>), false},
-    {12, sort_pass_kernel<12, 3, false>, sizeof(PassSmem<12>), false},
-    {8, sort_pass_kernel<8, 4, false>, sizeof(PassSmem<8>), false},
-    {12, sort_pass_pipelined_kernel<12, 2>, sizeof(PipeSmem<12>), true},
-    {8, sort_pass_pipelined_kernel<8, 3>, sizeof(PipeSmem<8>), true},
-    {12, sort_pass_kernel<12, 4, false, true>, sizeof(PassSmem<12, true>), false},
-    {16, sort_pass_kernel<16, 3, false, true>, sizeof(PassSmem<16, true>), false},
-    {20, sort_pass_kernel<20, 3, true, true>, sizeof(PassSmem<20, true>), false},
+    {256, 16, sort_pass_kernel<256, 16, 2>, sizeof(PassSmem<256, 16>), false},
+    {384, 12, sort_pass_kernel<384, 12, 2>, sizeof(PassSmem<384, 12>), false},
+    {512, 12, sort_pass_kernel<512, 12, 1>, sizeof(PassSmem<512, 12>), false},
+    {256, 8, sort_pass_kernel<256, 8, 4>, sizeof(PassSmem<256, 8>), false},
+    {256, 20, sort_pass_kernel<256, 20, 2>, sizeof(PassSmem<256, 20>), false},
+    {256, 12, sort_pass_kernel<256, 12, 3>, sizeof(PassSmem<256, 12>), false},
+    {256, 8, sort_pass_kernel<256, 8, 3>, sizeof(PassSmem<256, 8>), false},
+    {256, 12, sort_pass_pipelined_kernel<12, 2>, sizeof(PipeSmem<12>), true},
+    {256, 8, sort_pass_pipelined_kernel<8, 3>, sizeof(PipeSmem<8>), true},
+    {256, 12, sort_pass_kernel<256, 12, 4, true>, sizeof(PassSmem<256, 12, true>), false},
+    {256, 16, sort_pass_kernel<256, 16, 3, true>, sizeof(PassSmem<256, 16, true>), false},
+    {256, 20, sort_pass_kernel<256, 20, 2, true>, sizeof(PassSmem<256, 20, true>), false},
 };
 constexpr int kFallbackVariant = 5;  // for inputs a pipelined variant cannot copy
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 constexpr int kMinItems = 8;  // sizes the look-back words for every variant
 static_assert(kThreads * kMinItems == (int)kSortPlanTile, "look-back sizing");
-int g_variant = 5;
+int g_variant = -1;  // the variant that serves where the caller names none; negative: by the number of pairs
+// Small tiles while they all run at once, then fewer and larger ones, which have
+// fewer earlier tiles to look back on. 63-bit keys, 8 / 16 / 20 a thread, us:
+// 262,144 pairs 104 / 120 / 119; 524,288 125 / 126 / 125; 2,097,152 268 / 236 /
+// 253; 16,777,216 1256 / 1128 / 1091.
+int variant_for(uint32_t n) { return n < (1u << 19) ? 3 : (n < (1u << 23) ? 0 : 4); }
 
 // Per-device set-up state: the pass kernels' shared-memory attribute is set
 // once on each device that sorts, and the SM count is cached per device.
 constexpr int kMaxDevices = 64;
 bool g_init_done[kMaxDevices] = {};
 int g_num_sms[kMaxDevices] = {};
+int g_resident[kMaxDevices][kNumVariants] = {};  // blocks of each pass kernel the device holds
 std::mutex g_init_mutex;
 
 int current_device() {
@@ -596,6 +671,12 @@ cudaError_t sort_init() {
         e = cudaFuncSetAttribute(kVariants[v].kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kVariants[v].smem);
         if (e != cudaSuccess) return e;
+        int per_sm = 0, sms = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kVariants[v].kernel, kVariants[v].threads,
+                                                          kVariants[v].smem);
+        if (e != cudaSuccess) return e;
+        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+        g_resident[dev][v] = std::max(1, per_sm * sms);
     }
     // Tuning knob for benchmarks: ASTRO_SORT_VARIANT selects a pass variant.
     if (const char* env = getenv("ASTRO_SORT_VARIANT")) {
@@ -663,7 +744,7 @@ cudaError_t sort_launch(const uint64_t* keys_in, const uint32_t* vals_in, uint64
                           reinterpret_cast<uint32_t*>(t + plan.vals_tmp), n_est, d_count, key_bits,
                           current_device(), st, own);
     }
-    int vi = variant == 0 ? g_variant : (int)variant - 1;
+    int vi = variant != 0 ? (int)variant - 1 : (g_variant >= 0 ? g_variant : variant_for(n_est));
     // Bulk copies need 16-byte aligned sources; the temporaries always are.
     // The stalled test pass needs one block per tile (no persistent blocks).
     if (kVariants[vi].pipelined &&
@@ -671,16 +752,9 @@ cudaError_t sort_launch(const uint64_t* keys_in, const uint32_t* vals_in, uint64
          (((uintptr_t)keys_in | (uintptr_t)(vals_in ? vals_in : nullptr)) & 15u) != 0))
         vi = kFallbackVariant;
     const PassVariant& pv = kVariants[vi];
-    const uint32_t tile = (uint32_t)(kThreads * pv.items);
+    const uint32_t tile = (uint32_t)(pv.threads * pv.items);
     const uint32_t ntiles = (uint32_t)(((uint64_t)n_est + tile - 1) / tile);
-    uint32_t grid = ntiles;
-    if (pv.pipelined) {
-        int per_sm = 0;
-        cudaError_t eo = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pv.kernel, kThreads,
-                                                                       pv.smem);
-        if (eo != cudaSuccess) return eo;
-        grid = std::min<uint32_t>(ntiles, (uint32_t)std::max(1, per_sm) * (uint32_t)num_sms());
-    }
+    const uint32_t grid = std::min(ntiles, (uint32_t)g_resident[current_device()][vi]);
     char* base = static_cast<char*>(temp);
     uint64_t* keys_tmp = reinterpret_cast<uint64_t*>(base + plan.keys_tmp);
     uint32_t* vals_tmp = reinterpret_cast<uint32_t*>(base + plan.vals_tmp);
@@ -709,7 +783,7 @@ cudaError_t sort_launch(const uint64_t* keys_in, const uint32_t* vals_in, uint64
         uint32_t* vout = to_out ? vals_out : vals_tmp;
         const uint32_t shift = 8u * p;
         const uint32_t bits = key_bits == 0 ? 0u : std::min(8u, key_bits - shift);
-        pv.kernel<<<grid, kThreads, pv.smem, st>>>(
+        pv.kernel<<<grid, pv.threads, pv.smem, st>>>(
             kin, vin, kout, vout, d_count, n_est, excl + p * kRadix,
             lookback + (size_t)p * plan.ntiles * kRadix, counters + p, shift, bits, err, spin_limit);
         kin = kout;

@@ -177,17 +177,18 @@ typedef struct astro_params {
     uint32_t group_size;      /* PHYSICAL group walk: at most this many consecutive
                                  particles share one tree walk (one warp; two
                                  particles per lane above 32), 1..64; 0 = 32 */
-    uint32_t sort_variant;    /* radix sort pass kernel (items per thread / blocks
-                                 per SM / ranking): 0 = library default,
-                                 1 = 16/2/ballot, 2 = 16/2/match, 3 = 12/3/match,
-                                 4 = 8/4/match, 5 = 20/2/match, 6 = 12/3/ballot,
-                                 7 = 8/4/ballot; 8 = 12/2 and 9 = 8/3 ballot with
-                                 persistent blocks that bulk-copy the next tile
-                                 while ranking the current one (16-byte aligned
-                                 inputs; others use 6); lean passes that keep no
-                                 value in registers (values prefetched to L2 and
-                                 gathered by a staged 16-bit index): 10 =
-                                 12/4/ballot, 11 = 16/3/ballot, 12 = 20/3/match */
+    uint32_t sort_variant;    /* radix sort pass kernel (threads x items per
+                                 thread / blocks per SM): 0 = library default
+                                 (4, 1 or 5 by the number of pairs),
+                                 1 = 256x16/2, 2 = 384x12/2, 3 = 512x12/1,
+                                 4 = 256x8/4, 5 = 256x20/2, 6 = 256x12/3,
+                                 7 = 256x8/3; 8 = 256x12/2 and 9 = 256x8/3 that
+                                 bulk-copy the next tile while ranking the
+                                 current one (16-byte aligned inputs; others
+                                 use 6); lean passes that keep no value in
+                                 registers (values prefetched to L2 and gathered
+                                 by a staged 16-bit index): 10 = 256x12/4,
+                                 11 = 256x16/3, 12 = 256x20/2 */
     uint32_t light_sources;   /* REFERENCE: astro_step runs the lighting pass
                                  with the first light_sources particles (at most
                                  5) as lights (Renderer.swift:539; numStars = 5);
