@@ -13,6 +13,9 @@
 //      tile in sorted order in shared memory, obtains the counts of all
 //      earlier tiles by decoupled look-back (bounded waits), and writes each
 //      digit's run of the tile with contiguous stores.
+// Digits that all keys share are skipped, and where the top digits alone nearly
+// tell the keys apart only those are sorted, and the few keys that share them are
+// ordered in place of the remaining passes (see SortSchedule).
 // Few pairs are sorted in one launch instead (sort_small.cu).
 // A stable LSD sort yields the one stable permutation, so the result equals
 // the reference's bit by bit, including the order of equal keys.
@@ -31,7 +34,34 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kRadix = 256;
 constexpr int kMaxPasses = 8;
-constexpr int kHistBlocksPerSm = 8;
+constexpr int kHistBlocksPerSm = 4, kHistCopies = 4;
+
+// Words of the scratch's counter block: [8] histogram blocks done, [9] error
+// word, from kScheduleWord on the schedule, from kTicketWord on one ticket
+// counter a launch. All zero when a sort starts.
+constexpr uint32_t kDoneWord = 8, kScheduleWord = 10, kTicketWord = 16;
+// The schedule is worked out on the device by the last histogram block, which
+// knows the digit counts: word 0 holds the number m of digits that not all keys
+// share (at least 1) and in bits 8-15 the number of top digits to sort by (0: all
+// m, from the lowest up); word 1 the m digits, lowest first, four bits each;
+// word 4 is set when a run of keys that share their top digits was too long.
+//
+// Top digits: stable passes over the top kTopDigits digits, then ordering by
+// reading: a key finds its place among the others that share them, about
+// kNeighbours at most on average (fixup_kernel). Should a run be too long for
+// that, all m digits are sorted from the input after all.
+//
+// 63-bit keys without / with it: uniform ones, 1,500,000 194 / 172 us, 2,097,152
+// 226 / 190, 16,777,216 1005 / 628 (262,144 122 / 136, so not below kTopMin).
+// Keys of clustered particles do not qualify and pay for the question: 48 bits,
+// 1,500,000 158 / 185 us, 5,000,000 310 / 335. A fix-up that gives up costs its
+// passes: 4,194,304 351 -> 495. (Four or five top digits let clustered 63-bit keys
+// qualify, 5,000,000 399 -> 370 us, but some runs were too long: 690 us.)
+constexpr uint32_t kTopDigits = 3, kSavedPasses = 3;  // of at least 6 digits
+constexpr uint32_t kTopMin = 5u << 18;
+constexpr float kNeighbours = 4.f;
+constexpr uint32_t kSamples = 4096, kSampleSlots = 2 * kSamples;
+constexpr uint32_t kFixTile = 2048, kFixHalo = 128;
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -98,23 +128,70 @@ __device__ __forceinline__ uint32_t warp_rank(uint32_t* hist, uint32_t digit, bo
     return rank;
 }
 
-// All digit histograms in one read of the keys. Each warp counts into its own
-// shared-memory copy with atomics; a warp whose 32 keys share a digit (the
+// Place of sample k: spread over the input regardless of its order.
+__device__ __forceinline__ uint32_t sample_place(uint32_t k, uint32_t n) {
+    uint32_t h = (k + 1u) * 0x9E3779B1u;
+    h = (h ^ (h >> 15)) * 0x85EBCA77u;
+    h ^= h >> 13;
+    return __umulhi(h, n);
+}
+
+// Whether the digits from `shift` up leave a key about kNeighbours others with
+// the same ones: of S keys at random places, S^2 / 2 times the chance that two
+// keys agree do.
+__device__ __forceinline__ bool top_suffices(const uint64_t* samples, uint32_t n, uint32_t shift) {
+    extern __shared__ uint32_t slots[];  // hashes of prefixes; all ones: empty
+    __shared__ uint32_t s_equal;
+    const uint32_t tid = threadIdx.x;
+    __syncthreads();
+    if (tid == 0) s_equal = 0;
+#pragma unroll 1
+    for (uint32_t i = tid; i < kSampleSlots; i += kThreads) slots[i] = ~0u;
+    __syncthreads();
+    uint32_t equal = 0;
+    // (Not unrolled: one block runs this, and fetching 16 copies of the code took
+    // 45 us.)
+#pragma unroll 1
+    for (uint32_t k = tid; k < kSamples; k += kThreads) {
+        const uint64_t prefix = __ldcg(samples + k) >> shift;
+        const uint32_t id = min((uint32_t)((prefix * 0x9E3779B97F4A7C15ull) >> 32), ~1u);
+        uint32_t at = id & (kSampleSlots - 1u);
+        while (true) {  // half of the slots stay empty
+            const uint32_t was = atomicCAS(&slots[at], ~0u, id);
+            equal += was == id ? 1u : 0u;
+            if (was == ~0u || was == id) break;
+            at = (at + 1u) & (kSampleSlots - 1u);
+        }
+    }
+    equal = __reduce_add_sync(kFullMask, equal);
+    if ((tid & 31) == 0) atomicAdd(&s_equal, equal);
+    __syncthreads();
+    return (float)s_equal <= 0.5f * (float)kSamples * (float)kSamples * kNeighbours / (float)n + 4.f;
+}
+
+// All digit histograms in one read of the keys. Two warps share a copy of the
+// counters in shared memory, which they count into with atomics (16.7 M keys, 8
+// digits: 87 us against 97 with a copy for each, which left 24 warps an SM); a warp whose 32 keys share a digit (the
 // usual case for the high digits of Morton keys of a Morton-ordered state)
 // adds 32 with a single atomic.
-__global__ __launch_bounds__(kThreads) void sort_histogram_kernel(
+// The last block then schedules the passes.
+__global__ __launch_bounds__(kThreads, kHistBlocksPerSm) void sort_histogram_kernel(
     const uint64_t* __restrict__ keys, const uint32_t* __restrict__ d_count, uint32_t n_est,
     uint32_t key_bits, uint32_t passes, uint32_t* __restrict__ hist, uint32_t* __restrict__ excl,
-    uint32_t* __restrict__ done) {
-    extern __shared__ uint32_t s_hist[];  // [kWarps][passes][kRadix]
+    uint32_t* __restrict__ counters, bool skip_shared, bool try_top, uint64_t* __restrict__ samples) {
+    extern __shared__ uint32_t s_hist[];  // [kHistCopies][passes][kRadix]
     __shared__ uint32_t s_warp[kWarps];
     __shared__ bool s_last;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t n = d_count ? min(*d_count, n_est) : n_est;
-    const uint32_t per_warp = passes * kRadix;
-    for (uint32_t i = tid; i < kWarps * per_warp; i += kThreads) s_hist[i] = 0;
+    const uint32_t per_copy = passes * kRadix;
+    for (uint32_t i = tid; i < kHistCopies * per_copy; i += kThreads) s_hist[i] = 0;
     __syncthreads();
-    uint32_t* my_hist = s_hist + warp * per_warp;
+    // The first blocks fetch the samples, whose scattered reads would take the
+    // last block about 40 us (`samples`: the temporaries, unused until then).
+    if (try_top && n != 0u && blockIdx.x < kSamples / kThreads)
+        samples[blockIdx.x * kThreads + tid] = keys[sample_place(blockIdx.x * kThreads + tid, n)];
+    uint32_t* my_hist = s_hist + (warp % kHistCopies) * per_copy;
     const uint32_t last_mask = key_bits == 0 ? 0u : (1u << (key_bits - 8u * (passes - 1u))) - 1u;
     // Each thread takes kHistKeys keys per round (independent loads in flight).
     constexpr int kHistKeys = 4;
@@ -150,20 +227,43 @@ __global__ __launch_bounds__(kThreads) void sort_histogram_kernel(
         }
     }
     __syncthreads();
-    for (uint32_t i = tid; i < per_warp; i += kThreads) {
+    for (uint32_t i = tid; i < per_copy; i += kThreads) {
         uint32_t c = 0;
-        for (int w = 0; w < kWarps; ++w) c += s_hist[w * per_warp + i];
+        for (int w = 0; w < kHistCopies; ++w) c += s_hist[w * per_copy + i];
         if (c) atomicAdd(&hist[i], c);
     }
     __threadfence();
     __syncthreads();
-    if (tid == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    if (tid == 0) s_last = atomicAdd(counters + kDoneWord, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
+    __shared__ float s_agree[kMaxPasses];  // chance that two keys have the same digit
+    if (tid < kMaxPasses) s_agree[tid] = 0.f;
+    uint32_t m = 0, digits = 0;
+#pragma unroll 1
     for (uint32_t p = 0; p < passes; ++p) {
         uint32_t c = __ldcg(&hist[p * kRadix + tid]);
         excl[p * kRadix + tid] = block_exclusive_scan(c, s_warp);
+        float f = (float)c / (float)n;
+        f *= f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(kFullMask, f, o);
+        if (lane == 0) atomicAdd(&s_agree[p], f);
+        if (__syncthreads_or(c == n) == 0 || !skip_shared) digits |= p << (4u * m++);
+    }
+    if (m == 0) m = 1;  // equal keys: one pass copies them
+    uint32_t top = 0;
+    if (try_top && n >= kTopMin && m >= kTopDigits + kSavedPasses) {
+        const uint32_t lowest = (digits >> (4u * (m - kTopDigits))) & 15u;
+        float others = (float)n;  // if the digits were independent
+        for (uint32_t k = m - kTopDigits; k < m; ++k) others *= s_agree[(digits >> (4u * k)) & 15u];
+        // Keys of clustered particles share their digits far more often.
+        if (others <= 16.f * kNeighbours && top_suffices(samples, n, 8u * lowest)) top = kTopDigits;
+    }
+    if (tid == 0) {
+        counters[kScheduleWord] = m | (top << 8);
+        counters[kScheduleWord + 1] = digits;
     }
 }
 
@@ -179,6 +279,61 @@ struct StageArrays<kTile, true> {
     uint64_t keys[kTile];
     uint16_t src[kTile];
 };
+
+// What the launches of a sort share.
+struct SortArgs {
+    const uint64_t* keys_in;
+    const uint32_t* vals_in;  // null: the places 0, 1, ...
+    uint64_t *keys_tmp, *keys_out;
+    uint32_t *vals_tmp, *vals_out;
+    const uint32_t* d_count;
+    uint32_t n_est, key_bits;
+    const uint32_t* excl;
+    uint32_t* lookback;
+    size_t lookback_stride;  // words of one pass
+    uint32_t* counters;
+    uint32_t early;  // launches before the fix-up (0: no fix-up)
+    uint32_t* err;
+    uint32_t spin_limit;
+};
+// One pass: where from, where to, which digit.
+struct Pass {
+    const uint64_t* keys_in;
+    const uint32_t* vals_in;
+    uint64_t* keys_out;
+    uint32_t* vals_out;
+    const uint32_t* excl;
+    uint32_t* lookback;
+    uint32_t shift, digit_bits;
+};
+// The pass that launch `launch` has to run under the schedule; false: none. The
+// passes alternate between the temporaries and the output so that the last one
+// (or the fix-up) ends in the output.
+__device__ __forceinline__ bool pick_pass(const SortArgs& a, uint32_t launch, Pass& p) {
+    const uint32_t w = a.counters[kScheduleWord], digits = a.counters[kScheduleWord + 1];
+    const uint32_t m = w & 255u, top = w >> 8;
+    uint32_t i = launch, at = i, count = m, stages = m;
+    if (top != 0u && launch < a.early) {
+        count = top;
+        at = m - top + i;
+        stages = top + 1u;
+    } else if (top != 0u) {
+        if (a.counters[kScheduleWord + 4] == 0u) return false;
+        at = i -= a.early;
+    }
+    if (i >= count) return false;
+    const uint32_t digit = (digits >> (4u * at)) & 15u;
+    const bool to_out = ((stages - 1u - i) & 1u) == 0u;
+    p.keys_in = i == 0u ? a.keys_in : (to_out ? a.keys_tmp : a.keys_out);
+    p.vals_in = i == 0u ? a.vals_in : (to_out ? a.vals_tmp : a.vals_out);
+    p.keys_out = to_out ? a.keys_out : a.keys_tmp;
+    p.vals_out = to_out ? a.vals_out : a.vals_tmp;
+    p.excl = a.excl + digit * kRadix;
+    p.lookback = a.lookback + i * a.lookback_stride;
+    p.shift = 8u * digit;
+    p.digit_bits = min(8u, a.key_bits - min(a.key_bits, p.shift));
+    return true;
+}
 
 template <int kBlock, int kItems, bool kLean = false>
 struct PassSmem {
@@ -220,12 +375,7 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 // add up are the same, it only moves), blocks of 384 to 1,024 threads with
 // larger tiles (their warps rank at once and scatter at once: 130-150 us).
 template <int kBlock, int kItems, int kMinBlocks, bool kLean = false>
-__global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(
-    const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-    uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-    const uint32_t* __restrict__ d_count, uint32_t n_est, const uint32_t* __restrict__ excl,
-    uint32_t* __restrict__ lookback, uint32_t* __restrict__ tile_counter, uint32_t shift,
-    uint32_t digit_bits, uint32_t* __restrict__ err, uint32_t spin_limit) {
+__global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(SortArgs args, uint32_t launch) {
     using Smem = PassSmem<kBlock, kItems, kLean>;
     constexpr int kBlockWarps = kBlock / 32;
     constexpr int kTile = Smem::kTile;
@@ -233,7 +383,20 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t n = d_count ? min(*d_count, n_est) : n_est;
+    uint32_t* tile_counter = args.counters + kTicketWord + launch;
+    if (tid == 0) sm.next_tile = atomicAdd(tile_counter, 1u);
+    Pass pass_args;
+    if (!pick_pass(args, launch, pass_args)) return;
+    const uint64_t* __restrict__ keys_in = pass_args.keys_in;
+    const uint32_t* __restrict__ vals_in = pass_args.vals_in;
+    uint64_t* __restrict__ keys_out = pass_args.keys_out;
+    uint32_t* __restrict__ vals_out = pass_args.vals_out;
+    const uint32_t* excl = pass_args.excl;
+    uint32_t* lookback = pass_args.lookback;
+    const uint32_t shift = pass_args.shift, digit_bits = pass_args.digit_bits;
+    uint32_t* err = args.err;
+    const uint32_t spin_limit = args.spin_limit;
+    const uint32_t n = args.d_count ? min(*args.d_count, args.n_est) : args.n_est;
     const uint32_t ntiles = n / kTile + (n % kTile != 0 ? 1u : 0u);
     const uint32_t dmask = (1u << digit_bits) - 1u;
     const uint32_t lt = lanemask_lt();
@@ -303,7 +466,8 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(
         }
         __syncthreads();
 
-        uint32_t val[kLean ? 1 : kItems], pos[kItems];
+        [[maybe_unused]] uint32_t val[kLean ? 1 : kItems];
+        uint32_t pos[kItems];
 #pragma unroll
         for (int k = 0; k < kItems; ++k) {
             const bool valid = kWhole || first + 32u * k < tile_n;
@@ -376,7 +540,6 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(
         return next;
     };
 
-    if (tid == 0) sm.next_tile = atomicAdd(tile_counter, 1u);
     __syncthreads();
     uint32_t tile = sm.next_tile;
     if (tile >= ntiles) return;
@@ -456,18 +619,25 @@ struct PipeSmem {
 };
 
 template <int kItems, int kMinBlocks>
-__global__ __launch_bounds__(kThreads, kMinBlocks) void sort_pass_pipelined_kernel(
-    const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-    uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-    const uint32_t* __restrict__ d_count, uint32_t n_est, const uint32_t* __restrict__ excl,
-    uint32_t* __restrict__ lookback, uint32_t* __restrict__ tile_counter, uint32_t shift,
-    uint32_t digit_bits, uint32_t* __restrict__ err, uint32_t spin_limit) {
+__global__ __launch_bounds__(kThreads, kMinBlocks) void sort_pass_pipelined_kernel(SortArgs args, uint32_t launch) {
     using Smem = PipeSmem<kItems>;
     constexpr int kTile = Smem::kTile;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t n = d_count ? min(*d_count, n_est) : n_est;
+    Pass pass_args;
+    if (!pick_pass(args, launch, pass_args)) return;
+    const uint64_t* __restrict__ keys_in = pass_args.keys_in;
+    const uint32_t* __restrict__ vals_in = pass_args.vals_in;
+    uint64_t* __restrict__ keys_out = pass_args.keys_out;
+    uint32_t* __restrict__ vals_out = pass_args.vals_out;
+    const uint32_t* excl = pass_args.excl;
+    uint32_t* lookback = pass_args.lookback;
+    uint32_t* tile_counter = args.counters + kTicketWord + launch;
+    const uint32_t shift = pass_args.shift, digit_bits = pass_args.digit_bits;
+    uint32_t* err = args.err;
+    const uint32_t spin_limit = args.spin_limit;
+    const uint32_t n = args.d_count ? min(*args.d_count, args.n_est) : args.n_est;
     const uint32_t ntiles = (uint32_t)(((uint64_t)n + kTile - 1) / kTile);
     const uint32_t nfull = n / kTile;  // tiles fetched by bulk copies
     const uint32_t dmask = (1u << digit_bits) - 1u;
@@ -592,12 +762,81 @@ __global__ __launch_bounds__(kThreads, kMinBlocks) void sort_pass_pipelined_kern
         if ((pending >> k) & 1u) mbar_wait(&sm.bar[k], (phase >> k) & 1u, err, spin_limit);
 }
 
+// ------------------------------------------------------------- fix-up ----
+// Orders keys that are sorted, stably, by their top digits. Where a key's run (the neighbours that share these digits) begins
+// and ends is read off a bit mask of the runs' heads; its place is the run's
+// beginning plus the keys of the run that come before it. A run of more than
+// 2 kFixHalo keys, or one that reaches a halo's far edge, gives up (word 4).
+// 16.7 M pairs, two others a run on average: 109 us, bound by its instructions
+// (384 MB are 59 us); scanning left and right from each key 119 us.
+__global__ __launch_bounds__(kThreads) void fixup_kernel(SortArgs a) {
+    constexpr uint32_t kKeys = kFixTile + 2 * kFixHalo;
+    __shared__ uint64_t s_key[kKeys];
+    __shared__ uint32_t s_head[kKeys / 32];
+    static_assert(kKeys % kThreads == 0, "whole warps look for heads");
+    const uint32_t w = a.counters[kScheduleWord], digits = a.counters[kScheduleWord + 1];
+    const uint32_t m = w & 255u, top = w >> 8, tid = threadIdx.x;
+    if (top == 0u) return;
+    const uint32_t n = a.d_count ? min(*a.d_count, a.n_est) : a.n_est;
+    const uint32_t begin = blockIdx.x * kFixTile;
+    if (begin >= n) return;
+    uint32_t* failed = a.counters + kScheduleWord + 4;
+    const uint32_t shift = 8u * ((digits >> (4u * (m - top))) & 15u);
+    const uint32_t tile = min(kFixTile, n - begin);
+    const uint32_t lead = min(begin, kFixHalo), count = lead + tile + min(n - begin - tile, kFixHalo);
+    const uint64_t* src = a.keys_tmp + (begin - lead);
+#pragma unroll
+    for (uint32_t i = tid; i < kKeys; i += kThreads)
+        if (i < count) s_key[i] = __ldcs(src + i);
+    __syncthreads();
+#pragma unroll
+    for (uint32_t i = tid; i < kKeys; i += kThreads) {
+        const bool head = i >= count || i == 0u || ((s_key[i] ^ s_key[i - 1]) >> shift) != 0ull;
+        const uint32_t heads = __ballot_sync(kFullMask, head);
+        if ((tid & 31u) == 0u) s_head[i / 32u] = heads;
+    }
+    __syncthreads();
+    bool long_run = false;
+    for (uint32_t i = lead + tid; i < lead + tile; i += kThreads) {
+        const uint64_t key = s_key[i];
+        const uint32_t val = __ldcs(a.vals_tmp + (begin - lead) + i);
+        uint32_t word = i / 32u;
+        uint32_t bits = s_head[word] & (0xFFFFFFFFu >> (31u - (i & 31u)));
+        while (bits == 0u) bits = s_head[--word];  // entry 0 is a head
+        const uint32_t from = 32u * word + 31u - __clz(bits);
+        word = i / 32u;
+        bits = s_head[word] & ((0xFFFFFFFEu << (i & 31u)));
+        while (bits == 0u && ++word < kKeys / 32u) bits = s_head[word];
+        const uint32_t to = bits == 0u ? count : min(count, 32u * word + (uint32_t)__ffs(bits) - 1u);
+        uint32_t place = from;
+        if ((from == 0u && lead == kFixHalo) || (to == count && begin - lead + count < n) || to - from > 2u * kFixHalo) {
+            long_run = true;
+            place = i;
+        } else {
+            // Keys of a run differ by less than 2^56: the sign of a difference
+            // orders them. Equal keys before i count, those behind it do not.
+            for (uint32_t j = from; j < to; ++j)
+                place += (uint32_t)((s_key[j] - key - (j < i ? 1ull : 0ull)) >> 63);
+        }
+        a.keys_out[begin - lead + place] = key;
+        a.vals_out[begin - lead + place] = val;
+    }
+    if (long_run) atomicOr(failed, 1u);
+}
+
+// Empties the look-back words of the early passes when all digits have to be
+// sorted after all.
+__global__ __launch_bounds__(kThreads) void refill_kernel(SortArgs a, size_t words) {
+    if (a.counters[kScheduleWord + 4] == 0u) return;
+    for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < words; i += (size_t)gridDim.x * kThreads)
+        a.lookback[i] = 0u;
+}
+
 // Pass-kernel variants (threads, items per thread, blocks per SM; the pipelined
 // ones copy the next tile in bulk and need 16-byte aligned inputs).
 struct PassVariant {
     int threads, items;
-    void (*kernel)(const uint64_t*, const uint32_t*, uint64_t*, uint32_t*, const uint32_t*, uint32_t,
-                   const uint32_t*, uint32_t*, uint32_t*, uint32_t, uint32_t, uint32_t*, uint32_t);
+    void (*kernel)(SortArgs, uint32_t);
     size_t smem;
     bool pipelined;
 };
@@ -684,7 +923,7 @@ cudaError_t sort_init() {
         if (v >= 0 && v < kNumVariants) g_variant = v;
     }
     e = cudaFuncSetAttribute(sort_histogram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(kWarps * kMaxPasses * kRadix * sizeof(uint32_t)));
+                             (int)(kHistCopies * kMaxPasses * kRadix * sizeof(uint32_t)));
     if (e == cudaSuccess) e = sort_small_init(dev);
     if (e == cudaSuccess) g_init_done[dev] = true;
     return e;
@@ -698,12 +937,11 @@ SortPlan sort_plan(uint32_t max_len, uint32_t key_bits) {
     p.tile = kSortPlanTile;
     p.ntiles = (uint32_t)(((uint64_t)max_len + p.tile - 1) / p.tile);
     size_t off = 0;
-    // Zeroed at the start of every sort: counters ([0..7] tile tickets per
-    // pass, [8] histogram blocks done, [9] error word), histograms and
-    // look-back words.
+    // Zeroed at the start of every sort: counters (a block of 64 words),
+    // histograms and look-back words.
     p.zero_begin = off;
     p.counters = off;
-    off = align_up(off + 4ull * 16, 256);
+    off = align_up(off + 4ull * 64, 256);
     p.hist = off;
     off = align_up(off + 4ull * kMaxPasses * kRadix, 256);
     p.lookback = off;
@@ -720,6 +958,11 @@ SortPlan sort_plan(uint32_t max_len, uint32_t key_bits) {
 }
 
 namespace {
+
+bool overlaps(const void* a, size_t na, const void* b, size_t nb) {
+    const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+    return x < y + nb && y < x + na;
+}
 
 // The sort's kernels on the scratch `temp` (laid out by sort_plan). With
 // `stall_first_tile` (test hook, one pass only) the first pass hands out
@@ -766,28 +1009,34 @@ cudaError_t sort_launch(const uint64_t* keys_in, const uint32_t* vals_in, uint64
     cudaError_t e = cudaMemsetAsync(base + plan.zero_begin, 0, plan.zero_end - plan.zero_begin, st);
     if (e != cudaSuccess) return e;
     if (stall_first_tile) {
-        // Pass 0's ticket counter starts at 1 (its low byte set to 1).
-        e = cudaMemsetAsync(counters, 1, 1, st);
+        // The ticket counter starts at 1 (its low byte set to 1).
+        e = cudaMemsetAsync(counters + kTicketWord, 1, 1, st);
         if (e != cudaSuccess) return e;
     }
     const uint32_t hist_blocks = (uint32_t)std::min<uint64_t>(
         ((uint64_t)n_est + 4 * kThreads - 1) / (4 * kThreads), (uint64_t)num_sms() * kHistBlocksPerSm);
-    const size_t hist_smem = (size_t)kWarps * plan.passes * kRadix * sizeof(uint32_t);
-    sort_histogram_kernel<<<hist_blocks, kThreads, hist_smem, st>>>(keys_in, d_count, n_est, key_bits,
-                                                                    plan.passes, hist, excl, counters + 8);
-    const uint64_t* kin = keys_in;
-    const uint32_t* vin = vals_in;
-    for (uint32_t p = 0; p < plan.passes; ++p) {
-        const bool to_out = ((plan.passes - 1 - p) % 2) == 0;
-        uint64_t* kout = to_out ? keys_out : keys_tmp;
-        uint32_t* vout = to_out ? vals_out : vals_tmp;
-        const uint32_t shift = 8u * p;
-        const uint32_t bits = key_bits == 0 ? 0u : std::min(8u, key_bits - shift);
-        pv.kernel<<<grid, pv.threads, pv.smem, st>>>(
-            kin, vin, kout, vout, d_count, n_est, excl + p * kRadix,
-            lookback + (size_t)p * plan.ntiles * kRadix, counters + p, shift, bits, err, spin_limit);
-        kin = kout;
-        vin = vout;
+    // The passes may be reordered or left out only if no pass overwrites the
+    // input (a caller may sort in place with an even number of passes).
+    const bool apart = !overlaps(keys_in, 8ull * n_est, keys_out, 8ull * n_est) &&
+                       !(vals_in && overlaps(vals_in, 4ull * n_est, vals_out, 4ull * n_est)) && !stall_first_tile;
+    const bool try_top = apart && n_est >= kTopMin && plan.passes >= kTopDigits + kSavedPasses;
+    const uint32_t early = try_top ? kTopDigits : 0u;
+    const size_t hist_smem = std::max((size_t)kHistCopies * plan.passes * kRadix * sizeof(uint32_t),
+                                      try_top ? (size_t)kSampleSlots * sizeof(uint32_t) : (size_t)0);
+    sort_histogram_kernel<<<hist_blocks, kThreads, hist_smem, st>>>(keys_in, d_count, n_est, key_bits, plan.passes,
+                                                                    hist, excl, counters, apart, try_top, keys_tmp);
+    const size_t stride = (size_t)plan.ntiles * kRadix;
+    const SortArgs args{keys_in,  vals_in, keys_tmp, keys_out, vals_tmp, vals_out, d_count, n_est,
+                        key_bits, excl,    lookback, stride,   counters, early,    err,     spin_limit};
+    // Where the top digits may suffice: as many passes, the fix-up, and launches
+    // for all passes, which a schedule without top digits goes on with and a fix-up
+    // that gave up starts over with. A launch with nothing to do takes about 2 us.
+    for (uint32_t l = 0; l < plan.passes + early; ++l) {
+        if (try_top && l == early) {
+            fixup_kernel<<<(n_est - 1u) / kFixTile + 1u, kThreads, 0, st>>>(args);
+            refill_kernel<<<num_sms(), kThreads, 0, st>>>(args, plan.passes * stride);
+        }
+        pv.kernel<<<grid, pv.threads, pv.smem, st>>>(args, l);
     }
     return cudaGetLastError();
 }
