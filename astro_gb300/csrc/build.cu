@@ -59,11 +59,12 @@ __device__ __forceinline__ uint32_t quantise(float x, float lo, float scale) {
 // to pos here (x64 is the master copy).
 template <bool kPrec>
 __global__ __launch_bounds__(256) void encode_phys_kernel(const Chunk* __restrict__ chunks,
-                                                          const SysInfo* __restrict__ sys,
-                                                          float4* __restrict__ pos,
+                                                          const SysInfo* sys,
+                                                          float4* pos,
                                                           const double* __restrict__ x64,
-                                                          uint64_t* __restrict__ codes, uint32_t n,
+                                                          uint64_t* codes, uint32_t n,
                                                           uint32_t lbits) {
+    after_previous();
     const Chunk c = chunks[blockIdx.x];
     const SysInfo& s = sys[c.sys];
     const float lox = s.lo[0], loy = s.lo[1], loz = s.lo[2], scale = s.scale;
@@ -139,6 +140,7 @@ __global__ __launch_bounds__(256) void bbox_kernel(const Chunk* __restrict__ chu
                                                    const double* __restrict__ x64, uint32_t n,
                                                    uint32_t* __restrict__ bb32,
                                                    unsigned long long* __restrict__ bb64) {
+    after_previous();
     const Chunk c = chunks[blockIdx.x];
     if (kPrec) {
         unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
@@ -170,6 +172,7 @@ template <bool kPrec>
 __global__ void setup_kernel(SysInfo* __restrict__ sys, uint32_t nsys,
                              uint32_t* __restrict__ bb32, unsigned long long* __restrict__ bb64,
                              uint32_t lbits, float theta, uint32_t root_offset) {
+    after_previous();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nsys) return;
     SysInfo& info = sys[s];
@@ -213,11 +216,12 @@ __global__ void setup_kernel(SysInfo* __restrict__ sys, uint32_t nsys,
 
 // Permute the PHYSICAL state into the new Morton order (B <- A[perm]).
 template <bool kPrec>
-__global__ void reorder_kernel(const uint32_t* __restrict__ perm, const float4* __restrict__ pos_a,
+__global__ void reorder_kernel(const uint32_t* perm, const float4* __restrict__ pos_a,
                                const float4* __restrict__ vel_a, const uint32_t* __restrict__ id_a,
                                const double* __restrict__ x_a, float4* __restrict__ pos_b,
                                float4* __restrict__ vel_b, uint32_t* __restrict__ id_b,
                                double* __restrict__ x_b, uint32_t n, ClearArgs clear) {
+    after_previous();
     clear_scratch(clear);
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
@@ -257,6 +261,7 @@ constexpr uint32_t topo_items(uint32_t n) { return n <= kTopoSmall ? 2u : (n <= 
 // holds its first particle (the bottom-up aggregation climbs these links).
 template <int kTopoItems>
 __global__ __launch_bounds__(kTopoThreads) void topology_kernel(TopoArgs a) {
+    after_previous();
     constexpr int kTopoTile = kTopoThreads * kTopoItems;
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_off[ASTRO_MAX_LAYERS];
@@ -887,6 +892,7 @@ __device__ __forceinline__ void climb_chain(const AggArgs& a, uint32_t l, uint32
 
 template <bool kPrec, bool kQuad>
 __global__ __launch_bounds__(128) void aggregate_leaf_kernel(AggArgs a, uint32_t top, uint32_t work_top) {
+    after_previous();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t u0 = a.layer_count[0];
     NodeRec<kPrec> r;
@@ -901,6 +907,7 @@ __global__ __launch_bounds__(128) void aggregate_leaf_kernel(AggArgs a, uint32_t
 template <bool kPrec, bool kQuad, bool kWork>
 __global__ __launch_bounds__(128) void aggregate_internal_kernel(AggArgs a, uint32_t l, uint32_t top,
                                                                  uint32_t work_top) {
+    after_previous();
     const uint32_t u = a.layer_count[l], count = kWork ? a.work_count[l] : u;
     for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < count; i0 += gridDim.x * blockDim.x) {
         const uint32_t i = i0 + threadIdx.x;
@@ -1022,6 +1029,7 @@ __device__ __forceinline__ void aggregate_wide(const AggArgs& a, uint32_t l, uin
 constexpr uint32_t kTopThreads = 512;
 template <bool kPrec, bool kQuad>
 __global__ __launch_bounds__(kTopThreads, 1) void aggregate_top_kernel(AggArgs a, uint32_t l0) {
+    after_previous();
     using Sum = typename NodeRec<kPrec>::Sum;
     cg::cluster_group cluster = cg::this_cluster();
     // Consecutive warps of nodes go to different blocks.
@@ -1101,12 +1109,14 @@ __global__ __launch_bounds__(kTopThreads, 1) void aggregate_top_kernel(AggArgs a
 
 // One launch per large layer, the rest of the tree in one cluster.
 __global__ __launch_bounds__(128) void aggregate_ref_leaf_kernel(AggArgs a) {
+    after_previous();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t u0 = a.layer_count[0];
     if (j < u0) aggregate_ref_leaf(a, j, u0);
 }
 
 __global__ __launch_bounds__(128) void aggregate_ref_internal_kernel(AggArgs a, uint32_t l) {
+    after_previous();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t u = a.layer_count[l];
     if (j < u) aggregate_ref_internal(a, l, j, u);
@@ -1114,6 +1124,7 @@ __global__ __launch_bounds__(128) void aggregate_ref_internal_kernel(AggArgs a, 
 
 // Layers l0 and up in one launch of one cluster, as above.
 __global__ __launch_bounds__(kTopThreads, 1) void aggregate_ref_top_kernel(AggArgs a, uint32_t l0) {
+    after_previous();
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t first = ((threadIdx.x >> 5) * cluster.num_blocks() + cluster.block_rank()) * 32u +
                            (threadIdx.x & 31u);
@@ -1462,9 +1473,9 @@ cudaError_t launch_encode_phys(bool prec, const Chunk* chunks, uint32_t nchunks,
                                float4* pos, const double* x64, uint64_t* codes, uint32_t n,
                                uint32_t lbits, cudaStream_t st) {
     if (prec)
-        encode_phys_kernel<true><<<nchunks, 256, 0, st>>>(chunks, sys, pos, x64, codes, n, lbits);
+        return launch_after(encode_phys_kernel<true>, nchunks, 256, 0, st, chunks, sys, pos, x64, codes, n, lbits);
     else
-        encode_phys_kernel<false><<<nchunks, 256, 0, st>>>(chunks, sys, pos, x64, codes, n, lbits);
+        return launch_after(encode_phys_kernel<false>, nchunks, 256, 0, st, chunks, sys, pos, x64, codes, n, lbits);
     return cudaGetLastError();
 }
 
@@ -1480,10 +1491,10 @@ cudaError_t launch_setup(bool prec, SysInfo* sys, uint32_t nsys, uint32_t* bb32,
                          unsigned long long* bb64, uint32_t lbits, float theta, uint32_t root_offset,
                          cudaStream_t st) {
     if (prec)
-        setup_kernel<true><<<blocks_for(nsys, 128), 128, 0, st>>>(sys, nsys, bb32, bb64, lbits,
+        return launch_after(setup_kernel<true>, blocks_for(nsys, 128), 128, 0, st, sys, nsys, bb32, bb64, lbits,
                                                                   theta, root_offset);
     else
-        setup_kernel<false><<<blocks_for(nsys, 128), 128, 0, st>>>(sys, nsys, bb32, bb64, lbits,
+        return launch_after(setup_kernel<false>, blocks_for(nsys, 128), 128, 0, st, sys, nsys, bb32, bb64, lbits,
                                                                    theta, root_offset);
     return cudaGetLastError();
 }
@@ -1493,10 +1504,10 @@ cudaError_t launch_reorder(bool prec, const uint32_t* perm, const float4* pos_a,
                            uint32_t* id_b, double* x_b, uint32_t n, const ClearArgs& clear,
                            cudaStream_t st) {
     if (prec)
-        reorder_kernel<true><<<blocks_for(n, 256), 256, 0, st>>>(perm, pos_a, vel_a, id_a, x_a, pos_b,
+        return launch_after(reorder_kernel<true>, blocks_for(n, 256), 256, 0, st, perm, pos_a, vel_a, id_a, x_a, pos_b,
                                                                  vel_b, id_b, x_b, n, clear);
     else
-        reorder_kernel<false><<<blocks_for(n, 256), 256, 0, st>>>(perm, pos_a, vel_a, id_a, x_a, pos_b,
+        return launch_after(reorder_kernel<false>, blocks_for(n, 256), 256, 0, st, perm, pos_a, vel_a, id_a, x_a, pos_b,
                                                                   vel_b, id_b, x_b, n, clear);
     return cudaGetLastError();
 }
@@ -1511,9 +1522,9 @@ uint32_t topology_tiles_max(uint32_t max_n) {
 cudaError_t launch_topology(const TopoArgs& a, cudaStream_t st) {
     if (a.n == 0) return cudaSuccess;
     switch (topo_items(a.n)) {
-        case 2: topology_kernel<2><<<a.ntiles, kTopoThreads, 0, st>>>(a); break;
-        case 4: topology_kernel<4><<<a.ntiles, kTopoThreads, 0, st>>>(a); break;
-        default: topology_kernel<8><<<a.ntiles, kTopoThreads, 0, st>>>(a); break;
+        case 2: return launch_after(topology_kernel<2>, a.ntiles, kTopoThreads, 0, st, a);
+        case 4: return launch_after(topology_kernel<4>, a.ntiles, kTopoThreads, 0, st, a);
+        default: return launch_after(topology_kernel<8>, a.ntiles, kTopoThreads, 0, st, a);
     }
     return cudaGetLastError();
 }
@@ -1540,11 +1551,13 @@ void cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, uint32_t
     cfg->gridDim = dim3(blocks);
     cfg->blockDim = dim3(kTopThreads);
     cfg->stream = st;
-    attr->id = cudaLaunchAttributeClusterDimension;
-    attr->val.clusterDim.x = blocks;
-    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_after does
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg->attrs = attr;
-    cfg->numAttrs = 1;
+    cfg->numAttrs = 2;
 }
 
 cudaError_t launch_cluster(TopKernel kernel, const AggArgs& a, uint32_t l0, cudaStream_t st) {
@@ -1558,8 +1571,8 @@ cudaError_t launch_cluster(TopKernel kernel, const AggArgs& a, uint32_t l0, cuda
     }
     if (blocks == 0) return cudaErrorInvalidDevice;
     cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr;
-    cluster_config(&cfg, &attr, blocks, st);
+    cudaLaunchAttribute attr[2];
+    cluster_config(&cfg, attr, blocks, st);
     return cudaLaunchKernelEx(&cfg, kernel, a, l0);
 }
 
@@ -1572,11 +1585,13 @@ cudaError_t launch_physical(const AggArgs& a, const LayerTable& t, cudaStream_t 
     while (lw < l0 && t.size[lw] >= kWorkMinNodes) ++lw;
     for (uint32_t l = 0; l < l0; ++l) {
         const uint32_t g = blocks_for(t.size[l], t0);
-        if (l == 0) aggregate_leaf_kernel<kPrec, kQuad><<<g, t0, 0, st>>>(a, l0, lw);
+        cudaError_t e;
+        if (l == 0) e = launch_after(aggregate_leaf_kernel<kPrec, kQuad>, g, t0, 0, st, a, l0, lw);
         else if (l < lw)
-            aggregate_internal_kernel<kPrec, kQuad, true><<<std::min(g, kWorkBlocks), t0, 0, st>>>(a, l, l0, lw);
-        else
-            aggregate_internal_kernel<kPrec, kQuad, false><<<g, t0, 0, st>>>(a, l, l0, lw);
+            e = launch_after(aggregate_internal_kernel<kPrec, kQuad, true>, std::min(g, kWorkBlocks), t0, 0, st, a, l,
+                             l0, lw);
+        else e = launch_after(aggregate_internal_kernel<kPrec, kQuad, false>, g, t0, 0, st, a, l, l0, lw);
+        if (e != cudaSuccess) return e;
     }
     return launch_cluster(aggregate_top_kernel<kPrec, kQuad>, a, l0, st);
 }
@@ -1597,8 +1612,9 @@ cudaError_t build_init() {
         if (e != cudaSuccess) return e;
         for (; blocks > 1; blocks /= 2) {
             cudaLaunchConfig_t cfg;
-            cudaLaunchAttribute attr;
-            cluster_config(&cfg, &attr, blocks, nullptr);
+            cudaLaunchAttribute attr[2];
+            cluster_config(&cfg, attr, blocks, nullptr);
+            cfg.numAttrs = 1;
             int clusters = 0;
             if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) == cudaSuccess && clusters > 0) break;
             (void)cudaGetLastError();
@@ -1615,8 +1631,9 @@ cudaError_t launch_aggregate(int mode, const AggArgs& a, const LayerTable& t, cu
     const uint32_t l0 = top_first_layer(t);
     for (uint32_t l = 0; l < l0; ++l) {
         const uint32_t g = blocks_for(t.size[l], t0);
-        if (l == 0) aggregate_ref_leaf_kernel<<<g, t0, 0, st>>>(a);
-        else aggregate_ref_internal_kernel<<<g, t0, 0, st>>>(a, l);
+        const cudaError_t e = l == 0 ? launch_after(aggregate_ref_leaf_kernel, g, t0, 0, st, a)
+                                     : launch_after(aggregate_ref_internal_kernel, g, t0, 0, st, a, l);
+        if (e != cudaSuccess) return e;
     }
     return launch_cluster(aggregate_ref_top_kernel, a, l0, st);
 }

@@ -78,9 +78,10 @@ __device__ __forceinline__ uint32_t warps_before(const uint32_t* tmp, uint32_t w
 }
 
 __global__ __launch_bounds__(kMaxThreads, 1) void sort_small_kernel(
-    const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint64_t* keys_out,
-    uint32_t* vals_out, uint64_t* keys_tmp, uint32_t* vals_tmp, const uint32_t* __restrict__ d_count,
+    const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out,
+    uint32_t* vals_out, uint64_t* keys_tmp, uint32_t* vals_tmp, const uint32_t* d_count,
     uint32_t n_est, uint32_t key_bits, uint32_t slice, uint32_t* __restrict__ clear_err) {
+    after_previous();
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, warps = blockDim.x >> 5;
@@ -252,10 +253,11 @@ __global__ __launch_bounds__(kMaxThreads, 1) void sort_small_kernel(
 // elements, so those stages only need the warp.
 constexpr uint32_t kTinyThreads = 1024;
 __global__ __launch_bounds__(kTinyThreads, 1) void sort_tiny_kernel(
-    const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+    const uint64_t* keys_in, const uint32_t* vals_in,
     uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-    const uint32_t* __restrict__ d_count, uint32_t n_est, uint64_t mask, uint32_t size,
+    const uint32_t* d_count, uint32_t n_est, uint64_t mask, uint32_t size,
     uint32_t* __restrict__ clear_err) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* const keys = reinterpret_cast<uint64_t*>(smem_raw);
     uint32_t* const at = reinterpret_cast<uint32_t*>(keys + size);
@@ -264,7 +266,7 @@ __global__ __launch_bounds__(kTinyThreads, 1) void sort_tiny_kernel(
     if (clear_err && tid == 0) *clear_err = 0u;
     // Padding sorts behind every pair: the largest key, later positions.
     for (uint32_t i = tid; i < size; i += blockDim.x) {
-        keys[i] = i < n ? __ldg(keys_in + i) : ~0ull;
+        keys[i] = i < n ? keys_in[i] : ~0ull;
         at[i] = i;
     }
     __syncthreads();
@@ -288,7 +290,7 @@ __global__ __launch_bounds__(kTinyThreads, 1) void sort_tiny_kernel(
     }
     for (uint32_t i = tid; i < n; i += blockDim.x) {
         keys_out[i] = keys[i];
-        vals_out[i] = vals_in ? __ldg(vals_in + at[i]) : at[i];
+        vals_out[i] = vals_in ? vals_in[at[i]] : at[i];
     }
 }
 
@@ -302,11 +304,13 @@ cudaError_t launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, ui
     cfg->blockDim = dim3(threads);
     cfg->dynamicSmemBytes = small_smem(slice, threads);
     cfg->stream = st;
-    attr->id = cudaLaunchAttributeClusterDimension;
-    attr->val.clusterDim.x = blocks;
-    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_after does
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg->attrs = attr;
-    cfg->numAttrs = 1;
+    cfg->numAttrs = 2;
     return cudaSuccess;
 }
 
@@ -328,8 +332,9 @@ cudaError_t sort_small_init(int dev) {
     uint32_t size = 16;
     for (; size > 1; size /= 2) {
         cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute attr;
-        launch_config(&cfg, &attr, size, kMaxThreads, kMaxSlice, nullptr);
+        cudaLaunchAttribute attr[2];
+        launch_config(&cfg, attr, size, kMaxThreads, kMaxSlice, nullptr);
+        cfg.numAttrs = 1;
         int clusters = 0;
         if (cudaOccupancyMaxActiveClusters(&clusters, sort_small_kernel, &cfg) == cudaSuccess && clusters > 0)
             break;
@@ -359,9 +364,8 @@ cudaError_t sort_small(const uint64_t* keys_in, const uint32_t* vals_in, uint64_
         uint32_t size = 64;
         while (size < n_est) size *= 2u;
         const uint64_t mask = key_bits >= 64u ? ~0ull : (1ull << key_bits) - 1ull;
-        sort_tiny_kernel<<<1, std::min(kTinyThreads, size / 2u), size * 12u, st>>>(
-            keys_in, vals_in, keys_out, vals_out, d_count, n_est, mask, size, clear_err);
-        return cudaGetLastError();
+        return launch_after(sort_tiny_kernel, 1, std::min(kTinyThreads, size / 2u), size * 12u, st, keys_in, vals_in,
+                            keys_out, vals_out, d_count, n_est, mask, size, clear_err);
     }
     // About a thousand pairs a block, then more per block once the cluster is
     // full, in equal slices (a multiple of 32 pairs).
@@ -371,8 +375,8 @@ cudaError_t sort_small(const uint64_t* keys_in, const uint32_t* vals_in, uint64_
     if (slice > kMaxSlice) return cudaErrorInvalidValue;
     const uint32_t threads = small_threads(slice);
     cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr;
-    launch_config(&cfg, &attr, blocks, threads, slice, st);
+    cudaLaunchAttribute attr[2];
+    launch_config(&cfg, attr, blocks, threads, slice, st);
     return cudaLaunchKernelEx(&cfg, sort_small_kernel, keys_in, vals_in, keys_out, vals_out, keys_tmp,
                               vals_tmp, d_count, n_est, key_bits, slice, clear_err);
 }
