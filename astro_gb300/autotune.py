@@ -13,8 +13,8 @@ The knobs are fields of astro_params that change speed, not physics:
   lbits         tree depth, i.e. the depth of the walk (layers = lbits + 1)
   bucket        leaf tile size: an opened node holding <= bucket particles
                 is summed particle by particle
-  sort_variant  radix sort pass kernel (items per thread / blocks per SM /
-                ranking / pipelined / lean)
+  sort_variant  radix sort pass kernel (threads, items per thread, blocks per
+                SM)
   walk_frontier the group walk's frontier: runs of consecutive child nodes
                 or a list of node indices
 

@@ -267,19 +267,6 @@ __global__ __launch_bounds__(kThreads, kHistBlocksPerSm) void sort_histogram_ker
     }
 }
 
-// The tile in sorted order for the scatter: keys with their values, or
-// (lean passes) keys with the tile-local index of their value.
-template <int kTile, bool kLean>
-struct StageArrays {
-    uint64_t keys[kTile];
-    uint32_t vals[kTile];
-};
-template <int kTile>
-struct StageArrays<kTile, true> {
-    uint64_t keys[kTile];
-    uint16_t src[kTile];
-};
-
 // What the launches of a sort share.
 struct SortArgs {
     const uint64_t* keys_in;
@@ -335,26 +322,19 @@ __device__ __forceinline__ bool pick_pass(const SortArgs& a, uint32_t launch, Pa
     return true;
 }
 
-template <int kBlock, int kItems, bool kLean = false>
+template <int kBlock, int kItems>
 struct PassSmem {
     static constexpr int kTile = kBlock * kItems;
-    StageArrays<kTile, kLean> stage;            // the tile in sorted order
-    uint32_t warp_hist[kBlock / 32][kRadix];    // per-warp digit counts, then the next slot of each
+    uint64_t keys[kTile];  // the tile in sorted order
+    uint32_t vals[kTile];
+    uint32_t warp_hist[kBlock / 32][kRadix];  // per-warp digit counts, then the next slot of each
     uint32_t out_base[kRadix];  // first output slot of each digit less its first slot in the tile
     uint32_t warp_sum[kWarps];
     uint32_t next_tile;
 };
 
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
 // One onesweep pass. kItems pairs per thread, ranked with per-bit ballots and
-// per-warp counters. kLean keeps no value in registers:
-// the tile's values are prefetched into L2 when the keys are loaded and
-// gathered by their tile-local index (staged as 16 bits beside the key) in
-// the scatter, so fewer registers and less shared memory let more blocks
-// share an SM.
+// per-warp counters.
 //
 // A pass is a chain of latencies, not of bytes (384 MB at 16.7 M pairs are 59
 // us): the ticket, the loads, the ranking, the wait for the earlier tiles'
@@ -374,9 +354,9 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 // tile. Tried: wider windows and a look-back inside the ranking (the words to
 // add up are the same, it only moves), blocks of 384 to 1,024 threads with
 // larger tiles (their warps rank at once and scatter at once: 130-150 us).
-template <int kBlock, int kItems, int kMinBlocks, bool kLean = false>
+template <int kBlock, int kItems, int kMinBlocks>
 __global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(SortArgs args, uint32_t launch) {
-    using Smem = PassSmem<kBlock, kItems, kLean>;
+    using Smem = PassSmem<kBlock, kItems>;
     constexpr int kBlockWarps = kBlock / 32;
     constexpr int kTile = Smem::kTile;
     static_assert(kTile <= 65536, "tile-local indices fit 16 bits");
@@ -417,12 +397,6 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(SortArgs 
         } else {
 #pragma unroll
             for (int k = 0; k < kItems; ++k) key[k] = first + 32u * k < len ? __ldcs(src + first + 32 * k) : ~0ull;
-        }
-        if constexpr (kLean) {
-            // One prefetch per 32 values (a 128-byte line) of each item.
-            if (vals_in && lane == 0)
-                for (int k = 0; k < kItems; ++k)
-                    if (first + 32u * k < len) prefetch_l2(vals_in + (size_t)t * kTile + first + 32 * k);
         }
     };
     // Whole tiles (all but the last) take a copy of the code without checks.
@@ -466,20 +440,17 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(SortArgs 
         }
         __syncthreads();
 
-        [[maybe_unused]] uint32_t val[kLean ? 1 : kItems];
-        uint32_t pos[kItems];
+        uint32_t val[kItems], pos[kItems];
 #pragma unroll
         for (int k = 0; k < kItems; ++k) {
             const bool valid = kWhole || first + 32u * k < tile_n;
             const uint32_t vmask = kWhole ? kFullMask : __ballot_sync(kFullMask, valid);
             pos[k] = warp_rank(my_hist, digit_of(key[k], shift, dmask), valid, vmask, lane, lt);
         }
-        if constexpr (!kLean) {
 #pragma unroll
-            for (int k = 0; k < kItems; ++k) {
-                const uint32_t i = first + 32u * k;
-                val[k] = (kWhole || i < tile_n) ? (tile_vals ? __ldcs(tile_vals + i) : tile_base + i) : 0u;
-            }
+        for (int k = 0; k < kItems; ++k) {
+            const uint32_t i = first + 32u * k;
+            val[k] = (kWhole || i < tile_n) ? (tile_vals ? __ldcs(tile_vals + i) : tile_base + i) : 0u;
         }
         if (tid < kRadix) {
             uint32_t prefix = 0;
@@ -494,47 +465,21 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(SortArgs 
 #pragma unroll
         for (int k = 0; k < kItems; ++k) {
             if (kWhole || first + 32u * k < tile_n) {
-                sm.stage.keys[pos[k]] = key[k];
-                if constexpr (kLean) sm.stage.src[pos[k]] = (uint16_t)(first + 32u * k);
-                else sm.stage.vals[pos[k]] = val[k];
+                sm.keys[pos[k]] = key[k];
+                sm.vals[pos[k]] = val[k];
             }
         }
         __syncthreads();
         const uint32_t next = sm.next_tile;
         if (next < ntiles) load_keys(next);
-        if constexpr (kLean) {
-            // Gather every value of this thread's slots first (independent
-            // loads in flight), then store.
-            uint32_t v[kItems];
-#pragma unroll
-            for (int k = 0; k < kItems; ++k) {
-                const uint32_t i = tid + (uint32_t)k * kBlock;
-                v[k] = 0u;
-                if (kWhole || i < tile_n) {
-                    const uint32_t src = sm.stage.src[i];
-                    v[k] = tile_vals ? __ldcs(tile_vals + src) : tile_base + src;
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kItems; ++k) {
-                const uint32_t i = tid + (uint32_t)k * kBlock;
-                if (kWhole || i < tile_n) {
-                    const uint64_t key_i = sm.stage.keys[i];
-                    const uint32_t o = sm.out_base[digit_of(key_i, shift, dmask)] + i;
-                    keys_out[o] = key_i;
-                    vals_out[o] = v[k];
-                }
-            }
-        } else {
 #pragma unroll(kWhole ? kItems : 1)
-            for (int k = 0; k < kItems; ++k) {
-                const uint32_t i = tid + (uint32_t)k * kBlock;
-                if (kWhole || i < tile_n) {
-                    const uint64_t key_i = sm.stage.keys[i];
-                    const uint32_t o = sm.out_base[digit_of(key_i, shift, dmask)] + i;
-                    keys_out[o] = key_i;
-                    vals_out[o] = sm.stage.vals[i];
-                }
+        for (int k = 0; k < kItems; ++k) {
+            const uint32_t i = tid + (uint32_t)k * kBlock;
+            if (kWhole || i < tile_n) {
+                const uint64_t key_i = sm.keys[i];
+                const uint32_t o = sm.out_base[digit_of(key_i, shift, dmask)] + i;
+                keys_out[o] = key_i;
+                vals_out[o] = sm.vals[i];
             }
         }
         return next;
@@ -551,215 +496,6 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(SortArgs 
         tile = tile_len(tile) == (uint32_t)kTile ? pass(tile, std::true_type{}) : pass(tile, std::false_type{});
         if (tile >= ntiles) return;
     }
-}
-
-// ------------------------------------------------------ pipelined pass ----
-// Persistent blocks. Each block takes the ticket of its next tile before it
-// ranks the current one and has that tile's keys (and values) brought into
-// shared memory by bulk asynchronous copies (cp.async.bulk completing on an
-// mbarrier), so the load of tile t+1 overlaps the ranking, look-back and
-// scatter of tile t. Only whole tiles whose source addresses are 16-byte
-// aligned are copied this way; the last, partial tile is read directly.
-// Tickets keep their order, so a tile's look-back only waits on tiles that
-// running blocks hold and finish first. Every wait is bounded.
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-// Bounded wait for the phase of the given parity; false (and the error bit)
-// after `limit` polls.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* err,
-                                          uint32_t limit) {
-    for (uint32_t polls = 0; polls < limit; ++polls) {
-        if (mbar_test(bar, parity)) return true;
-        if (polls > 64) __nanosleep(32);
-    }
-    atomicOr(err, kErrLookbackTimeout);
-    return false;
-}
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_addr(dst)),
-        "l"(src), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
-}
-
-template <int kItems>
-struct PipeSmem {
-    static constexpr int kTile = kThreads * kItems;
-    uint64_t keys[2][kTile];  // tile buffers; the current one is reused as the scatter stage
-    uint32_t vals[2][kTile];
-    uint32_t warp_hist[kWarps][kRadix];
-    uint32_t tile_start[kRadix];
-    uint32_t global_base[kRadix];
-    uint32_t scan_tmp[kWarps];
-    uint32_t tile_next;
-    uint32_t pad;
-    uint64_t bar[2];
-};
-
-template <int kItems, int kMinBlocks>
-__global__ __launch_bounds__(kThreads, kMinBlocks) void sort_pass_pipelined_kernel(SortArgs args, uint32_t launch) {
-    using Smem = PipeSmem<kItems>;
-    constexpr int kTile = Smem::kTile;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    Pass pass_args;
-    if (!pick_pass(args, launch, pass_args)) return;
-    const uint64_t* __restrict__ keys_in = pass_args.keys_in;
-    const uint32_t* __restrict__ vals_in = pass_args.vals_in;
-    uint64_t* __restrict__ keys_out = pass_args.keys_out;
-    uint32_t* __restrict__ vals_out = pass_args.vals_out;
-    const uint32_t* excl = pass_args.excl;
-    uint32_t* lookback = pass_args.lookback;
-    uint32_t* tile_counter = args.counters + kTicketWord + launch;
-    const uint32_t shift = pass_args.shift, digit_bits = pass_args.digit_bits;
-    uint32_t* err = args.err;
-    const uint32_t spin_limit = args.spin_limit;
-    const uint32_t n = args.d_count ? min(*args.d_count, args.n_est) : args.n_est;
-    const uint32_t ntiles = (uint32_t)(((uint64_t)n + kTile - 1) / kTile);
-    const uint32_t nfull = n / kTile;  // tiles fetched by bulk copies
-    const uint32_t dmask = (1u << digit_bits) - 1u;
-    const uint32_t lt = lanemask_lt();
-    const uint32_t tx_bytes = kTile * 8u + (vals_in ? kTile * 4u : 0u);
-
-    if (tid == 0) {
-        mbar_init(&sm.bar[0]);
-        mbar_init(&sm.bar[1]);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        sm.tile_next = atomicAdd(tile_counter, 1u);
-    }
-    __syncthreads();
-    uint32_t cur = sm.tile_next;
-    if (cur >= ntiles) return;
-    // Thread 0 issues the copies; phase and pending bits are kept by every
-    // thread (all of them wait).
-    auto issue = [&](uint32_t t, uint32_t buf) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_expect_tx(&sm.bar[buf], tx_bytes);
-        bulk_load(sm.keys[buf], keys_in + (size_t)t * kTile, kTile * 8u, &sm.bar[buf]);
-        if (vals_in) bulk_load(sm.vals[buf], vals_in + (size_t)t * kTile, kTile * 4u, &sm.bar[buf]);
-    };
-    // Per-buffer bits: the mbarrier phase parity to wait for, and whether a
-    // copy into the buffer is in flight.
-    uint32_t phase = 0u, pending = 0u;
-    uint32_t b = 0;
-    if (cur < nfull) {
-        if (tid == 0) issue(cur, 0);
-        pending |= 1u;
-    }
-    while (true) {
-        if (tid == 0) sm.tile_next = atomicAdd(tile_counter, 1u);
-        for (uint32_t i = tid; i < kWarps * kRadix; i += kThreads) (&sm.warp_hist[0][0])[i] = 0;
-        __syncthreads();
-        const uint32_t next = sm.tile_next;
-        if (next < nfull) {
-            if (tid == 0) issue(next, b ^ 1u);
-            pending |= 1u << (b ^ 1u);
-        }
-        const uint64_t tile_base = (uint64_t)cur * kTile;
-        const uint32_t warp_off = warp * 32u * kItems;
-        uint64_t key[kItems];
-        uint32_t val[kItems], pos[kItems];
-        if ((pending >> b) & 1u) {
-            mbar_wait(&sm.bar[b], (phase >> b) & 1u, err, spin_limit);
-            phase ^= 1u << b;
-            pending &= ~(1u << b);
-#pragma unroll
-            for (int k = 0; k < kItems; ++k) {
-                const uint32_t li = warp_off + 32u * k + lane;
-                key[k] = sm.keys[b][li];
-                val[k] = vals_in ? sm.vals[b][li] : (uint32_t)(tile_base + li);
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < kItems; ++k) {
-                const uint64_t i = tile_base + warp_off + 32ull * k + lane;
-                const bool valid = i < n;
-                key[k] = valid ? __ldcs(keys_in + i) : ~0ull;
-                val[k] = valid ? (vals_in ? __ldcs(vals_in + i) : (uint32_t)i) : 0u;
-            }
-        }
-        // Ranking with per-bit ballots, in item order (stable).
-#pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const bool valid = tile_base + warp_off + 32ull * k + lane < n;
-            pos[k] = warp_rank(sm.warp_hist[warp], digit_of(key[k], shift, dmask), valid,
-                                      __ballot_sync(kFullMask, valid), lane, lt);
-        }
-        __syncthreads();
-        uint32_t tile_cnt = 0;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const uint32_t c = sm.warp_hist[w][tid];
-            sm.warp_hist[w][tid] = tile_cnt;
-            tile_cnt += c;
-        }
-        uint32_t* my_word = lookback + (size_t)cur * kRadix + tid;
-        st_relaxed_u32(my_word, (cur == 0 ? kLbInclusive : kLbAggregate) | tile_cnt);
-        const uint32_t tile_start = block_exclusive_scan(tile_cnt, sm.scan_tmp);
-        sm.tile_start[tid] = tile_start;
-        uint32_t prefix = 0;
-        if (cur > 0) {
-            prefix = lookback_window(lookback, cur, tid, err, kRadix, spin_limit);
-            st_relaxed_u32(my_word, kLbInclusive | (prefix + tile_cnt));
-        }
-        sm.global_base[tid] = excl[tid] + prefix;
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const uint32_t digit = digit_of(key[k], shift, dmask);
-            pos[k] += sm.tile_start[digit] + sm.warp_hist[warp][digit];
-        }
-        // The current buffer is free (its contents are in registers): stage
-        // the tile there in sorted order.
-#pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const uint64_t i = tile_base + warp_off + 32ull * k + lane;
-            if (i < n) {
-                sm.keys[b][pos[k]] = key[k];
-                sm.vals[b][pos[k]] = val[k];
-            }
-        }
-        __syncthreads();
-        const uint32_t tile_n = (uint32_t)min((uint64_t)kTile, (uint64_t)n - tile_base);
-        for (uint32_t i = tid; i < tile_n; i += kThreads) {
-            const uint64_t kk = sm.keys[b][i];
-            const uint32_t digit = digit_of(kk, shift, dmask);
-            const uint32_t o = sm.global_base[digit] + (i - sm.tile_start[digit]);
-            keys_out[o] = kk;
-            vals_out[o] = sm.vals[b][i];
-        }
-        __syncthreads();
-        if (next >= ntiles) break;
-        cur = next;
-        b ^= 1u;
-    }
-    // A copy is only left in flight if a wait gave up; wait for it (bounded)
-    // before the block's shared memory is released.
-    for (uint32_t k = 0; k < 2; ++k)
-        if ((pending >> k) & 1u) mbar_wait(&sm.bar[k], (phase >> k) & 1u, err, spin_limit);
 }
 
 // ------------------------------------------------------------- fix-up ----
@@ -832,29 +568,23 @@ __global__ __launch_bounds__(kThreads) void refill_kernel(SortArgs a, size_t wor
         a.lookback[i] = 0u;
 }
 
-// Pass-kernel variants (threads, items per thread, blocks per SM; the pipelined
-// ones copy the next tile in bulk and need 16-byte aligned inputs).
+// Pass-kernel variants (threads, items per thread, blocks per SM). The numbers
+// are settings that callers keep, so the last five, which once had kernels of
+// their own, stand for the shapes that took their place.
 struct PassVariant {
     int threads, items;
     void (*kernel)(SortArgs, uint32_t);
     size_t smem;
-    bool pipelined;
 };
+template <int kBlock, int kItems, int kMinBlocks>
+constexpr PassVariant pass_variant() {
+    return {kBlock, kItems, sort_pass_kernel<kBlock, kItems, kMinBlocks>, sizeof(PassSmem<kBlock, kItems>)};
+}
 const PassVariant kVariants[] = {
-    {256, 16, sort_pass_kernel<256, 16, 2>, sizeof(PassSmem<256, 16>), false},
-    {384, 12, sort_pass_kernel<384, 12, 2>, sizeof(PassSmem<384, 12>), false},
-    {512, 12, sort_pass_kernel<512, 12, 1>, sizeof(PassSmem<512, 12>), false},
-    {256, 8, sort_pass_kernel<256, 8, 4>, sizeof(PassSmem<256, 8>), false},
-    {256, 20, sort_pass_kernel<256, 20, 2>, sizeof(PassSmem<256, 20>), false},
-    {256, 12, sort_pass_kernel<256, 12, 3>, sizeof(PassSmem<256, 12>), false},
-    {256, 8, sort_pass_kernel<256, 8, 3>, sizeof(PassSmem<256, 8>), false},
-    {256, 12, sort_pass_pipelined_kernel<12, 2>, sizeof(PipeSmem<12>), true},
-    {256, 8, sort_pass_pipelined_kernel<8, 3>, sizeof(PipeSmem<8>), true},
-    {256, 12, sort_pass_kernel<256, 12, 4, true>, sizeof(PassSmem<256, 12, true>), false},
-    {256, 16, sort_pass_kernel<256, 16, 3, true>, sizeof(PassSmem<256, 16, true>), false},
-    {256, 20, sort_pass_kernel<256, 20, 2, true>, sizeof(PassSmem<256, 20, true>), false},
+    pass_variant<256, 16, 2>(), pass_variant<384, 12, 2>(), pass_variant<512, 12, 1>(), pass_variant<256, 8, 4>(),
+    pass_variant<256, 20, 2>(), pass_variant<256, 12, 3>(), pass_variant<256, 8, 3>(),  pass_variant<256, 12, 3>(),
+    pass_variant<256, 8, 4>(),  pass_variant<256, 12, 3>(), pass_variant<256, 16, 2>(), pass_variant<256, 20, 2>(),
 };
-constexpr int kFallbackVariant = 5;  // for inputs a pipelined variant cannot copy
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 constexpr int kMinItems = 8;  // sizes the look-back words for every variant
 static_assert(kThreads * kMinItems == (int)kSortPlanTile, "look-back sizing");
@@ -987,13 +717,7 @@ cudaError_t sort_launch(const uint64_t* keys_in, const uint32_t* vals_in, uint64
                           reinterpret_cast<uint32_t*>(t + plan.vals_tmp), n_est, d_count, key_bits,
                           current_device(), st, own);
     }
-    int vi = variant != 0 ? (int)variant - 1 : (g_variant >= 0 ? g_variant : variant_for(n_est));
-    // Bulk copies need 16-byte aligned sources; the temporaries always are.
-    // The stalled test pass needs one block per tile (no persistent blocks).
-    if (kVariants[vi].pipelined &&
-        (stall_first_tile ||
-         (((uintptr_t)keys_in | (uintptr_t)(vals_in ? vals_in : nullptr)) & 15u) != 0))
-        vi = kFallbackVariant;
+    const int vi = variant != 0 ? (int)variant - 1 : (g_variant >= 0 ? g_variant : variant_for(n_est));
     const PassVariant& pv = kVariants[vi];
     const uint32_t tile = (uint32_t)(pv.threads * pv.items);
     const uint32_t ntiles = (uint32_t)(((uint64_t)n_est + tile - 1) / tile);

@@ -855,9 +855,8 @@ def main(argv=None):
             "e2e": r["e2e"], "gpu_launches": r["launches"],
             "roofline": {"kernel": ("traverse_ref_kernel"
                                     if WORKLOADS[args.workload].preset == "reference"
-                                    else ("group_far_kernel + group_eval_kernel"
-                                          if r["far_nodes"] and r["p"].group_size > 32
-                                          else "group_eval_kernel") if group
+                                    else ("group_far_kernel + group_eval_fast_kernel"
+                                          if r["far_nodes"] else "group_eval_fast_kernel") if group
                                     else "traverse_phys_kernel"),
                          "bound": "fp32",
                          "achieved": r["achieved"], "peak": r["fp32_peak"], "unit": "TFLOP/s",

@@ -182,13 +182,8 @@ typedef struct astro_params {
                                  (4, 1 or 5 by the number of pairs),
                                  1 = 256x16/2, 2 = 384x12/2, 3 = 512x12/1,
                                  4 = 256x8/4, 5 = 256x20/2, 6 = 256x12/3,
-                                 7 = 256x8/3; 8 = 256x12/2 and 9 = 256x8/3 that
-                                 bulk-copy the next tile while ranking the
-                                 current one (16-byte aligned inputs; others
-                                 use 6); lean passes that keep no value in
-                                 registers (values prefetched to L2 and gathered
-                                 by a staged 16-bit index): 10 = 256x12/4,
-                                 11 = 256x16/3, 12 = 256x20/2 */
+                                 7 = 256x8/3; 8 to 12 are kept for settings
+                                 made earlier and equal 6, 4, 6, 1 and 5 */
     uint32_t light_sources;   /* REFERENCE: astro_step runs the lighting pass
                                  with the first light_sources particles (at most
                                  5) as lights (Renderer.swift:539; numStars = 5);
