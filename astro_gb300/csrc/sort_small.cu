@@ -21,9 +21,12 @@
 // match instead of votes: 89 us. From kClusterPairs on the onesweep passes are
 // as fast (100,003 42-bit keys: 66 us there, 67 us here).
 //
-// At most kTinyPairs pairs are sorted by one block with a bitonic network on
-// (key, position): 12 us for 1,024 pairs and 6 us for 205 (15 and 12 us for three
-// radix passes of one block).
+// At most kBlockPairs pairs are sorted by one block in shared memory: by radix
+// passes (sort_block_kernel), or, at most kTinyPairs pairs of more than
+// kTinyBits bits, by a bitonic network on (key, position). Radix / bitonic, us:
+// 300 pairs of 24 bits 4.3 / 7.2, of 63 bits 9.7 / 7.2; 1,024 of 24 bits 7.6 /
+// 12.0, of 63 bits 17.9 / 12.0; 2,048 of 63 bits 23.8 / 24.9; 4,096 of 24 bits
+// 14.5 / 51.7, of 63 bits 35.7 / 51.6.
 #include <algorithm>
 #include <mutex>
 
@@ -38,7 +41,8 @@ namespace astro {
 namespace {
 
 constexpr uint32_t kRadix = 256;
-constexpr uint32_t kTinyPairs = 4096;      // one block, bitonic
+constexpr uint32_t kBlockPairs = 4096;     // one block
+constexpr uint32_t kTinyPairs = 1024, kTinyBits = 40;
 constexpr uint32_t kClusterPairs = 65536;  // a cluster, radix passes
 constexpr uint32_t kMaxSlice = 8192;  // pairs per block
 constexpr uint32_t kMaxThreads = 1024;
@@ -248,8 +252,124 @@ __global__ __launch_bounds__(kMaxThreads, 1) void sort_small_kernel(
         }
 }
 
-// Bitonic sort of at most kTinyPairs pairs in shared memory; a thread takes one
-// or two compare-exchanges a stage. Strides of up to 32 stay inside a warp's 64
+// Radix passes of one block over pairs that stay in shared memory between them:
+// kItems pairs a thread, ranked as in sort_small_kernel.
+__host__ __device__ constexpr size_t block_smem(uint32_t pairs, uint32_t threads) {
+    return (size_t)pairs * 12u + (size_t)(threads / 32u) * kRadix * 2u + 4u * kRadix + 4u * 8u;
+}
+template <int kItems>
+__global__ __launch_bounds__(kMaxThreads, 1) void sort_block_kernel(
+    const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* __restrict__ keys_out,
+    uint32_t* __restrict__ vals_out, const uint32_t* d_count, uint32_t n_est, uint32_t key_bits,
+    uint32_t* __restrict__ clear_err) {
+    after_previous();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, warps = blockDim.x >> 5;
+    const uint32_t room = kItems * blockDim.x;
+    uint64_t* const keys = reinterpret_cast<uint64_t*>(smem_raw);
+    uint32_t* const vals = reinterpret_cast<uint32_t*>(keys + room);
+    uint16_t* const warp_hist = reinterpret_cast<uint16_t*>(vals + room);  // [warps][kRadix]
+    uint32_t* const start = reinterpret_cast<uint32_t*>(warp_hist + warps * kRadix);
+    uint32_t* const scan_tmp = start + kRadix;
+    uint16_t* const my_hist = warp_hist + warp * kRadix;
+    const uint32_t n = d_count ? min(*d_count, n_est) : n_est;
+    if (clear_err && tid == 0) *clear_err = 0u;
+    const uint32_t warp_first = warp * 32u * kItems + lane;
+    const uint32_t lt = lanemask_lt();
+    uint64_t key[kItems];
+    uint32_t val[kItems], pos[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const uint32_t i = warp_first + 32u * k;
+        key[k] = i < n ? keys_in[i] : 0ull;
+        val[k] = i < n ? (vals_in ? vals_in[i] : i) : 0u;
+    }
+    const uint32_t passes = key_bits == 0 ? 1u : (key_bits + 7u) / 8u;
+#pragma unroll 1
+    for (uint32_t p = 0; p < passes; ++p) {
+        const uint32_t shift = 8u * p;
+        const uint32_t dmask = (1u << min(8u, key_bits - min(shift, key_bits))) - 1u;
+        reinterpret_cast<uint4*>(my_hist)[lane] = make_uint4(0u, 0u, 0u, 0u);
+        if (p > 0) {
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) {
+                key[k] = keys[warp_first + 32u * k];
+                val[k] = vals[warp_first + 32u * k];
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            const bool valid = warp_first + 32u * k < n;
+            const uint32_t digit = (uint32_t)(key[k] >> shift) & dmask;
+            uint32_t peers = __ballot_sync(kFullMask, valid);
+#pragma unroll
+            for (uint32_t t = 0; t < 8u; ++t) {
+                const bool bit = (digit >> t) & 1u;
+                const uint32_t m = __ballot_sync(kFullMask, bit);
+                peers &= bit ? m : ~m;
+            }
+            pos[k] = __popc(peers & lt);
+            if (valid) pos[k] += my_hist[digit];
+            __syncwarp();
+            if (valid && (peers & ~lt) == (1u << lane)) my_hist[digit] = (uint16_t)(pos[k] + 1u);
+            __syncwarp();
+        }
+        __syncthreads();
+        // The warps' exclusive offsets of every digit and its count, four lanes a
+        // digit with a quarter of the warps each.
+        for (uint32_t d0 = 0; d0 < kRadix; d0 += blockDim.x / 4u) {
+            const uint32_t d = d0 + tid / 4u, q = tid % 4u;
+            uint32_t c[kMaxThreads / 128u], sum = 0;
+#pragma unroll
+            for (uint32_t t = 0; t < kMaxThreads / 128u; ++t) {
+                const uint32_t w = q * (kMaxThreads / 128u) + t;
+                c[t] = w < warps && d < kRadix ? (uint32_t)warp_hist[w * kRadix + d] : 0u;
+                sum += c[t];
+            }
+            uint32_t run = sum;
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFullMask, run, o, 4);
+                if (q >= (uint32_t)o) run += y;
+            }
+            if (q == 3u && d < kRadix) start[d] = run;
+            run -= sum;
+#pragma unroll
+            for (uint32_t t = 0; t < kMaxThreads / 128u; ++t) {
+                const uint32_t w = q * (kMaxThreads / 128u) + t;
+                if (w < warps && d < kRadix) warp_hist[w * kRadix + d] = (uint16_t)run;
+                run += c[t];
+            }
+        }
+        __syncthreads();
+        uint32_t incl = 0, count = 0;
+        if (tid < kRadix) {
+            count = start[tid];
+            incl = warp_scan(count, lane);
+            if (lane == 31u) scan_tmp[warp] = incl;
+        }
+        __syncthreads();
+        if (tid < kRadix) start[tid] = incl - count + warps_before(scan_tmp, warp, lane);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            if (warp_first + 32u * k >= n) continue;
+            const uint32_t digit = (uint32_t)(key[k] >> shift) & dmask;
+            const uint32_t at = start[digit] + my_hist[digit] + pos[k];
+            keys[at] = key[k];
+            vals[at] = val[k];
+        }
+        __syncthreads();
+    }
+    for (uint32_t i = tid; i < n; i += blockDim.x) {
+        keys_out[i] = keys[i];
+        vals_out[i] = vals[i];
+    }
+}
+
+// Bitonic sort of at most kTinyPairs pairs in shared memory, a compare-exchange a
+// thread and stage. Strides of up to 32 stay inside a warp's 64
 // elements, so those stages only need the warp.
 constexpr uint32_t kTinyThreads = 1024;
 __global__ __launch_bounds__(kTinyThreads, 1) void sort_tiny_kernel(
@@ -324,6 +444,11 @@ cudaError_t sort_small_init(int dev) {
     cudaError_t e = cudaFuncSetAttribute(sort_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)small_smem(kMaxSlice, kMaxThreads));
     if (e != cudaSuccess) return e;
+    for (auto k : {sort_block_kernel<1>, sort_block_kernel<2>, sort_block_kernel<4>}) {
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)block_smem(kBlockPairs, kMaxThreads));
+        if (e != cudaSuccess) return e;
+    }
     e = cudaFuncSetAttribute(sort_tiny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(kTinyPairs * 12u));
     if (e != cudaSuccess) return e;
@@ -347,7 +472,7 @@ cudaError_t sort_small_init(int dev) {
 uint32_t sort_small_max(int dev) {
     std::lock_guard<std::mutex> lock(g_small_mutex);
     return dev >= 0 && dev < (int)kMaxDevices && g_cluster[dev] > 0
-               ? std::max(kTinyPairs, std::min(kClusterPairs, g_cluster[dev] * kMaxSlice))
+               ? std::max(kBlockPairs, std::min(kClusterPairs, g_cluster[dev] * kMaxSlice))
                : 0u;
 }
 
@@ -359,6 +484,13 @@ cudaError_t sort_small(const uint64_t* keys_in, const uint32_t* vals_in, uint64_
     {
         std::lock_guard<std::mutex> lock(g_small_mutex);
         cap = g_cluster[dev];
+    }
+    if (n_est <= kBlockPairs && (n_est > kTinyPairs || key_bits <= kTinyBits)) {
+        const uint32_t items = n_est <= 1024u ? 1u : (n_est <= 2048u ? 2u : 4u);
+        const uint32_t threads = std::max(kRadix, ((n_est + items - 1u) / items + 31u) / 32u * 32u);
+        auto kernel = items == 1u ? sort_block_kernel<1> : (items == 2u ? sort_block_kernel<2> : sort_block_kernel<4>);
+        return launch_after(kernel, 1, threads, block_smem(items * threads, threads), st, keys_in, vals_in, keys_out,
+                            vals_out, d_count, n_est, key_bits, clear_err);
     }
     if (n_est <= kTinyPairs) {
         uint32_t size = 64;
