@@ -8,15 +8,14 @@ The knobs are fields of astro_params that change speed, not physics:
 
   block_warps   traversal block size (warps per block: 4 or 8)
   group_size    particles per warp: consecutive sorted particles sharing one
-                tree walk (1..64; two per lane above 32; groups of <= 16 run
-                as several copies that split the source lists)
+                tree walk (1..64; the lanes hold pairs and split the source
+                lists)
   lbits         tree depth, i.e. the depth of the walk (layers = lbits + 1)
   bucket        leaf tile size: an opened node holding <= bucket particles
                 is summed particle by particle
   sort_variant  radix sort pass kernel (threads, items per thread, blocks per
                 SM)
-  walk_frontier the group walk's frontier: runs of consecutive child nodes
-                or a list of node indices
+  walk_frontier accepted for settings made earlier; both values walk alike
 
   far_ratio     accepted nodes further than (group radius) / far_ratio from
                 the group's centre are summed through one second-order

@@ -8,8 +8,8 @@
 // The reference finds the runs of every layer with one sort + scan + scatter
 // per layer over all N entries. Here a single pass over the sorted keys finds
 // the node starts of all layers at once (topology_kernel); the large layers
-// are aggregated one launch each and the small top layers in one climbing
-// launch (aggregate_tree_kernel).
+// are aggregated one launch each and the small top layers in one launch of a
+// thread-block cluster (aggregate_top_kernel).
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -627,7 +627,7 @@ __device__ __forceinline__ void aggregate_ref_internal(const AggArgs& a, uint32_
 
 // ---- PHYSICAL ----
 
-// A node's record as the climbing thread holds it: raw sums (FP32 in the
+// A node's record as the thread that makes it holds it: raw sums (FP32 in the
 // plain form, FP64 in the precision form), centre of mass and mass,
 // quadrupole, particles and key.
 template <bool kPrec>
@@ -833,9 +833,10 @@ __device__ __forceinline__ void aggregate_internal(const AggArgs& a, uint32_t l,
 // (capacity), by looking at every node in smaller ones, where the list's
 // atomics and indirection cost more than the idle threads.
 //
-// What bounds it: the record stores (56 bytes a node of a chain), in the
-// precision form the FP64 pipe (64 cycles an instruction and warp), and in
-// small trees the launches and load latencies. Aggregation before and after
+// What bounds it: the record stores (56 bytes a node of a chain), the latency of
+// the leaves' dependent loads, and in small trees the launches. (Not the FP64
+// pipe: conversions done with integers instead left the leaf pass of 4,194,304
+// bodies in the precision form at 175 us.) Aggregation before and after
 // (one launch a layer, each re-reading its children): 6,000,007-body cube at 21
 // bits 4.55 -> 1.83 ms, two Plummer spheres of 4,194,304 in the precision form
 // 481 -> 342 us, 256 systems 590 -> 424 us, 524,288-body disk 146 -> 105 us.

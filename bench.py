@@ -67,9 +67,9 @@ L2_FLUSH_BYTES = 256 << 20  # larger than the 129 MB L2
 # the kernels the roofline times for (workload, form, lbits): its "traffic".
 # C5 at lbits 6: one ncu capture of each of the same kernels on the same law
 # at 2,097,152 particles (lbits 5, 64 particles per leaf as at full size;
-# cold cache): the evaluation 228.44 MB and the far-node sums 51.15 MB,
+# cold cache): the evaluation 201.60 MB and the far-node sums 51.07 MB,
 # scaled by the particle count (x8).
-NCU_EVAL_DRAM_BYTES: dict = {("c5", "plain", 6): (228.444672e6 + 51.145472e6) * 8}
+NCU_EVAL_DRAM_BYTES: dict = {("c5", "plain", 6): (201.602560e6 + 51.072512e6) * 8}
 
 
 def parse(argv=None):
@@ -128,22 +128,31 @@ def workload(args):
     return w
 
 
-CLIMB_MIN_NODES = 32768  # build.cu: layers of at least this capacity get a launch each
+LAYER_MIN_NODES = 32768  # build.cu: layers of at least this capacity get a launch each
+SMALL_SORT_PAIRS = 65536  # sort_small.cu: sorted in one launch
+TOP_DIGITS_PAIRS = 5 << 18  # sort.cu: from here, and six digits, the top digits are tried first
 
 
-def kernels_per_step(key_bits: int, layer_sizes, preset: str = "physical") -> int:
+def kernels_per_step(key_bits: int, layer_sizes, preset: str = "physical", pairs: int | None = None,
+                     far: bool = False) -> int:
     """This library's kernel launches in one step. PHYSICAL: bbox, setup,
-    encode, sort histogram + one pass per 8 key bits, Morton reorder,
-    topology, the per-layer aggregations below the climb + the climbing
-    one, the group walk and its evaluation (9 + passes + per-layer
-    aggregations). REFERENCE: encode, sort histogram + passes, topology,
-    aggregations, traversal, lights snapshot + lighting, integrate (8 +
-    passes + per-layer aggregations)."""
+    encode, sort histogram + one pass per 8 key bits (one launch for few
+    pairs, five more where the top digits are tried first), Morton reorder,
+    topology, the per-layer aggregations + the small layers' one, the group
+    walk, the far sums (where a far ratio is set) and the evaluation (9 +
+    passes + per-layer aggregations without far sums). REFERENCE: encode,
+    sort histogram + passes, topology, aggregations, traversal, lights
+    snapshot + lighting, integrate (8 + passes + per-layer aggregations)."""
     passes = (key_bits + 7) // 8
     l0 = 0
-    while l0 + 1 < len(layer_sizes) and layer_sizes[l0] >= CLIMB_MIN_NODES:
+    while l0 + 1 < len(layer_sizes) and layer_sizes[l0] >= LAYER_MIN_NODES:
         l0 += 1
-    return (9 if preset == "physical" else 8) + passes + l0
+    sort = 1 + passes
+    if pairs is not None and pairs <= SMALL_SORT_PAIRS:
+        sort = 1
+    elif pairs is not None and pairs >= TOP_DIGITS_PAIRS and passes >= 6:
+        sort += 5
+    return (8 if preset == "physical" else 7) + sort + l0 + (1 if far else 0)
 
 
 def walk_flags(args, L, flags):
@@ -591,7 +600,8 @@ def run_ours(args, world, rank, local):
                "how": "pinned host buffers; per step astro_upload_async, astro_step, "
                       "astro_download_async (copies overlap the steps), one synchronize at the end"}
 
-    launches_per_step = kernels_per_step(key_bits, sizes_, w.preset)
+    launches_per_step = kernels_per_step(key_bits, sizes_, w.preset, n_tree if is_ref else n,
+                                         args.walk == "group" and not is_ref and p.far_ratio > 0.0)
     sim.close()
     del flush
     torch.cuda.empty_cache()

@@ -175,8 +175,8 @@ typedef struct astro_params {
                                  (0 = default); the group walk's kernels have
                                  their own block sizes */
     uint32_t group_size;      /* PHYSICAL group walk: at most this many consecutive
-                                 particles share one tree walk (one warp; two
-                                 particles per lane above 32), 1..64; 0 = 32 */
+                                 particles share one tree walk (one warp),
+                                 1..64; 0 = 32 */
     uint32_t sort_variant;    /* radix sort pass kernel (threads x items per
                                  thread / blocks per SM): 0 = library default
                                  (4, 1 or 5 by the number of pairs),
@@ -308,7 +308,7 @@ int astro_read_far_stats(astro_ctx* ctx, uint64_t* far_nodes, uint64_t* far_inte
 /* Device times of the last group-walk traversal made by a stage call
  * (astro_traverse; graph-replayed steps are not timed): the walk that
  * builds the interaction lists, and the evaluation that sums them
- * (including the per-walk far-node sums for groups of more than 32)
+ * (including the per-walk far-node sums)
  * (CUDA events on the context's stream; waits for them). */
 int astro_read_traverse_times(astro_ctx* ctx, float* walk_ms, float* eval_ms);
 
