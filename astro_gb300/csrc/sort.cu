@@ -136,10 +136,15 @@ __device__ __forceinline__ uint32_t sample_place(uint32_t k, uint32_t n) {
     return __umulhi(h, n);
 }
 
-// Whether the digits from `shift` up leave a key about kNeighbours others with
-// the same ones: of S keys at random places, S^2 / 2 times the chance that two
-// keys agree do.
-__device__ __forceinline__ bool top_suffices(const uint64_t* samples, uint32_t n, uint32_t shift) {
+// The bits of a key that take part.
+__device__ __forceinline__ uint64_t key_mask(uint32_t key_bits) {
+    return key_bits >= 64u ? ~0ull : (1ull << key_bits) - 1ull;
+}
+
+// Whether the digits from `shift` up (of the bits that take part) leave a key
+// about kNeighbours others with the same ones: of S keys at random places, S^2 / 2
+// times the chance that two keys agree do.
+__device__ __forceinline__ bool top_suffices(const uint64_t* samples, uint32_t n, uint32_t shift, uint64_t mask) {
     extern __shared__ uint32_t slots[];  // hashes of prefixes; all ones: empty
     __shared__ uint32_t s_equal;
     const uint32_t tid = threadIdx.x;
@@ -153,7 +158,7 @@ __device__ __forceinline__ bool top_suffices(const uint64_t* samples, uint32_t n
     // 45 us.)
 #pragma unroll 1
     for (uint32_t k = tid; k < kSamples; k += kThreads) {
-        const uint64_t prefix = __ldcg(samples + k) >> shift;
+        const uint64_t prefix = (__ldcg(samples + k) & mask) >> shift;
         const uint32_t id = min((uint32_t)((prefix * 0x9E3779B97F4A7C15ull) >> 32), ~1u);
         uint32_t at = id & (kSampleSlots - 1u);
         while (true) {  // half of the slots stay empty
@@ -259,7 +264,7 @@ __global__ __launch_bounds__(kThreads, kHistBlocksPerSm) void sort_histogram_ker
         float others = (float)n;  // if the digits were independent
         for (uint32_t k = m - kTopDigits; k < m; ++k) others *= s_agree[(digits >> (4u * k)) & 15u];
         // Keys of clustered particles share their digits far more often.
-        if (others <= 16.f * kNeighbours && top_suffices(samples, n, 8u * lowest)) top = kTopDigits;
+        if (others <= 16.f * kNeighbours && top_suffices(samples, n, 8u * lowest, key_mask(key_bits))) top = kTopDigits;
     }
     if (tid == 0) {
         counters[kScheduleWord] = m | (top << 8);
@@ -499,12 +504,16 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(SortArgs 
 }
 
 // ------------------------------------------------------------- fix-up ----
-// Orders keys that are sorted, stably, by their top digits. Where a key's run (the neighbours that share these digits) begins
-// and ends is read off a bit mask of the runs' heads; its place is the run's
-// beginning plus the keys of the run that come before it. A run of more than
+// Orders keys that are sorted, stably, by their top digits. Where a key's run (the
+// neighbours that share these digits) begins and ends is read off a bit mask of
+// the runs' heads; its place is the run's beginning plus the keys of the run that
+// come before it. Like the passes, all of this looks at the low key_bits bits only:
+// a caller may keep anything above them (kMasked: key_bits < 64; the masks in the
+// inner loop cost 11 us at 16.7 M pairs). A run of more than
 // 2 kFixHalo keys, or one that reaches a halo's far edge, gives up (word 4).
 // 16.7 M pairs, two others a run on average: 109 us, bound by its instructions
 // (384 MB are 59 us); scanning left and right from each key 119 us.
+template <bool kMasked>
 __global__ __launch_bounds__(kThreads) void fixup_kernel(SortArgs a) {
     constexpr uint32_t kKeys = kFixTile + 2 * kFixHalo;
     __shared__ uint64_t s_key[kKeys];
@@ -518,6 +527,7 @@ __global__ __launch_bounds__(kThreads) void fixup_kernel(SortArgs a) {
     if (begin >= n) return;
     uint32_t* failed = a.counters + kScheduleWord + 4;
     const uint32_t shift = 8u * ((digits >> (4u * (m - top))) & 15u);
+    const uint64_t mask = kMasked ? key_mask(a.key_bits) : ~0ull;
     const uint32_t tile = min(kFixTile, n - begin);
     const uint32_t lead = min(begin, kFixHalo), count = lead + tile + min(n - begin - tile, kFixHalo);
     const uint64_t* src = a.keys_tmp + (begin - lead);
@@ -527,14 +537,14 @@ __global__ __launch_bounds__(kThreads) void fixup_kernel(SortArgs a) {
     __syncthreads();
 #pragma unroll
     for (uint32_t i = tid; i < kKeys; i += kThreads) {
-        const bool head = i >= count || i == 0u || ((s_key[i] ^ s_key[i - 1]) >> shift) != 0ull;
+        const bool head = i >= count || i == 0u || (((s_key[i] ^ s_key[i - 1]) & mask) >> shift) != 0ull;
         const uint32_t heads = __ballot_sync(kFullMask, head);
         if ((tid & 31u) == 0u) s_head[i / 32u] = heads;
     }
     __syncthreads();
     bool long_run = false;
     for (uint32_t i = lead + tid; i < lead + tile; i += kThreads) {
-        const uint64_t key = s_key[i];
+        const uint64_t key = s_key[i], low = key & mask;
         const uint32_t val = __ldcs(a.vals_tmp + (begin - lead) + i);
         uint32_t word = i / 32u;
         uint32_t bits = s_head[word] & (0xFFFFFFFFu >> (31u - (i & 31u)));
@@ -552,7 +562,7 @@ __global__ __launch_bounds__(kThreads) void fixup_kernel(SortArgs a) {
             // Keys of a run differ by less than 2^56: the sign of a difference
             // orders them. Equal keys before i count, those behind it do not.
             for (uint32_t j = from; j < to; ++j)
-                place += (uint32_t)((s_key[j] - key - (j < i ? 1ull : 0ull)) >> 63);
+                place += (uint32_t)(((s_key[j] & mask) - low - (j < i ? 1ull : 0ull)) >> 63);
         }
         a.keys_out[begin - lead + place] = key;
         a.vals_out[begin - lead + place] = val;
@@ -757,7 +767,9 @@ cudaError_t sort_launch(const uint64_t* keys_in, const uint32_t* vals_in, uint64
     // that gave up starts over with. A launch with nothing to do takes about 2 us.
     for (uint32_t l = 0; l < plan.passes + early; ++l) {
         if (try_top && l == early) {
-            fixup_kernel<<<(n_est - 1u) / kFixTile + 1u, kThreads, 0, st>>>(args);
+            const uint32_t tiles = (n_est - 1u) / kFixTile + 1u;
+            if (key_bits < 64u) fixup_kernel<true><<<tiles, kThreads, 0, st>>>(args);
+            else fixup_kernel<false><<<tiles, kThreads, 0, st>>>(args);
             refill_kernel<<<num_sms(), kThreads, 0, st>>>(args, plan.passes * stride);
         }
         pv.kernel<<<grid, pv.threads, pv.smem, st>>>(args, l);
