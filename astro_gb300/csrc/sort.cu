@@ -44,24 +44,29 @@ constexpr uint32_t kDoneWord = 8, kScheduleWord = 10, kTicketWord = 16;
 // knows the digit counts: word 0 holds the number m of digits that not all keys
 // share (at least 1) and in bits 8-15 the number of top digits to sort by (0: all
 // m, from the lowest up); word 1 the m digits, lowest first, four bits each;
-// word 4 is set when a run of keys that share their top digits was too long.
+// word 4 kLongRuns and kStartOver as met on the way; word 5 the long runs listed.
 //
 // Top digits: stable passes over the top kTopDigits digits, then ordering by
 // reading: a key finds its place among the others that share them, about
-// kNeighbours at most on average (fixup_kernel). Should a run be too long for
-// that, all m digits are sorted from the input after all.
+// kNeighbours at most on average (fixup_kernel). A run of more than kFixHalo of them
+// is sorted by a block of its own (runs_kernel); should one be longer than kRunMax,
+// all m digits are sorted from the input after all.
 //
 // 63-bit keys without / with it: uniform ones, 1,500,000 194 / 172 us, 2,097,152
-// 226 / 190, 16,777,216 1005 / 628 (262,144 122 / 136, so not below kTopMin).
+// 226 / 167, 16,777,216 1005 / 526 (262,144 122 / 136, so not below kTopMin).
 // Keys of clustered particles do not qualify and pay for the question: 48 bits,
-// 1,500,000 158 / 185 us, 5,000,000 310 / 335. A fix-up that gives up costs its
-// passes: 4,194,304 351 -> 495. (Four or five top digits let clustered 63-bit keys
-// qualify, 5,000,000 399 -> 370 us, but some runs were too long: 690 us.)
+// 5,000,000 298 / 310. Uniform keys of 48 bits but for one place that holds 500 or
+// 5,000 of them, 2,000,000: 265 and 278 us when every long run had all digits
+// sorted, 161 and 191 with blocks for them (155 without the place). (Four or five
+// top digits let clustered 63-bit keys qualify, 5,000,000 399 -> 370 us, but with
+// longer runs.)
 constexpr uint32_t kTopDigits = 3, kSavedPasses = 3;  // of at least 6 digits
 constexpr uint32_t kTopMin = 5u << 18;
 constexpr float kNeighbours = 4.f;
 constexpr uint32_t kSamples = 4096, kSampleSlots = 2 * kSamples;
 constexpr uint32_t kFixTile = 2048, kFixHalo = 128;
+constexpr uint32_t kRunThreads = 1024, kRunMax = 32u * kRunThreads;
+constexpr uint32_t kLongRuns = 1u, kStartOver = 2u;
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -285,6 +290,7 @@ struct SortArgs {
     size_t lookback_stride;  // words of one pass
     uint32_t* counters;
     uint32_t early;  // launches before the fix-up (0: no fix-up)
+    uint32_t* runs;  // beginnings of the long runs
     uint32_t* err;
     uint32_t spin_limit;
 };
@@ -310,7 +316,7 @@ __device__ __forceinline__ bool pick_pass(const SortArgs& a, uint32_t launch, Pa
         at = m - top + i;
         stages = top + 1u;
     } else if (top != 0u) {
-        if (a.counters[kScheduleWord + 4] == 0u) return false;
+        if ((a.counters[kScheduleWord + 4] & kStartOver) == 0u) return false;
         at = i -= a.early;
     }
     if (i >= count) return false;
@@ -509,8 +515,9 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void sort_pass_kernel(SortArgs 
 // the runs' heads; its place is the run's beginning plus the keys of the run that
 // come before it. Like the passes, all of this looks at the low key_bits bits only:
 // a caller may keep anything above them (kMasked: key_bits < 64; the masks in the
-// inner loop cost 11 us at 16.7 M pairs). A run of more than
-// 2 kFixHalo keys, or one that reaches a halo's far edge, gives up (word 4).
+// inner loop cost 11 us at 16.7 M pairs). A key sees kFixHalo keys on each side of
+// its tile, so all keys of a run agree whether it has more than kFixHalo of them; the
+// first one then lists it for runs_kernel.
 // 16.7 M pairs, two others a run on average: 109 us, bound by its instructions
 // (384 MB are 59 us); scanning left and right from each key 119 us.
 template <bool kMasked>
@@ -525,7 +532,6 @@ __global__ __launch_bounds__(kThreads) void fixup_kernel(SortArgs a) {
     const uint32_t n = a.d_count ? min(*a.d_count, a.n_est) : a.n_est;
     const uint32_t begin = blockIdx.x * kFixTile;
     if (begin >= n) return;
-    uint32_t* failed = a.counters + kScheduleWord + 4;
     const uint32_t shift = 8u * ((digits >> (4u * (m - top))) & 15u);
     const uint64_t mask = kMasked ? key_mask(a.key_bits) : ~0ull;
     const uint32_t tile = min(kFixTile, n - begin);
@@ -542,7 +548,6 @@ __global__ __launch_bounds__(kThreads) void fixup_kernel(SortArgs a) {
         if ((tid & 31u) == 0u) s_head[i / 32u] = heads;
     }
     __syncthreads();
-    bool long_run = false;
     for (uint32_t i = lead + tid; i < lead + tile; i += kThreads) {
         const uint64_t key = s_key[i], low = key & mask;
         const uint32_t val = __ldcs(a.vals_tmp + (begin - lead) + i);
@@ -554,28 +559,121 @@ __global__ __launch_bounds__(kThreads) void fixup_kernel(SortArgs a) {
         bits = s_head[word] & ((0xFFFFFFFEu << (i & 31u)));
         while (bits == 0u && ++word < kKeys / 32u) bits = s_head[word];
         const uint32_t to = bits == 0u ? count : min(count, 32u * word + (uint32_t)__ffs(bits) - 1u);
-        uint32_t place = from;
-        if ((from == 0u && lead == kFixHalo) || (to == count && begin - lead + count < n) || to - from > 2u * kFixHalo) {
-            long_run = true;
-            place = i;
-        } else {
-            // Keys of a run differ by less than 2^56: the sign of a difference
-            // orders them. Equal keys before i count, those behind it do not.
-            for (uint32_t j = from; j < to; ++j)
-                place += (uint32_t)(((s_key[j] & mask) - low - (j < i ? 1ull : 0ull)) >> 63);
+        if (to - from > kFixHalo) {  // of those in sight
+            if (from == i) {
+                const uint32_t first = begin - lead + i, past = min(n, first + kRunMax);
+                const bool too_long = past < n && (((src[i + kRunMax] ^ key) & mask) >> shift) == 0ull;
+                atomicOr(a.counters + kScheduleWord + 4, too_long ? kStartOver : kLongRuns);
+                if (!too_long) a.runs[atomicAdd(a.counters + kScheduleWord + 5, 1u)] = first;
+            }
+            continue;
         }
+        // Keys of a run differ by less than 2^56: the sign of a difference
+        // orders them. Equal keys before i count, those behind it do not.
+        uint32_t place = from;
+        for (uint32_t j = from; j < to; ++j)
+            place += (uint32_t)(((s_key[j] & mask) - low - (j < i ? 1ull : 0ull)) >> 63);
         a.keys_out[begin - lead + place] = key;
         a.vals_out[begin - lead + place] = val;
     }
-    if (long_run) atomicOr(failed, 1u);
 }
 
-// Empties the look-back words of the early passes when all digits have to be
-// sorted after all.
-__global__ __launch_bounds__(kThreads) void refill_kernel(SortArgs a, size_t words) {
-    if (a.counters[kScheduleWord + 4] == 0u) return;
-    for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < words; i += (size_t)gridDim.x * kThreads)
-        a.lookback[i] = 0u;
+// The long runs, a block each: stable passes over the digits below the top ones,
+// between the temporaries and the output, where a warp ranks a contiguous part of
+// the run 32 keys at a time. The keys stay in L2 and the chain of loads bounds it:
+// 7 us for a run of 500 keys, 36 for one of 5,000, three digits.
+// Where all digits have to be sorted after all it empties the look-back words (the
+// early passes', and the list, which stands where the fourth pass has its words).
+__global__ __launch_bounds__(kRunThreads) void runs_kernel(SortArgs a, size_t words) {
+    const uint32_t flags = a.counters[kScheduleWord + 4];
+    if (flags == 0u) return;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    if (flags & kStartOver) {
+        for (size_t i = (size_t)blockIdx.x * kRunThreads + tid; i < words; i += (size_t)gridDim.x * kRunThreads)
+            a.lookback[i] = 0u;
+        return;
+    }
+    constexpr uint32_t kRunWarps = kRunThreads / 32;
+    __shared__ uint32_t s_hist[kRunWarps][kRadix];
+    __shared__ uint32_t s_sum[kWarps];
+    const uint32_t w = a.counters[kScheduleWord], digits = a.counters[kScheduleWord + 1];
+    const uint32_t m = w & 255u, low = m - (w >> 8), listed = a.counters[kScheduleWord + 5];
+    const uint32_t n = a.d_count ? min(*a.d_count, a.n_est) : a.n_est;
+    const uint32_t top_shift = 8u * ((digits >> (4u * low)) & 15u);
+    const uint64_t mask = key_mask(a.key_bits);
+    const uint32_t lt = lanemask_lt();
+    uint32_t* const my_hist = s_hist[warp];
+    for (uint32_t r = blockIdx.x; r < listed; r += gridDim.x) {
+        // Where the run ends: its keys are a prefix of what follows, so 1,024
+        // places 32 apart and then 32 places tell. (What others do to their runs
+        // leaves the top digits as they are.)
+        const uint32_t first = a.runs[r];
+        const uint64_t head = __ldcg(a.keys_tmp + first) & mask;
+        const auto belongs = [&](uint32_t i) {
+            return first + i < n && (((__ldcg(a.keys_tmp + first + i) & mask) ^ head) >> top_shift) == 0ull;
+        };
+        const uint32_t base = 32u * ((uint32_t)__syncthreads_count(belongs(32u * tid)) - 1u);
+        const uint32_t len = base + __popc(__ballot_sync(kFullMask, belongs(base + lane)));
+        const uint32_t part = (len + kRunThreads - 1u) / kRunThreads * 32u;  // a warp's share
+        const uint32_t begin = min(len, warp * part), end = min(len, begin + part);
+        __syncthreads();  // all have read before any key moves
+        uint64_t *src = a.keys_tmp + first, *dst = a.keys_out + first;
+        uint32_t *src_val = a.vals_tmp + first, *dst_val = a.vals_out + first;
+        for (uint32_t d = 0; d < low; ++d) {
+            const uint32_t shift = 8u * ((digits >> (4u * d)) & 15u);
+#pragma unroll
+            for (uint32_t k = 0; k < kRadix / 32u; ++k) my_hist[32u * k + lane] = 0u;
+            __syncwarp();
+            for (uint32_t i = begin + lane; i < end; i += 32u)
+                atomicAdd(&my_hist[digit_of(__ldcg(src + i), shift, 0xFFu)], 1u);
+            __syncthreads();
+            uint32_t count = 0, incl = 0;
+            if (tid < kRadix) {
+                for (uint32_t k = 0; k < kRunWarps; ++k) count += s_hist[k][tid];
+                incl = count;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+                    if (lane >= (uint32_t)o) incl += y;
+                }
+                if (lane == 31u) s_sum[warp] = incl;
+            }
+            __syncthreads();
+            if (tid < kRadix) {
+                uint32_t run = incl - count;
+                for (uint32_t k = 0; k < warp; ++k) run += s_sum[k];
+                for (uint32_t k = 0; k < kRunWarps; ++k) {
+                    const uint32_t c = s_hist[k][tid];
+                    s_hist[k][tid] = run;
+                    run += c;
+                }
+            }
+            __syncthreads();
+            for (uint32_t i0 = begin; i0 < end; i0 += 32u) {
+                const uint32_t i = i0 + lane;
+                const bool valid = i < end;
+                const uint64_t key = valid ? __ldcg(src + i) : 0ull;
+                const uint32_t val = valid ? __ldcg(src_val + i) : 0u;
+                const uint32_t at = warp_rank(my_hist, digit_of(key, shift, 0xFFu), valid,
+                                              __ballot_sync(kFullMask, valid), lane, lt);
+                if (valid) {
+                    dst[at] = key;
+                    dst_val[at] = val;
+                }
+            }
+            __syncthreads();
+            uint64_t* const k = src;
+            src = dst, dst = k;
+            uint32_t* const v = src_val;
+            src_val = dst_val, dst_val = v;
+        }
+        if (src != a.keys_out + first)
+            for (uint32_t i = tid; i < len; i += kRunThreads) {
+                dst[i] = __ldcg(src + i);
+                dst_val[i] = __ldcg(src_val + i);
+            }
+        __syncthreads();
+    }
 }
 
 // Pass-kernel variants (threads, items per thread, blocks per SM). The numbers
@@ -761,16 +859,17 @@ cudaError_t sort_launch(const uint64_t* keys_in, const uint32_t* vals_in, uint64
                                                                     hist, excl, counters, apart, try_top, keys_tmp);
     const size_t stride = (size_t)plan.ntiles * kRadix;
     const SortArgs args{keys_in,  vals_in, keys_tmp, keys_out, vals_tmp, vals_out, d_count, n_est,
-                        key_bits, excl,    lookback, stride,   counters, early,    err,     spin_limit};
+                        key_bits, excl,    lookback, stride,   counters, early,    lookback + (size_t)kTopDigits * stride,
+                        err,      spin_limit};
     // Where the top digits may suffice: as many passes, the fix-up, and launches
-    // for all passes, which a schedule without top digits goes on with and a fix-up
-    // that gave up starts over with. A launch with nothing to do takes about 2 us.
+    // for all passes, which a schedule without top digits goes on with and a run that
+    // is too long starts over with. A launch with nothing to do takes about 2 us.
     for (uint32_t l = 0; l < plan.passes + early; ++l) {
         if (try_top && l == early) {
             const uint32_t tiles = (n_est - 1u) / kFixTile + 1u;
             if (key_bits < 64u) fixup_kernel<true><<<tiles, kThreads, 0, st>>>(args);
             else fixup_kernel<false><<<tiles, kThreads, 0, st>>>(args);
-            refill_kernel<<<num_sms(), kThreads, 0, st>>>(args, plan.passes * stride);
+            runs_kernel<<<2 * num_sms(), kRunThreads, 0, st>>>(args, plan.passes * stride);
         }
         pv.kernel<<<grid, pv.threads, pv.smem, st>>>(args, l);
     }
