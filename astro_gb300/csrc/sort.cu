@@ -52,16 +52,17 @@ constexpr uint32_t kDoneWord = 8, kScheduleWord = 10, kTicketWord = 16;
 // is sorted by a block of its own (runs_kernel); should one be longer than kRunMax,
 // all m digits are sorted from the input after all.
 //
-// 63-bit keys without / with it: uniform ones, 1,500,000 194 / 172 us, 2,097,152
-// 226 / 167, 16,777,216 1005 / 526 (262,144 122 / 136, so not below kTopMin).
-// Keys of clustered particles do not qualify and pay for the question: 48 bits,
-// 5,000,000 298 / 310. Uniform keys of 48 bits but for one place that holds 500 or
-// 5,000 of them, 2,000,000: 265 and 278 us when every long run had all digits
-// sorted, 161 and 191 with blocks for them (155 without the place). (Four or five
-// top digits let clustered 63-bit keys qualify, 5,000,000 399 -> 370 us, but with
-// longer runs.)
+// 63-bit keys without / with it: uniform ones, 2,097,152 226 / 167 us, 16,777,216
+// 1005 / 526. Keys of clustered particles do not qualify and pay for the question
+// and its idle launches: 48 bits, 5,000,000 298 / 310, 1,400,000 140 / 161 (146
+// before the resident passes), so not below kTopMin: uniform ones of 63 bits lose by
+// that, 1,400,000 181 / 148, but no keys are slower than they were. Uniform keys of
+// 48 bits but for one place that holds 500 or 5,000 of them, 2,000,000: 265 and 278
+// us when every long run had all digits sorted, 161 and 191 with blocks for them (155
+// without the place). (Four or five top digits let clustered 63-bit keys qualify,
+// 5,000,000 399 -> 370 us, but with longer runs.)
 constexpr uint32_t kTopDigits = 3, kSavedPasses = 3;  // of at least 6 digits
-constexpr uint32_t kTopMin = 5u << 18;
+constexpr uint32_t kTopMin = 3u << 19;
 constexpr float kNeighbours = 4.f;
 constexpr uint32_t kSamples = 4096, kSampleSlots = 2 * kSamples;
 constexpr uint32_t kFixTile = 2048, kFixHalo = 128;
