@@ -71,32 +71,6 @@ constexpr uint32_t kLongRuns = 1u, kStartOver = 2u;
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// Exclusive scan of one value per thread over a 256-thread block.
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s_warp) {
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(kFullMask, x, o);
-        if (lane >= (uint32_t)o) x += y;
-    }
-    if (lane == 31) s_warp[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kWarps ? s_warp[lane] : 0u;
-#pragma unroll
-        for (int o = 1; o < kWarps; o <<= 1) {
-            uint32_t y = __shfl_up_sync(kFullMask, w, o);
-            if (lane >= (uint32_t)o) w += y;
-        }
-        if (lane < kWarps) s_warp[lane] = w;
-    }
-    __syncthreads();
-    uint32_t r = (warp ? s_warp[warp - 1] : 0u) + x - v;
-    __syncthreads();
-    return r;
-}
-
 // The digit of a pass. Passes start at multiples of 8 bits, so a digit lies in
 // one word of the key.
 __device__ __forceinline__ uint32_t digit_of(uint64_t key, uint32_t shift, uint32_t dmask) {
@@ -191,7 +165,6 @@ __global__ __launch_bounds__(kThreads, kHistBlocksPerSm) void sort_histogram_ker
     uint32_t key_bits, uint32_t passes, uint32_t* __restrict__ hist, uint32_t* __restrict__ excl,
     uint32_t* __restrict__ counters, bool skip_shared, bool try_top, uint64_t* __restrict__ samples) {
     extern __shared__ uint32_t s_hist[];  // [kHistCopies][passes][kRadix]
-    __shared__ uint32_t s_warp[kWarps];
     __shared__ bool s_last;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t n = d_count ? min(*d_count, n_est) : n_est;
@@ -249,20 +222,46 @@ __global__ __launch_bounds__(kThreads, kHistBlocksPerSm) void sort_histogram_ker
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    __shared__ float s_agree[kMaxPasses];  // chance that two keys have the same digit
-    if (tid < kMaxPasses) s_agree[tid] = 0.f;
-    uint32_t m = 0, digits = 0;
-#pragma unroll 1
-    for (uint32_t p = 0; p < passes; ++p) {
-        uint32_t c = __ldcg(&hist[p * kRadix + tid]);
-        excl[p * kRadix + tid] = block_exclusive_scan(c, s_warp);
-        float f = (float)c / (float)n;
-        f *= f;
+    // A warp each turns a digit's counts into offsets, eight counts a lane (the block
+    // for one digit after the other took 2 us more for six of them: 200,000 pairs of
+    // 48 bits 80 -> 76).
+    __shared__ float s_agree[kMaxPasses];   // chance that two keys have the same digit
+    __shared__ bool s_shared[kMaxPasses];   // all keys have the same digit
+    static_assert(kWarps == kMaxPasses && kRadix == 8 * 32, "a warp a pass");
+    if (warp < passes) {
+        const uint4* from = reinterpret_cast<const uint4*>(hist + warp * kRadix) + 2u * lane;
+        uint4* to = reinterpret_cast<uint4*>(excl + warp * kRadix) + 2u * lane;
+        const uint4 x = __ldcg(from), y = __ldcg(from + 1);
+        const uint32_t c[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+        uint32_t o[8], run = 0;
+        float agree = 0.f;
+        bool all = false;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(kFullMask, f, o);
-        if (lane == 0) atomicAdd(&s_agree[p], f);
-        if (__syncthreads_or(c == n) == 0 || !skip_shared) digits |= p << (4u * m++);
+        for (int k = 0; k < 8; ++k) {
+            o[k] = run;
+            run += c[k];
+            all |= c[k] == n;
+            const float f = (float)c[k] / (float)n;
+            agree += f * f;
+        }
+        uint32_t incl = run;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t z = __shfl_up_sync(kFullMask, incl, d);
+            if (lane >= (uint32_t)d) incl += z;
+        }
+        const uint32_t before = incl - run;
+        to[0] = make_uint4(before + o[0], before + o[1], before + o[2], before + o[3]);
+        to[1] = make_uint4(before + o[4], before + o[5], before + o[6], before + o[7]);
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) agree += __shfl_xor_sync(kFullMask, agree, d);
+        all = __any_sync(kFullMask, all);
+        if (lane == 0) s_agree[warp] = agree, s_shared[warp] = all;
     }
+    __syncthreads();
+    uint32_t m = 0, digits = 0;
+    for (uint32_t p = 0; p < passes; ++p)
+        if (!s_shared[p] || !skip_shared) digits |= p << (4u * m++);
     if (m == 0) m = 1;  // equal keys: one pass copies them
     uint32_t top = 0;
     if (try_top && n >= kTopMin && m >= kTopDigits + kSavedPasses) {
@@ -698,11 +697,13 @@ constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 constexpr int kMinItems = 8;  // sizes the look-back words for every variant
 static_assert(kThreads * kMinItems == (int)kSortPlanTile, "look-back sizing");
 int g_variant = -1;  // the variant that serves where the caller names none; negative: by the number of pairs
-// Small tiles while they all run at once, then fewer and larger ones, which have
-// fewer earlier tiles to look back on. 63-bit keys, 8 / 16 / 20 a thread, us:
-// 262,144 pairs 104 / 120 / 119; 524,288 125 / 126 / 125; 2,097,152 268 / 236 /
-// 253; 16,777,216 1256 / 1128 / 1091.
-int variant_for(uint32_t n) { return n < (1u << 19) ? 3 : (n < (1u << 23) ? 0 : 4); }
+// Small tiles while they all run at once (with room for their registers: at four
+// blocks an SM a tile takes longer), then fewer and larger ones, which have fewer
+// earlier tiles to look back on. 63-bit keys, 8 a thread at three / four blocks, 16,
+// us: 150,000 pairs 80 / 92 / 96; 350,000 98 / 107 / 98 (110 before the resident
+// passes, which at four blocks were slower than those from 400,000 to 524,287);
+// 524,288 106 / 119 / 102. 16 / 20 a thread: 2,097,152 236 / 253; 16,777,216 1128 / 1091.
+int variant_for(uint32_t n) { return n < (1u << 19) ? 6 : (n < (1u << 23) ? 0 : 4); }
 
 // Per-device set-up state: the pass kernels' shared-memory attribute is set
 // once on each device that sorts, and the SM count is cached per device.

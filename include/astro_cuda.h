@@ -179,7 +179,7 @@ typedef struct astro_params {
                                  1..64; 0 = 32 */
     uint32_t sort_variant;    /* radix sort pass kernel (threads x items per
                                  thread / blocks per SM): 0 = library default
-                                 (4, 1 or 5 by the number of pairs),
+                                 (7, 1 or 5 by the number of pairs),
                                  1 = 256x16/2, 2 = 384x12/2, 3 = 512x12/1,
                                  4 = 256x8/4, 5 = 256x20/2, 6 = 256x12/3,
                                  7 = 256x8/3; 8 to 12 are kept for settings
