@@ -95,7 +95,9 @@ __device__ __forceinline__ uint32_t next_block(const TraverseArgs& a, ListOut& L
 
 // Writes the first n items (at most a block) of a list's buffer to the pool
 // and moves what lies behind the block to the buffer's front: node ids (first
-// words), 64 a block, or ranges, 32 a block.
+// words), 64 a block, or ranges, 32 a block. All lanes move a word, also where
+// nothing is left: the warp waits before it returns, since other lanes put the
+// next items into the same words and only a barrier orders the two stores.
 __device__ __forceinline__ void write_ids(const TraverseArgs& a, ListOut& L, BlockCache& bc,
                                           uint2* buf, uint32_t lane, uint32_t n) {
     const uint32_t blk = next_block(a, L, bc, lane, n);
@@ -108,6 +110,7 @@ __device__ __forceinline__ void write_ids(const TraverseArgs& a, ListOut& L, Blo
     const uint2 rest = buf[kListBlockWords + lane];
     __syncwarp();
     buf[lane] = rest;
+    __syncwarp();
 }
 __device__ __forceinline__ void write_ranges(const TraverseArgs& a, ListOut& L, BlockCache& bc,
                                              uint2* buf, uint32_t lane, uint32_t n) {
@@ -118,6 +121,7 @@ __device__ __forceinline__ void write_ranges(const TraverseArgs& a, ListOut& L, 
     const uint2 rest = buf[32u + lane];
     __syncwarp();
     buf[lane] = rest;
+    __syncwarp();
 }
 // The same for n <= 32 runs of the next frontier, at position `at` of nxt; a
 // frontier buffer that is too small records what it wanted and drops them.
@@ -134,6 +138,7 @@ __device__ __forceinline__ uint32_t write_runs(const TraverseArgs& a, uint2* nxt
     const uint2 rest = buf[32u + lane];
     __syncwarp();
     buf[lane] = rest;
+    __syncwarp();
     return fits ? at + n : at;
 }
 
