@@ -25,10 +25,12 @@
 namespace astro {
 namespace {
 
-// The packed loops need no self test and may sum massless padding when a
-// source at distance zero gives a finite factor m / eps^3 (times a zero
-// offset or a zero mass): eps^2 >= 2^-80 keeps 1 / eps^3 <= 2^120. Every
-// r^2 is then a normal float, so rsqrt_ftz applies.
+// The packed loops need no self test and may sum massless particles as padding:
+// a source at distance zero adds its factor m / eps^3 times a zero offset, and
+// eps^2 >= 2^-80 keeps 1 / eps^3 at most 2^120 (the factor is finite for masses
+// below 2^128 eps^3, 256 at the bound). Every r^2 is then a normal float, so
+// rsqrt_ftz applies. A quadrupole's factor 1 / r^5 is finite from 2e-8 only, so
+// cells are padded with a massless one where a listed cell lies, not at the origin.
 constexpr float kPackedMinEps2 = 8.2718061e-25f;  // 2^-80
 
 // Clamp, acceleration and kick-drift of particle i (updateSpheres' v += a dt,
@@ -282,7 +284,7 @@ __device__ __forceinline__ uint32_t sum_lists(const TraverseArgs& a, uint2 gr, c
     t.clear();
 
     // Cells, one list block (64) at a time: gathered into shared memory,
-    // zero (massless) past the list's end. The next block's ids are loaded
+    // massless at the first one's place past the list's end. The next block's ids are loaded
     // before the current block is summed.
     if (d.n_cell > 0) {
         uint32_t blk = d.cell_first, left = d.n_cell;
@@ -308,6 +310,13 @@ __device__ __forceinline__ uint32_t sum_lists(const TraverseArgs& a, uint2 gr, c
                         qyz[h] = __ldg(&a.node_qyz[nd]);
                     }
                 }
+            }
+            if (m < kListBlockWords) {
+                const float4 pad = make_float4(__shfl_sync(kFullMask, cm[0].x, 0), __shfl_sync(kFullMask, cm[0].y, 0),
+                                               __shfl_sync(kFullMask, cm[0].z, 0), 0.f);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (lane + 32u * h >= m) cm[h] = pad;
             }
             __syncwarp();
 #pragma unroll
