@@ -13,7 +13,7 @@
 //   list into four or eight parts.
 // group_eval_general_kernel — the exact form (every operation rounded as the
 //   CPU restatement rounds it, in its order), and the fast form where eps^2
-//   is too small for the packed loops (a particle's own entry is skipped).
+//   is no normal float (a particle's own entry is skipped).
 #include <algorithm>
 #include <mutex>
 
@@ -29,8 +29,12 @@ namespace {
 // a source at distance zero adds its factor m / eps^3 times a zero offset, and
 // eps^2 >= 2^-80 keeps 1 / eps^3 at most 2^120 (the factor is finite for masses
 // below 2^128 eps^3, 256 at the bound). Every r^2 is then a normal float, so
-// rsqrt_ftz applies. A quadrupole's factor 1 / r^5 is finite from 2e-8 only, so
-// cells are padded with a massless one where a listed cell lies, not at the origin.
+// rsqrt_ftz applies. Below the bound, down to the smallest normal eps^2, the loops
+// multiply the offset by 1/r three times and the mass last (kTiny), which stays
+// finite: three more products a pair, a step of a 50,000-body disk at eps 5e-13 in
+// groups of 32 483 us against 1,416 in the general kernel. A quadrupole's factor
+// 1 / r^5 is finite from 2e-8 only, so cells are padded with a massless one where a
+// listed cell lies, not at the origin.
 constexpr float kPackedMinEps2 = 8.2718061e-25f;  // 2^-80
 
 // Clamp, acceleration and kick-drift of particle i (updateSpheres' v += a dt,
@@ -154,7 +158,7 @@ struct PairSet {
 };
 
 // One source against the first kPairs pairs: m d / (r^2 + eps^2)^(3/2) without G.
-template <int kPairs>
+template <int kPairs, bool kTiny>
 __device__ __forceinline__ void add_source(PairSet& t, float4 p, float2 e2) {
 #pragma unroll
     for (int q = 0; q < kPairs; ++q) {
@@ -163,11 +167,18 @@ __device__ __forceinline__ void add_source(PairSet& t, float4 p, float2 e2) {
         const float2 dz = make_float2(p.z + t.nz[q].x, p.z + t.nz[q].y);
         const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
         const float2 inv = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
-        const float2 inv3 = __fmul2_rn(__fmul2_rn(inv, inv), inv);
-        const float2 sc = make_float2(p.w * inv3.x, p.w * inv3.y);
-        t.sx[q] = __ffma2_rn(dx, sc, t.sx[q]);
-        t.sy[q] = __ffma2_rn(dy, sc, t.sy[q]);
-        t.sz[q] = __ffma2_rn(dz, sc, t.sz[q]);
+        if constexpr (kTiny) {
+            const float2 u = __fmul2_rn(inv, inv), m = make_float2(p.w, p.w);
+            t.sx[q] = __ffma2_rn(__fmul2_rn(__fmul2_rn(dx, inv), u), m, t.sx[q]);
+            t.sy[q] = __ffma2_rn(__fmul2_rn(__fmul2_rn(dy, inv), u), m, t.sy[q]);
+            t.sz[q] = __ffma2_rn(__fmul2_rn(__fmul2_rn(dz, inv), u), m, t.sz[q]);
+        } else {
+            const float2 inv3 = __fmul2_rn(__fmul2_rn(inv, inv), inv);
+            const float2 sc = make_float2(p.w * inv3.x, p.w * inv3.y);
+            t.sx[q] = __ffma2_rn(dx, sc, t.sx[q]);
+            t.sy[q] = __ffma2_rn(dy, sc, t.sy[q]);
+            t.sz[q] = __ffma2_rn(dz, sc, t.sz[q]);
+        }
     }
 }
 
@@ -233,24 +244,24 @@ __device__ __forceinline__ void flush(FastSmem<kPrec>& sm, PairSet& t, uint32_t 
 }
 
 // The staged cells (count padded to the copies) or particles of one copy.
-template <bool kQuad, int kPairs>
+template <bool kQuad, bool kTiny, int kPairs>
 __device__ __forceinline__ void sum_cells(PairSet& t, const float* cell, uint32_t copies,
                                           uint32_t iters, float2 e2) {
     constexpr int kUnroll = kPairs == 1 ? 2 : 1;
 #pragma unroll kUnroll
     for (uint32_t i = 0; i < iters; ++i) {
         if constexpr (kQuad) add_cell_quad<kPairs>(t, cell, e2);
-        else add_source<kPairs>(t, *reinterpret_cast<const float4*>(cell), e2);
+        else add_source<kPairs, kTiny>(t, *reinterpret_cast<const float4*>(cell), e2);
         cell += copies * (kQuad ? kCellWords : 4);
     }
 }
-template <int kPairs>
+template <bool kTiny, int kPairs>
 __device__ __forceinline__ void sum_tile(PairSet& t, const float4* src, uint32_t copies,
                                          uint32_t iters, float2 e2) {
     constexpr int kUnroll = kPairs == 1 ? 4 : (kPairs == 2 ? 2 : 1);
 #pragma unroll kUnroll
     for (uint32_t i = 0; i < iters; ++i) {
-        add_source<kPairs>(t, *src, e2);
+        add_source<kPairs, kTiny>(t, *src, e2);
         src += copies;
     }
 }
@@ -259,7 +270,7 @@ __device__ __forceinline__ void sum_tile(PairSet& t, const float4* src, uint32_t
 // slot + width * k, k = 0 .. 2 pairs - 1, and its copy takes every
 // copies-th source (width 4: eight copies; width 8: four). Returns the
 // particles listed.
-template <bool kPrec, bool kQuad>
+template <bool kPrec, bool kQuad, bool kTiny>
 __device__ __forceinline__ uint32_t sum_lists(const TraverseArgs& a, uint2 gr, const GroupDesc& d,
                                               FastSmem<kPrec>& sm, uint32_t lane, uint32_t width,
                                               uint32_t pairs) {
@@ -341,10 +352,10 @@ __device__ __forceinline__ uint32_t sum_lists(const TraverseArgs& a, uint2 gr, c
             }
             const uint32_t iters = (m + copies - 1u) / copies;
             const float* cell = sm.u.cell + copy * (kQuad ? kCellWords : 4);
-            if (pairs == 4u) sum_cells<kQuad, 4>(t, cell, copies, iters, e2);
-            else if (pairs == 3u) sum_cells<kQuad, 3>(t, cell, copies, iters, e2);
-            else if (pairs == 2u) sum_cells<kQuad, 2>(t, cell, copies, iters, e2);
-            else sum_cells<kQuad, 1>(t, cell, copies, iters, e2);
+            if (pairs == 4u) sum_cells<kQuad, kTiny, 4>(t, cell, copies, iters, e2);
+            else if (pairs == 3u) sum_cells<kQuad, kTiny, 3>(t, cell, copies, iters, e2);
+            else if (pairs == 2u) sum_cells<kQuad, kTiny, 2>(t, cell, copies, iters, e2);
+            else sum_cells<kQuad, kTiny, 1>(t, cell, copies, iters, e2);
             flush(sm, t, lane, pairs);
             if (left == 0) break;
         }
@@ -409,10 +420,10 @@ __device__ __forceinline__ uint32_t sum_lists(const TraverseArgs& a, uint2 gr, c
             __syncwarp();
             const uint32_t iters = (cur + copies - 1u) / copies;
             const float4* src = sm.u.tile[b ^ 1] + copy;
-            if (pairs == 4u) sum_tile<4>(t, src, copies, iters, e2);
-            else if (pairs == 3u) sum_tile<3>(t, src, copies, iters, e2);
-            else if (pairs == 2u) sum_tile<2>(t, src, copies, iters, e2);
-            else sum_tile<1>(t, src, copies, iters, e2);
+            if (pairs == 4u) sum_tile<kTiny, 4>(t, src, copies, iters, e2);
+            else if (pairs == 3u) sum_tile<kTiny, 3>(t, src, copies, iters, e2);
+            else if (pairs == 2u) sum_tile<kTiny, 2>(t, src, copies, iters, e2);
+            else sum_tile<kTiny, 1>(t, src, copies, iters, e2);
             flush(sm, t, lane, pairs);
             __syncwarp();
         }
@@ -428,7 +439,7 @@ __device__ __forceinline__ uint32_t sum_lists(const TraverseArgs& a, uint2 gr, c
 // and 637 at five (96); 16,777,216-body cube 14.44, 15.64 and 14.64 ms.
 constexpr int kFastBlocks = 4;
 
-template <bool kPrec, bool kQuad>
+template <bool kPrec, bool kQuad, bool kTiny>
 __global__ __launch_bounds__(kFastWarps * 32, kFastBlocks) void group_eval_fast_kernel(
     TraverseArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -455,7 +466,7 @@ __global__ __launch_bounds__(kFastWarps * 32, kFastBlocks) void group_eval_fast_
         const GroupDesc d = load_desc(dp);
         const uint32_t width = gcount > 32u ? 8u : 4u;
         const uint32_t pairs = (gcount + 2u * width - 1u) / (2u * width);
-        const uint32_t sources = sum_lists<kPrec, kQuad>(a, gr, d, sm, lane, width, pairs);
+        const uint32_t sources = sum_lists<kPrec, kQuad, kTiny>(a, gr, d, sm, lane, width, pairs);
         __syncwarp();
         // Each lane finishes up to two particles: the copies' sums, the
         // far-node expansion, G, and the kick-drift. A particle's own entry
@@ -508,7 +519,12 @@ struct CellSlot<false> {
 };
 
 // Evaluation of one group whose particles sit kPer per lane (kPer = 2:
-// particles lane and lane + 32), sources in list order.
+// particles lane and lane + 32), sources in list order. In the fast form a group of
+// at most 16 runs as 32 / gcount copies (lane = rep * gcount + particle), each
+// of which takes every reps-th source of a staged part; a part's sum is added (in
+// the precision form Kahan-added) once. Without softening, 50,000-body disk in
+// groups of 16, lists and far sums: 563 us, one copy 1,223; of 32 555
+// (1,178 with every term compensated by itself).
 template <bool kExact, bool kPrec, bool kQuad, int kPer>
 __device__ __forceinline__ void eval_group(const TraverseArgs& a, const uint2 gr, const GroupDesc& d,
                                            const float* __restrict__ far_co,
@@ -517,17 +533,19 @@ __device__ __forceinline__ void eval_group(const TraverseArgs& a, const uint2 gr
                                            uint32_t& far_inter) {
     const uint32_t gcount = gr.y - gr.x;
     const float g = a.g, eps2 = a.eps2;
+    const uint32_t reps = kExact || kPer == 2 ? 1u : 32u / gcount;
+    const uint32_t rep = kPer == 2 ? 0u : lane / gcount;
     uint32_t ip[kPer];
     bool valid[kPer];
     float4 me[kPer];
-    uint32_t owned = 0;
+    uint32_t owned = 0;  // particles whose counts this lane keeps
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-        const uint32_t slot = lane + 32u * k;
-        valid[k] = slot < gcount;
+        const uint32_t slot = kPer == 2 ? lane + 32u * k : lane - rep * gcount;
+        valid[k] = kPer == 2 ? slot < gcount : rep < reps;
         ip[k] = gr.x + slot;
         me[k] = valid[k] ? a.pos[ip[k]] : make_float4(0.f, 0.f, 0.f, 0.f);
-        owned += valid[k] ? 1u : 0u;
+        owned += valid[k] && rep == 0u ? 1u : 0u;
     }
 
     float fx[kPer], fy[kPer], fz[kPer];
@@ -546,7 +564,6 @@ __device__ __forceinline__ void eval_group(const TraverseArgs& a, const uint2 gr
     }
 
     // G: in every term of the exact form, once at the end otherwise.
-    const float gt = kExact ? g : 1.0f;
     Accum<kExact, kPrec> cells[kPer], leaves[kPer];
     ChainCursor ccur{d.cell_first};
     for (uint32_t c0 = 0; c0 < d.n_cell; c0 += (uint32_t)kGeneralCells) {
@@ -573,21 +590,52 @@ __device__ __forceinline__ void eval_group(const TraverseArgs& a, const uint2 gr
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
             if (!valid[k]) continue;
-            for (uint32_t e = 0; e < m; ++e) {
-                const CellSlot<kQuad>& cs = s_cell[e];
-                const float4 c = cs.cm;
-                const float dx = __fsub_rn(c.x, me[k].x), dy = __fsub_rn(c.y, me[k].y),
-                            dz = __fsub_rn(c.z, me[k].z);
-                const float r2t =
-                    __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-                float tx, ty, tz;
-                if constexpr (kQuad)
-                    cell_term<kExact>(dx, dy, dz, r2t, c.w, true, cs.q, cs.q2.x, gt, eps2, tx, ty, tz);
-                else
-                    cell_term<kExact>(dx, dy, dz, r2t, c.w, false, make_float4(0.f, 0.f, 0.f, 0.f),
-                                      0.f, gt, eps2, tx, ty, tz);
-                cells[k].push(tx, ty, tz);
-                cells[k].step();
+            if constexpr (kExact) {
+                for (uint32_t e = 0; e < m; ++e) {
+                    const CellSlot<kQuad>& cs = s_cell[e];
+                    const float4 c = cs.cm;
+                    const float dx = __fsub_rn(c.x, me[k].x), dy = __fsub_rn(c.y, me[k].y),
+                                dz = __fsub_rn(c.z, me[k].z);
+                    const float r2t =
+                        __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                    float tx, ty, tz;
+                    if constexpr (kQuad)
+                        cell_term<true>(dx, dy, dz, r2t, c.w, true, cs.q, cs.q2.x, g, eps2, tx, ty, tz);
+                    else
+                        cell_term<true>(dx, dy, dz, r2t, c.w, false, make_float4(0.f, 0.f, 0.f, 0.f),
+                                        0.f, g, eps2, tx, ty, tz);
+                    cells[k].push(tx, ty, tz);
+                    cells[k].step();
+                }
+            } else {
+                float px = 0.f, py = 0.f, pz = 0.f;
+#pragma unroll 2
+                for (uint32_t e = rep; e < m; e += reps) {
+                    const CellSlot<kQuad>& cs = s_cell[e];
+                    const float4 c = cs.cm;
+                    const float dx = c.x - me[k].x, dy = c.y - me[k].y, dz = c.z - me[k].z;
+                    const float inv = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2))));
+                    const float u = inv * inv, inv3 = u * inv;
+                    float sa = inv3 * c.w;
+                    if constexpr (kQuad) {
+                        // inv^3 (M + 5/2 u^2 d.Qd) d - inv^5 Qd, u = 1/r^2.
+                        const float4 q = cs.q;
+                        const float qyz = cs.q2.x, qzz = cs.q2.y;
+                        const float qx = fmaf(q.x, dx, fmaf(q.z, dy, q.w * dz));
+                        const float qy = fmaf(q.z, dx, fmaf(q.y, dy, qyz * dz));
+                        const float qz = fmaf(q.w, dx, fmaf(qyz, dy, qzz * dz));
+                        const float dqd = fmaf(dx, qx, fmaf(dy, qy, dz * qz));
+                        sa = inv3 * fmaf(2.5f * u * u, dqd, c.w);
+                        const float sb = -(inv3 * u);
+                        px = fmaf(sb, qx, px);
+                        py = fmaf(sb, qy, py);
+                        pz = fmaf(sb, qz, pz);
+                    }
+                    px = fmaf(sa, dx, px);
+                    py = fmaf(sa, dy, py);
+                    pz = fmaf(sa, dz, pz);
+                }
+                cells[k].add(px, py, pz);
             }
         }
         inter += owned * m;
@@ -638,16 +686,33 @@ __device__ __forceinline__ void eval_group(const TraverseArgs& a, const uint2 gr
 #pragma unroll
             for (int k = 0; k < kPer; ++k) {
                 if (!valid[k]) continue;
-                for (uint32_t q = 0; q < cnt; ++q) {
-                    if (s_jdx[q] != ip[k]) {
-                        const float4 p = s_tile[q];
-                        float tx, ty, tz;
-                        particle_term<kExact>(__fsub_rn(p.x, me[k].x), __fsub_rn(p.y, me[k].y),
-                                              __fsub_rn(p.z, me[k].z), p.w, gt, eps2, tx, ty, tz);
-                        leaves[k].push(tx, ty, tz);
-                        ++inter;
+                if constexpr (kExact) {
+                    for (uint32_t q = 0; q < cnt; ++q) {
+                        if (s_jdx[q] != ip[k]) {
+                            const float4 p = s_tile[q];
+                            float tx, ty, tz;
+                            particle_term<true>(__fsub_rn(p.x, me[k].x), __fsub_rn(p.y, me[k].y),
+                                                __fsub_rn(p.z, me[k].z), p.w, g, eps2, tx, ty, tz);
+                            leaves[k].push(tx, ty, tz);
+                            ++inter;
+                        }
+                        leaves[k].step();
                     }
-                    leaves[k].step();
+                } else {
+                    float px = 0.f, py = 0.f, pz = 0.f;
+#pragma unroll 4
+                    for (uint32_t q = rep; q < cnt; q += reps) {
+                        const float4 p = s_tile[q];
+                        const float dx = p.x - me[k].x, dy = p.y - me[k].y, dz = p.z - me[k].z;
+                        const float inv = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2))));
+                        const bool other = s_jdx[q] != ip[k];
+                        const float sc = other ? p.w * (inv * inv * inv) : 0.f;
+                        px = fmaf(dx, sc, px);
+                        py = fmaf(dy, sc, py);
+                        pz = fmaf(dz, sc, pz);
+                        inter += other ? 1u : 0u;
+                    }
+                    leaves[k].add(px, py, pz);
                 }
             }
             __syncwarp();
@@ -658,7 +723,6 @@ __device__ __forceinline__ void eval_group(const TraverseArgs& a, const uint2 gr
     for (int k = 0; k < kPer; ++k) {
         cells[k].finish();
         leaves[k].finish();
-        if (!valid[k]) continue;
         float sx, sy, sz;
         if (kExact) {
             sx = __fadd_rn(cells[k].ax, leaves[k].ax);
@@ -671,11 +735,27 @@ __device__ __forceinline__ void eval_group(const TraverseArgs& a, const uint2 gr
             }
         } else {
             // Compensated sums: the running sum minus its pending correction.
-            sx = ((cells[k].ax - cells[k].cx) + (leaves[k].ax - leaves[k].cx) + fx[k]) * g;
-            sy = ((cells[k].ay - cells[k].cy) + (leaves[k].ay - leaves[k].cy) + fy[k]) * g;
-            sz = ((cells[k].az - cells[k].cz) + (leaves[k].az - leaves[k].cz) + fz[k]) * g;
+            sx = (cells[k].ax - cells[k].cx) + (leaves[k].ax - leaves[k].cx);
+            sy = (cells[k].ay - cells[k].cy) + (leaves[k].ay - leaves[k].cy);
+            sz = (cells[k].az - cells[k].cz) + (leaves[k].az - leaves[k].cz);
+            if (reps > 1u) {  // the copies' sums, in the owner's lane
+                __syncwarp();
+                s_tile[lane] = make_float4(sx, sy, sz, 0.f);
+                __syncwarp();
+                if (rep == 0u)
+                    for (uint32_t r = 1; r < reps; ++r) {
+                        const float4 t = s_tile[lane + r * gcount];
+                        sx += t.x;
+                        sy += t.y;
+                        sz += t.z;
+                    }
+                __syncwarp();
+            }
+            sx = (sx + fx[k]) * g;
+            sy = (sy + fy[k]) * g;
+            sz = (sz + fz[k]) * g;
         }
-        store_particle<kPrec>(a, ip[k], me[k], sx, sy, sz);
+        if (valid[k] && rep == 0u) store_particle<kPrec>(a, ip[k], me[k], sx, sy, sz);
     }
 }
 
@@ -747,10 +827,10 @@ struct Persistent {
     }
 };
 
-template <bool kPrec, bool kQuad>
+template <bool kPrec, bool kQuad, bool kTiny>
 cudaError_t launch_fast(const TraverseArgs& a, cudaStream_t st) {
     static Persistent shape;
-    auto kernel = group_eval_fast_kernel<kPrec, kQuad>;
+    auto kernel = group_eval_fast_kernel<kPrec, kQuad, kTiny>;
     const size_t smem = sizeof(FastSmem<kPrec>) * kFastWarps;
     uint32_t blocks = 0;
     const cudaError_t e = shape.get((const void*)kernel, kFastWarps * 32, smem, &blocks);
@@ -773,8 +853,8 @@ cudaError_t launch_general(const TraverseArgs& a, cudaStream_t st) {
 template <bool kPrec, bool kQuad>
 cudaError_t launch_form(const TraverseArgs& a, bool exact, cudaStream_t st) {
     if (exact) return launch_general<true, kPrec, kQuad>(a, st);
-    return a.eps2 >= kPackedMinEps2 ? launch_fast<kPrec, kQuad>(a, st)
-                                    : launch_general<false, kPrec, kQuad>(a, st);
+    if (a.eps2 >= kPackedMinEps2) return launch_fast<kPrec, kQuad, false>(a, st);
+    return a.eps2 >= kFltMin ? launch_fast<kPrec, kQuad, true>(a, st) : launch_general<false, kPrec, kQuad>(a, st);
 }
 
 }  // namespace
