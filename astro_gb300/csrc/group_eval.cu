@@ -102,7 +102,7 @@ __device__ __forceinline__ void add_stats(const TraverseArgs& a, uint32_t lane,
 // loop of its own. What can be saved is idle lanes and everything around that loop:
 // - Pairs are of two particles, not of two sources: a lane holds up to eight
 //   particles and the warp's lanes split each list into 32 / width parts, so
-//   a group of g <= 32 costs ceil(g / 8) / 8 of a pass over the lists per lane
+//   a group of 5 <= g <= 32 costs ceil(g / 8) / 8 of a pass over the lists per lane
 //   and one of g <= 64 ceil(g / 16) / 4 (one particle a lane: 1 for every g
 //   from 17 to 32). Sums, positions and the source take half the registers
 //   that source pairs took, and four independent pairs hide the latencies.
@@ -268,8 +268,8 @@ __device__ __forceinline__ void sum_tile(PairSet& t, const float4* src, uint32_t
 
 // The lists of one group: lane = copy * width + slot holds the particles
 // slot + width * k, k = 0 .. 2 pairs - 1, and its copy takes every
-// copies-th source (width 4: eight copies; width 8: four). Returns the
-// particles listed.
+// copies-th source (width 8: four copies; 4: eight; 2 and 1: 16 and 32). Returns
+// the particles listed.
 template <bool kPrec, bool kQuad, bool kTiny>
 __device__ __forceinline__ uint32_t sum_lists(const TraverseArgs& a, uint2 gr, const GroupDesc& d,
                                               FastSmem<kPrec>& sm, uint32_t lane, uint32_t width,
@@ -464,7 +464,11 @@ __global__ __launch_bounds__(kFastWarps * 32, kFastBlocks) void group_eval_fast_
         // The walk of the leaf's first chunk.
         const GroupDesc* dp = a.desc + (gi - rec.w);
         const GroupDesc d = load_desc(dp);
-        const uint32_t width = gcount > 32u ? 8u : 4u;
+        // Groups of one to four fill fewer slots, so more lanes split the lists
+        // (50,000-body sphere in groups of 1 / 2 / 4, lists alone: four slots
+        // 627 / 387 / 227 us, 446 / 283 / 172 so; one lane a particle and copy 453 /
+        // 301 / 201).
+        const uint32_t width = gcount > 32u ? 8u : (gcount > 4u ? 4u : (gcount > 2u ? 2u : 1u));
         const uint32_t pairs = (gcount + 2u * width - 1u) / (2u * width);
         const uint32_t sources = sum_lists<kPrec, kQuad, kTiny>(a, gr, d, sm, lane, width, pairs);
         __syncwarp();
