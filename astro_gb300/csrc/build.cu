@@ -843,8 +843,10 @@ __device__ __forceinline__ void aggregate_internal(const AggArgs& a, uint32_t l,
 // 481 -> 342 us, 256 systems 590 -> 424 us, 524,288-body disk 146 -> 105 us.
 // Work lists in every layer: disk 14 us more; in none: merger 64 us, 21 bits
 // 0.7 ms more; the whole tree in one climbing launch: merger 594 us, disk 124 us.
-constexpr uint32_t kLayerMinNodes = 32768;
+// The top layer, too, is a launch of its own where there are that many systems.
+constexpr uint32_t kLayerMinNodes = 24576;
 constexpr uint32_t kWorkMinNodes = 1u << 20;
+static_assert(kWorkMinNodes > ASTRO_MAX_SYSTEMS, "all nodes of the top layer are looked at, for the groups");
 
 // The children [cb, ce) of node jp of layer l (u nodes there, `below` nodes
 // one layer down).
@@ -917,21 +919,25 @@ __global__ __launch_bounds__(128) void aggregate_internal_kernel(AggArgs a, uint
         Children c{0u, 0u};
         NodeRec<kPrec> r;
         r.pb = r.pe = 0;
-        bool several = false;
+        bool several = false, root = false;
         if (i < count) {
             node = kWork ? a.work[a.offset[l] + i] : a.offset[l] + i;
             const uint32_t j = node - a.offset[l];
             c = children_of(a, node, j, u, l, a.layer_count[l - 1]);
             several = kWork || c.ce - c.cb != 1u;
-            if (several) {
+            if (several || l == a.lbits) {
                 r.pb = a.pbeg[node];
                 r.pe = (j + 1 < u) ? a.pbeg[node + 1] : a.n;
+            }
+            // The root of a system no larger than a group is a group by itself.
+            root = l == a.lbits && r.pe - r.pb <= a.group_size;
+            if (several) {
                 r.key = a.node_key[node];
                 aggregate_internal<kPrec, kQuad>(a, l, node, c.cb, c.ce, r);
             }
         }
-        if (__any_sync(kFullMask, r.pe - r.pb > a.group_size))
-            emit_groups(a, c.cb, r.pe - r.pb > a.group_size ? c.ce : c.cb, false, r.pb, r.pe);
+        const bool large = several && r.pe - r.pb > a.group_size;
+        if (__any_sync(kFullMask, large || root)) emit_groups(a, c.cb, large ? c.ce : c.cb, root, r.pb, r.pe);
         if (several) climb_chain<kPrec, kQuad>(a, l, node, top, work_top, r);
     }
 }
@@ -1553,7 +1559,7 @@ cudaError_t launch_topology(const TopoArgs& a, cudaStream_t st) {
 namespace {
 uint32_t top_first_layer(const LayerTable& t) {
     uint32_t l0 = 0;
-    while (l0 + 1 < t.n_layers && t.size[l0] >= kLayerMinNodes) ++l0;
+    while (l0 < t.n_layers && t.size[l0] >= kLayerMinNodes) ++l0;
     return l0;
 }
 
@@ -1602,7 +1608,7 @@ constexpr uint32_t kWorkBlocks = 152 * 16;  // several waves at any register cou
 template <bool kPrec, bool kQuad>
 cudaError_t launch_physical(const AggArgs& a, const LayerTable& t, cudaStream_t st) {
     const uint32_t t0 = 128, l0 = top_first_layer(t);
-    uint32_t lw = 0;  // layers below lw have work lists (sizes fall with the layer)
+    uint32_t lw = 0;  // layers below lw have work lists (sizes fall with the layer; not the top one's)
     while (lw < l0 && t.size[lw] >= kWorkMinNodes) ++lw;
     for (uint32_t l = 0; l < l0; ++l) {
         const uint32_t g = blocks_for(t.size[l], t0);
@@ -1614,7 +1620,7 @@ cudaError_t launch_physical(const AggArgs& a, const LayerTable& t, cudaStream_t 
         else e = launch_after(aggregate_internal_kernel<kPrec, kQuad, false>, g, t0, 0, st, a, l, l0, lw);
         if (e != cudaSuccess) return e;
     }
-    return launch_cluster(aggregate_top_kernel<kPrec, kQuad>, a, l0, st);
+    return l0 < t.n_layers ? launch_cluster(aggregate_top_kernel<kPrec, kQuad>, a, l0, st) : cudaSuccess;
 }
 }  // namespace
 
