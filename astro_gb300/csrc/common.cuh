@@ -70,7 +70,13 @@ __device__ __forceinline__ double ordered_to_f64(unsigned long long u) {
 // bodies 1,224 -> 1,187, a step of 16,384 bodies 143.0 -> 141.5. Not for walk, far
 // sums and evaluation, nor for the passes of larger sorts: blocks that wait beside
 // them cost a step of 524,288 bodies 1.5% and 0.7%, a sort of 16.7 M pairs 1.7%.
+//
+// A grid of more than kOverlapBlocks blocks is launched plainly and does neither:
+// waiting hides only the first blocks' start, and every block pays for it (encode of
+// 60,000 systems, a block each: 33 us before, 71 with the wait, 33 without).
+constexpr uint32_t kOverlapBlocks = 4864;  // 32 for each of 152 SMs
 __device__ __forceinline__ void after_previous() {
+    if (gridDim.x > kOverlapBlocks) return;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -83,7 +89,7 @@ cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
     cfg.stream = st;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+    attr.val.programmaticStreamSerializationAllowed = grid.x <= kOverlapBlocks ? 1 : 0;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
