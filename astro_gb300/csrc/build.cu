@@ -843,8 +843,12 @@ __device__ __forceinline__ void aggregate_internal(const AggArgs& a, uint32_t l,
 // 481 -> 342 us, 256 systems 590 -> 424 us, 524,288-body disk 146 -> 105 us.
 // Work lists in every layer: disk 14 us more; in none: merger 64 us, 21 bits
 // 0.7 ms more; the whole tree in one climbing launch: merger 594 us, disk 124 us.
-// The top layer, too, is a launch of its own where there are that many systems.
-constexpr uint32_t kLayerMinNodes = 24576;
+// Layers of 16,384 to 24,575 nodes by launches / in the cluster, us a step: cubes of
+// 20,000 bodies at 21 bits 198 / 255, of 24,000 at 8 bits 132 / 145 (but a sphere of
+// 16,384 at 8 bits 149 / 138, 256 systems with 16,384 nodes in a layer 8,050 / 7,864).
+// The top layer, too, is a launch of its own where there are that many systems
+// (24,000 of 16 bodies 244 / 260).
+constexpr uint32_t kLayerMinNodes = 18432;
 constexpr uint32_t kWorkMinNodes = 1u << 20;
 static_assert(kWorkMinNodes > ASTRO_MAX_SYSTEMS, "all nodes of the top layer are looked at, for the groups");
 

@@ -21,7 +21,7 @@ def _run(native, oracle, pm, vr, sizes, lbits, form, steps=2):
     assert out["interactions"] == ref["interactions"] and out["node_visits"] == ref["node_visits"]
 
 
-@pytest.mark.parametrize("nsys,most,lbits", [(24575, 12, 3), (24576, 12, 3), (24576, 1, 1), (33000, 20, 2),
+@pytest.mark.parametrize("nsys,most,lbits", [(18431, 12, 3), (18432, 12, 3), (24576, 1, 1), (33000, 20, 2),
                                              (65536, 3, 5)])
 @pytest.mark.parametrize("form", [0, 1])
 def test_top_layer_of_many_systems(native, oracle, nsys, most, lbits, form):
@@ -32,7 +32,7 @@ def test_top_layer_of_many_systems(native, oracle, nsys, most, lbits, form):
     _run(native, oracle, pm, vr, sizes, lbits, form)
 
 
-@pytest.mark.parametrize("n,lbits", [(24575, 21), (24576, 21), (24577, 9), (30001, 14), (32767, 21)])
+@pytest.mark.parametrize("n,lbits", [(18431, 21), (18432, 21), (24577, 9), (30001, 14), (32767, 21)])
 @pytest.mark.parametrize("form", [0, 1])
 def test_deep_trees_around_the_line(native, oracle, n, lbits, form):
     from astro_gb300 import ic
