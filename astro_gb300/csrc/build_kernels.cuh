@@ -252,7 +252,8 @@ struct SplatArgs {
     uint64_t* keys;          // fragments (pixel << id_bits | particle)
     uint32_t id_bits;        // bits that a particle's index needs
     uint32_t cap;
-    uint32_t* cursor;
+    uint32_t* cursor;        // [0] fragments, [1] and [2] listed primitives, from the front and the back
+    uint32_t* large;         // n words: primitives of too many pixels for a lane
     float4* image;           // width * height, row 0 = top
     float* depth;
 };

@@ -1384,7 +1384,7 @@ int astro_splat(astro_ctx* ctx, const astro_camera* camera, uint32_t width, uint
     cudaStream_t st = ctx->stream;
     if (!ctx->splat_prim) {
         CK(dev_alloc(&ctx->splat_prim, ctx->max_n));
-        CK(dev_alloc(&ctx->splat_kind, ctx->max_n + 1));  // + the fragment cursor
+        CK(dev_alloc(&ctx->splat_kind, 2ull * ctx->max_n + 3));  // + the cursors and the list
     }
     if (pixels > ctx->splat_pixels) {
         dev_free(ctx->splat_image);
@@ -1411,6 +1411,7 @@ int astro_splat(astro_ctx* ctx, const astro_camera* camera, uint32_t width, uint
     a.prim = ctx->splat_prim;
     a.kind = ctx->splat_kind;
     a.cursor = ctx->splat_kind + ctx->max_n;
+    a.large = a.cursor + 3;
     a.id_bits = std::max(1u, bits_for(ctx->n));
     a.image = ctx->splat_image;
     a.depth = ctx->splat_depth;
@@ -1420,7 +1421,7 @@ int astro_splat(astro_ctx* ctx, const astro_camera* camera, uint32_t width, uint
     for (int attempt = 0; attempt < 2; ++attempt) {
         a.keys = ctx->frag_keys;
         a.cap = ctx->frag_cap;
-        CK(cudaMemsetAsync(a.cursor, 0, sizeof(uint32_t), st));
+        CK(cudaMemsetAsync(a.cursor, 0, 3 * sizeof(uint32_t), st));
         CK(astro::launch_splat_emit(a, st));
         CK(cudaMemcpyAsync(&count, a.cursor, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));

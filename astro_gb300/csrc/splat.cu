@@ -94,12 +94,30 @@ __device__ __forceinline__ bool covers(uint32_t kind, float4 q, int px, int py) 
 // Fragments of 32 primitives per warp and round. A lane draws its own small
 // primitive (a box of at most kLaneCells pixels: dust points) - it counts the
 // pixels covered, the warp claims the slots of all its lanes with one atomic,
-// and the lane writes its keys; larger ones (discs) are then drawn one after
-// the other by the whole warp, one atomic for 32 pixels. Keys are
-// pixel << id_bits | particle; writes past cap are counted, not stored.
+// and the lane writes its keys. Larger ones go to a list from both ends: those of
+// up to kWarpCells pixels are drawn by a warp each afterwards, the rest in up to
+// kSlices parts of at least kPartCells (splat_emit_large_kernel). Keys are pixel << id_bits | particle; writes past
+// cap are counted, not stored.
 // One atomic per fragment on the one cursor took 185 us for 500,205 particles
-// (about two million fragments); one per 32 primitives 32 us.
-constexpr uint32_t kLaneCells = 64;
+// (about two million fragments); one per 32 primitives 32 us. With the large ones
+// drawn one after the other by the warp that met them, 3,000 points of 50 pixels took
+// 31.2 ms a picture and 300 that fill it 604 ms (11.2 and 38.3 with a warp for every
+// primitive); 1.9 and 15.1 now.
+constexpr uint32_t kLaneCells = 64, kWarpCells = 4096, kSlices = 256, kPartCells = 1024;
+
+struct Box {
+    int x0, y0;
+    uint32_t width, cells;  // (an image has at most 2^31 pixels)
+};
+__device__ __forceinline__ Box box_of(const SplatArgs& a, uint32_t kind, float4 q) {
+    const float h = kind == 2u ? __fmul_rn(q.w, 0.5f) : q.w;
+    int x0, x1, y0, y1;
+    span(q.x, h, a.width, x0, x1);
+    span(q.y, h, a.height, y0, y1);
+    if (x1 < x0 || y1 < y0) return Box{0, 0, 0u, 0u};
+    const uint32_t width = (uint32_t)(x1 - x0 + 1);
+    return Box{x0, y0, width, width * (uint32_t)(y1 - y0 + 1)};
+}
 
 __global__ __launch_bounds__(256) void splat_emit_kernel(SplatArgs a) {
     const uint32_t lane = threadIdx.x & 31u, lt = lanemask_lt();
@@ -107,21 +125,20 @@ __global__ __launch_bounds__(256) void splat_emit_kernel(SplatArgs a) {
     const uint32_t chunks = (a.n + 31u) / 32u;
     for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < chunks; c += warps) {
         const uint32_t i = c * 32u + lane;
-        uint32_t kind = i < a.n ? a.kind[i] : 0u;
+        const uint32_t kind = i < a.n ? a.kind[i] : 0u;
         const float4 q = kind ? a.prim[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float h = kind == 2u ? __fmul_rn(q.w, 0.5f) : q.w;
-        int x0 = 0, x1 = -1, y0 = 0, y1 = -1;
-        if (kind) {
-            span(q.x, h, a.width, x0, x1);
-            span(q.y, h, a.height, y0, y1);
-        }
-        if (x1 < x0 || y1 < y0) kind = 0u;
-        const uint64_t cells = kind ? (uint64_t)(uint32_t)(x1 - x0 + 1) * (uint32_t)(y1 - y0 + 1) : 0ull;
-        const bool small = cells <= kLaneCells;
+        const Box box = kind ? box_of(a, kind, q) : Box{0, 0, 0u, 0u};
+        const bool small = box.cells <= kLaneCells;
         uint32_t count = 0;
-        if (kind && small)
-            for (int py = y0; py <= y1; ++py)
-                for (int px = x0; px <= x1; ++px) count += covers(kind, q, px, py) ? 1u : 0u;
+        auto each = [&](auto&& draw) {
+            uint32_t x = 0, y = 0;
+            for (uint32_t k = 0; k < box.cells; ++k) {
+                const int px = box.x0 + (int)x, py = box.y0 + (int)y;
+                if (covers(kind, q, px, py)) draw(px, py);
+                if (++x == box.width) x = 0, ++y;
+            }
+        };
+        if (small) each([&](int, int) { ++count; });
         uint32_t incl = count;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -134,36 +151,62 @@ __global__ __launch_bounds__(256) void splat_emit_kernel(SplatArgs a) {
             if (lane == 0) base = atomicAdd(a.cursor, total);
             uint32_t slot = __shfl_sync(kFullMask, base, 0) + incl - count;
             if (count)
-                for (int py = y0; py <= y1; ++py)
-                    for (int px = x0; px <= x1; ++px) {
-                        if (!covers(kind, q, px, py)) continue;
-                        if (slot < a.cap)
-                            a.keys[slot] =
-                                ((uint64_t)((uint32_t)py * a.width + (uint32_t)px) << a.id_bits) | i;
-                        ++slot;
-                    }
+                each([&](int px, int py) {
+                    if (slot < a.cap)
+                        a.keys[slot] = ((uint64_t)((uint32_t)py * a.width + (uint32_t)px) << a.id_bits) | i;
+                    ++slot;
+                });
         }
-        for (uint32_t big = __ballot_sync(kFullMask, !small); big; big &= big - 1u) {
-            const uint32_t src = (uint32_t)__ffs(big) - 1u;
-            const uint32_t bkind = __shfl_sync(kFullMask, kind, src);
-            const float4 bq = make_float4(
-                __shfl_sync(kFullMask, q.x, src), __shfl_sync(kFullMask, q.y, src),
-                __shfl_sync(kFullMask, q.z, src), __shfl_sync(kFullMask, q.w, src));
-            const int bx = __shfl_sync(kFullMask, x0, src), by = __shfl_sync(kFullMask, y0, src);
-            const uint32_t bw = (uint32_t)(__shfl_sync(kFullMask, x1, src) - bx + 1);
-            const uint64_t bcells = __shfl_sync(kFullMask, cells, src);
-            for (uint64_t k0 = 0; k0 < bcells; k0 += 32u) {
-                const uint64_t k = k0 + lane;
-                const int px = bx + (int)(k % bw), py = by + (int)(k / bw);
-                const bool in = k < bcells && covers(bkind, bq, px, py);
-                const uint32_t m = __ballot_sync(kFullMask, in);
-                if (m == 0u) continue;
-                uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(a.cursor, (uint32_t)__popc(m));
-                const uint32_t slot = __shfl_sync(kFullMask, base, 0) + __popc(m & lt);
-                if (in && slot < a.cap)
-                    a.keys[slot] = ((uint64_t)((uint32_t)py * a.width + (uint32_t)px) << a.id_bits) |
-                                   (c * 32u + src);
+        const bool huge = box.cells > kWarpCells;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const bool mine = !small && huge == (e == 1);
+            const uint32_t m = __ballot_sync(kFullMask, mine);
+            if (m == 0u) continue;
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(a.cursor + 1 + e, (uint32_t)__popc(m));
+            const uint32_t at = __shfl_sync(kFullMask, base, 0) + __popc(m & lt);
+            if (mine) a.large[e == 0 ? at : a.n - 1u - at] = i;
+        }
+    }
+}
+
+// The listed primitives: a warp draws one, or one part of it, 128 pixels for an
+// atomic.
+__global__ __launch_bounds__(256) void splat_emit_large_kernel(SplatArgs a) {
+    const uint32_t lane = threadIdx.x & 31u, lt = lanemask_lt();
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t single = a.cursor[1];
+    const uint64_t items = single + (uint64_t)a.cursor[2] * kSlices;
+    for (uint64_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < items; t += warps) {
+        const bool whole = t < single;
+        const uint32_t i = a.large[whole ? (uint32_t)t : a.n - 1u - (uint32_t)((t - single) / kSlices)];
+        const uint32_t kind = a.kind[i];
+        const float4 q = a.prim[i];
+        const Box box = box_of(a, kind, q);
+        const uint32_t part = whole ? box.cells : max(kPartCells, (box.cells + kSlices - 1u) / kSlices);
+        const uint32_t begin = whole ? 0u : (uint32_t)min((t - single) % kSlices * part, (uint64_t)box.cells);
+        const uint32_t end = begin + min(part, box.cells - begin);
+        for (uint32_t k0 = begin; k0 < end; k0 += 128u) {
+            uint32_t m[4], cell[4], total = 0;
+#pragma unroll
+            for (uint32_t u = 0; u < 4u; ++u) {
+                const uint32_t k = k0 + 32u * u + lane;
+                const uint32_t y = k / box.width, x = k - y * box.width;
+                const int px = box.x0 + (int)x, py = box.y0 + (int)y;
+                m[u] = __ballot_sync(kFullMask, k < end && covers(kind, q, px, py));
+                cell[u] = (uint32_t)py * a.width + (uint32_t)px;
+                total += __popc(m[u]);
+            }
+            if (total == 0u) continue;
+            uint32_t slot = 0;
+            if (lane == 0) slot = atomicAdd(a.cursor, total);
+            slot = __shfl_sync(kFullMask, slot, 0);
+#pragma unroll
+            for (uint32_t u = 0; u < 4u; ++u) {
+                const uint32_t at = slot + __popc(m[u] & lt);
+                if ((m[u] >> lane & 1u) && at < a.cap) a.keys[at] = ((uint64_t)cell[u] << a.id_bits) | i;
+                slot += __popc(m[u]);
             }
         }
     }
@@ -219,6 +262,7 @@ cudaError_t launch_splat_emit(const SplatArgs& a, cudaStream_t st) {
     if (a.n == 0) return cudaSuccess;
     const uint32_t blocks = (uint32_t)std::min<uint64_t>(((uint64_t)a.n + 255) / 256, 152u * 64u);
     splat_emit_kernel<<<blocks, 256, 0, st>>>(a);
+    splat_emit_large_kernel<<<152u * 8u, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 
