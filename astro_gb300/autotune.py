@@ -6,7 +6,8 @@ it over the benchmark workloads and collects the results file.
 
 The knobs are fields of astro_params that change speed, not physics:
 
-  block_warps   traversal block size (warps per block: 4 or 8)
+  block_warps   per-particle traversal: block size (warps per block, 4 or 8);
+                the group walk's kernels have their own
   group_size    particles per warp: consecutive sorted particles sharing one
                 tree walk (1..64; the lanes hold pairs and split the source
                 lists)
@@ -14,8 +15,9 @@ The knobs are fields of astro_params that change speed, not physics:
   bucket        leaf tile size: an opened node holding <= bucket particles
                 is summed particle by particle
   sort_variant  radix sort pass kernel (threads, items per thread, blocks per
-                SM)
-  walk_frontier accepted for settings made earlier; both values walk alike
+                SM) of more than 65,536 particles
+  walk_frontier accepted for settings made earlier, not searched; both values
+                walk alike
 
   far_ratio     accepted nodes further than (group radius) / far_ratio from
                 the group's centre are summed through one second-order
@@ -33,8 +35,8 @@ theta, the softening, the quadrupole and opening-radius flags and the form
 
 Search: coordinate descent from the preset's defaults over the speed knobs,
 then every (open_delta_weight, far_ratio) pair (far_ratio rising until the
-error leaves its bound), then lbits, bucket, group_size, block_warps and
-walk_frontier once more. Each knob in turn is swept with the others fixed; the fastest setting
+error leaves its bound), then lbits, bucket, group_size and block_warps once
+more; a knob whose values would run the same kernels is left out. Each knob in turn is swept with the others fixed; the fastest setting
 is kept among those whose
 median relative acceleration error against the FP64 direct sum (on sampled
 particles) is at most max(target, 1.02 x the starting error) (max(0.8 x the
@@ -70,8 +72,8 @@ FORMS = {"plain": L.FORM_PLAIN, "precision": L.FORM_PRECISION}
 
 
 def candidates(knob: str, n: int) -> list[int]:
-    """The values the library's search tries for a knob (n: the largest
-    system's particle count)."""
+    """The values a knob may take in the library's search (n: the largest
+    system's particle count); of values that run the same kernels it tries one."""
     if knob == "lbits":
         # From about 8 particles per finest cell down to single occupancy.
         lo = max(3, int(np.ceil(np.log2(max(n, 8) / 8) / 3)))

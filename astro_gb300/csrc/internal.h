@@ -66,6 +66,7 @@ cudaError_t sort_pairs(const uint64_t* keys_in, const uint32_t* vals_in, uint64_
                        uint32_t key_bits, void* temp, size_t temp_bytes, cudaStream_t st,
                        uint32_t* err, uint32_t variant = 0);
 uint32_t sort_variant_count();
+uint32_t sort_shape_count();  // the first so many variants differ
 // The one-launch sort of up to sort_small_max(device) pairs (sort_small.cu);
 // clear_err: a word to zero, or NULL.
 cudaError_t sort_small_init(int dev);

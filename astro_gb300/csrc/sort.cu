@@ -770,6 +770,7 @@ cudaError_t sort_init() {
 }
 
 uint32_t sort_variant_count() { return (uint32_t)kNumVariants; }
+uint32_t sort_shape_count() { return 7u; }
 
 SortPlan sort_plan(uint32_t max_len, uint32_t key_bits) {
     SortPlan p{};

@@ -5,14 +5,15 @@
 // move, so every trial sees the same input) on the context's own particles
 // and measures each setting's median relative acceleration error against
 // the FP64 direct sum on sampled particles. Search: coordinate descent over
-// the speed knobs (lbits, bucket, group_size, block_warps, sort_variant,
-// walk_frontier),
+// the speed knobs (lbits, bucket, group_size, block_warps, sort_variant),
 // keeping the fastest setting whose error stays within
 // max(target, 1.02 x the starting error); then every (open_delta_weight,
 // far_ratio) pair, far_ratio rising until the error leaves
 // max(0.8 x target, 1.02 x the starting error); then lbits, bucket,
-// group_size, block_warps and walk_frontier once more within that bound. sort_variant is
-// judged by the sort stage's own time. theta, the softening, the walk flags
+// group_size and block_warps once more within that bound. sort_variant is
+// judged by the sort stage's own time. A knob is swept where its values run
+// different kernels (block_warps: the per-particle walk; sort_variant: counts above
+// the one-launch sort's), so that no noise is written down as a choice. theta, the softening, the walk flags
 // and the form are physics and stay as set; astro_autotune_keep also holds
 // the knobs its caller names (a workload quoted at a given tree depth).
 #include <algorithm>
@@ -41,7 +42,7 @@ struct Trial {
     double ms = 0, sort_ms = 0, err = 0;
 };
 
-enum Knob { kLbits, kBucket, kGroupSize, kBlockWarps, kSortVariant, kWalkFrontier };
+enum Knob { kLbits, kBucket, kGroupSize, kBlockWarps, kSortVariant };
 
 class Tuner {
 public:
@@ -194,13 +195,15 @@ std::vector<uint32_t> Tuner::candidates(Knob knob) const {
         }
         case kBucket: return {8, 16, 32, 64};
         case kGroupSize: return {8, 12, 16, 24, 32, 48, 64};
-        case kBlockWarps: return {4, 8};
+        case kBlockWarps:
+            if (!(base_.flags & ASTRO_FLAG_PER_PARTICLE)) return {};
+            return {4, 8};
         case kSortVariant: {
             std::vector<uint32_t> v;
-            for (uint32_t i = 1; i <= astro::sort_variant_count(); ++i) v.push_back(i);
+            if (pm_.size() > astro::sort_small_max(ctx_->device))
+                for (uint32_t i = 1; i <= astro::sort_shape_count(); ++i) v.push_back(i);
             return v;
         }
-        case kWalkFrontier: return {0, 1};
     }
     return {};
 }
@@ -213,7 +216,7 @@ int Tuner::sweep(Knob knob, double limit, Trial* best) {
         Knobs k = best->k;
         uint32_t* field = knob == kLbits ? &k.lbits : knob == kBucket ? &k.bucket
                           : knob == kGroupSize ? &k.group_size : knob == kBlockWarps ? &k.block_warps
-                          : knob == kWalkFrontier ? &k.walk_frontier : &k.sort_variant;
+                          : &k.sort_variant;
         if (*field == v) continue;
         *field = v;
         Trial t;
@@ -296,7 +299,7 @@ int Tuner::run(const char* path) {
     if ((r = measure(start, &best)) != ASTRO_OK) return r;
     const double bound = std::max((double)target_, 1.02 * best.err);
     const double acc_bound = std::max(0.8 * target_, 1.02 * best.err);
-    for (Knob k : {kLbits, kBucket, kGroupSize, kBlockWarps, kSortVariant, kWalkFrontier})
+    for (Knob k : {kLbits, kBucket, kGroupSize, kBlockWarps, kSortVariant})
         if ((r = sweep(k, bound, &best)) != ASTRO_OK) return r;
     // The accuracy knobs share one error budget.
     const Knobs base = best.k;
@@ -315,7 +318,7 @@ int Tuner::run(const char* path) {
         }
     }
     // The tree and launch knobs again (group boxes also decide far nodes).
-    for (Knob k : {kLbits, kBucket, kGroupSize, kBlockWarps, kWalkFrontier})
+    for (Knob k : {kLbits, kBucket, kGroupSize, kBlockWarps})
         if ((r = sweep(k, acc_bound, &best)) != ASTRO_OK) return r;
     if ((r = apply(best.k)) != ASTRO_OK) return r;
     return path ? write(path, best, bound, acc_bound) : ASTRO_OK;
