@@ -1503,11 +1503,8 @@ cudaError_t launch_encode_ref(const float4* pos, uint64_t* codes, uint32_t n_tre
 cudaError_t launch_encode_phys(bool prec, const Chunk* chunks, uint32_t nchunks, const SysInfo* sys,
                                float4* pos, const double* x64, uint64_t* codes, uint32_t n,
                                uint32_t lbits, cudaStream_t st) {
-    if (prec)
-        return launch_after(encode_phys_kernel<true>, nchunks, 256, 0, st, chunks, sys, pos, x64, codes, n, lbits);
-    else
-        return launch_after(encode_phys_kernel<false>, nchunks, 256, 0, st, chunks, sys, pos, x64, codes, n, lbits);
-    return cudaGetLastError();
+    return launch_after(prec ? encode_phys_kernel<true> : encode_phys_kernel<false>, nchunks, 256, 0, st, chunks, sys,
+                        pos, x64, codes, n, lbits);
 }
 
 cudaError_t launch_bbox(bool prec, const Chunk* chunks, uint32_t nchunks, const float4* pos,
@@ -1521,26 +1518,16 @@ cudaError_t launch_bbox(bool prec, const Chunk* chunks, uint32_t nchunks, const 
 cudaError_t launch_setup(bool prec, SysInfo* sys, uint32_t nsys, uint32_t* bb32,
                          unsigned long long* bb64, uint32_t lbits, float theta, uint32_t root_offset,
                          cudaStream_t st) {
-    if (prec)
-        return launch_after(setup_kernel<true>, blocks_for(nsys, 128), 128, 0, st, sys, nsys, bb32, bb64, lbits,
-                                                                  theta, root_offset);
-    else
-        return launch_after(setup_kernel<false>, blocks_for(nsys, 128), 128, 0, st, sys, nsys, bb32, bb64, lbits,
-                                                                   theta, root_offset);
-    return cudaGetLastError();
+    return launch_after(prec ? setup_kernel<true> : setup_kernel<false>, blocks_for(nsys, 128), 128, 0, st, sys, nsys,
+                        bb32, bb64, lbits, theta, root_offset);
 }
 
 cudaError_t launch_reorder(bool prec, const uint32_t* perm, const float4* pos_a, const float4* vel_a,
                            const uint32_t* id_a, const double* x_a, float4* pos_b, float4* vel_b,
                            uint32_t* id_b, double* x_b, uint32_t n, const ClearArgs& clear,
                            cudaStream_t st) {
-    if (prec)
-        return launch_after(reorder_kernel<true>, blocks_for(n, 256), 256, 0, st, perm, pos_a, vel_a, id_a, x_a, pos_b,
-                                                                 vel_b, id_b, x_b, n, clear);
-    else
-        return launch_after(reorder_kernel<false>, blocks_for(n, 256), 256, 0, st, perm, pos_a, vel_a, id_a, x_a, pos_b,
-                                                                  vel_b, id_b, x_b, n, clear);
-    return cudaGetLastError();
+    return launch_after(prec ? reorder_kernel<true> : reorder_kernel<false>, blocks_for(n, 256), 256, 0, st, perm, pos_a,
+                        vel_a, id_a, x_a, pos_b, vel_b, id_b, x_b, n, clear);
 }
 
 uint32_t topology_tiles(uint32_t n) { return blocks_for(n, kTopoThreads * topo_items(n)); }
@@ -1557,7 +1544,6 @@ cudaError_t launch_topology(const TopoArgs& a, cudaStream_t st) {
         case 4: return launch_after(topology_kernel<4>, a.ntiles, kTopoThreads, 0, st, a);
         default: return launch_after(topology_kernel<8>, a.ntiles, kTopoThreads, 0, st, a);
     }
-    return cudaGetLastError();
 }
 
 namespace {

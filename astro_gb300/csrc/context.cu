@@ -98,7 +98,7 @@ int validate_params(const astro_params* p, const char** why) {
     if (!(p->far_ratio >= 0.0f && p->far_ratio <= 0.5f))
         return (*why = "far_ratio must be in [0, 0.5]", ASTRO_ERR_INVALID_ARGUMENT);
     if (p->walk_frontier > 1)
-        return (*why = "walk_frontier must be 0 (runs) or 1 (node list)", ASTRO_ERR_INVALID_ARGUMENT);
+        return (*why = "walk_frontier must be 0 or 1", ASTRO_ERR_INVALID_ARGUMENT);
     if (p->light_sources > 0 && p->preset != ASTRO_PRESET_REFERENCE)
         return (*why = "the lighting pass needs the REFERENCE preset", ASTRO_ERR_INVALID_ARGUMENT);
     return ASTRO_OK;

@@ -417,7 +417,7 @@ __global__ __launch_bounds__(kTinyThreads, 1) void sort_tiny_kernel(
 uint32_t g_cluster[kMaxDevices] = {};  // largest cluster the device runs; 0: not asked yet
 std::mutex g_small_mutex;
 
-cudaError_t launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, uint32_t blocks,
+void launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, uint32_t blocks,
                           uint32_t threads, uint32_t slice, cudaStream_t st) {
     *cfg = cudaLaunchConfig_t{};
     cfg->gridDim = dim3(blocks);
@@ -431,7 +431,6 @@ cudaError_t launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, ui
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg->attrs = attr;
     cfg->numAttrs = 2;
-    return cudaSuccess;
 }
 
 }  // namespace

@@ -20,11 +20,6 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-template <bool kFtz>
-__device__ __forceinline__ float rsq(float x) {
-    if constexpr (kFtz) return rsqrt_ftz(x);
-    else return rsqrtf(x);
-}
 
 // Interaction terms of the PHYSICAL preset (G = g):
 //   particle / monopole:  t = G m d / (r^2 + eps^2)^(3/2)
