@@ -55,12 +55,12 @@ UNIT = "particle-updates/s"
 # two vector updates (6), counting an FMA as 2).
 FLOPS_PER_INTERACTION = 20
 FLOPS_PER_QUAD_CELL = 50
-# A far node's expansion about its walk's centre: 350 flops once per walk
-# (the field, its 6 first and 10 second derivatives from the monopole and
-# quadrupole, and their 19 sums; group_far_kernel, timed with the
-# evaluation), and 70 per particle of a group with far nodes to evaluate
-# the expansion (3 x (J rho, H rho rho, sums)).
-FLOPS_PER_FAR_NODE = 350
+# A far node's expansion about its walk's centre: 180 flops once per walk
+# (the field, its first and second derivatives from the monopole and
+# quadrupole with the traces in place of the zz components, and their 19 sums;
+# group_far_kernel, timed with the evaluation), and 70 per particle of a group
+# with far nodes to evaluate the expansion (3 x (J rho, H rho rho, sums)).
+FLOPS_PER_FAR_NODE = 180
 FLOPS_PER_FAR_EVAL = 70
 L2_FLUSH_BYTES = 256 << 20  # larger than the 129 MB L2
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of
@@ -97,7 +97,7 @@ def parse(argv=None):
                     help="group walk: nodes further than (group radius) / r from the group's "
                          "centre are summed through one expansion per group (0: none)")
     ap.add_argument("--walk-frontier", type=int, default=None, choices=[0, 1],
-                    help="group walk frontier: 0 = runs of consecutive nodes, 1 = node list")
+                    help="group walk frontier: 0 or 1, the same walk")
     ap.add_argument("--no-tuned", action="store_true", help="ignore the autotuner's file")
     ap.add_argument("--theta", type=float, default=0.7)
     ap.add_argument("--persistent", action="store_true")
