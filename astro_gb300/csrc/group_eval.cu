@@ -269,14 +269,17 @@ __device__ __forceinline__ void sum_tile(PairSet& t, const float4* src, uint32_t
 // The lists of one group: lane = copy * width + slot holds the particles
 // slot + width * k, k = 0 .. 2 pairs - 1, and its copy takes every
 // copies-th source (width 8: four copies; 4: eight; 2 and 1: 16 and 32). Returns
-// the particles listed.
+// the particles listed. width = 2^wbits, so that nothing is divided by it: divisions
+// by a width of four values made the kernel 52 KB instead of 42 (precision form with
+// quadrupoles), and its instruction cache misses cost 256 systems 190 us of 7,640,
+// 300 of 3,000 bodies 71 of 920 and 60,000 of 16 bodies 9 of 435 a step.
 template <bool kPrec, bool kQuad, bool kTiny>
 __device__ __forceinline__ uint32_t sum_lists(const TraverseArgs& a, uint2 gr, const GroupDesc& d,
-                                              FastSmem<kPrec>& sm, uint32_t lane, uint32_t width,
+                                              FastSmem<kPrec>& sm, uint32_t lane, uint32_t wbits,
                                               uint32_t pairs) {
     const uint32_t gcount = gr.y - gr.x;
-    const uint32_t copies = 32u / width;
-    const uint32_t copy = lane / width, slot = lane % width;
+    const uint32_t width = 1u << wbits, copies = 32u >> wbits;
+    const uint32_t copy = lane >> wbits, slot = lane & (width - 1u);
     const float2 e2 = make_float2(a.eps2, a.eps2);
     PairSet t;
 #pragma unroll
@@ -350,7 +353,7 @@ __device__ __forceinline__ uint32_t sum_lists(const TraverseArgs& a, uint2 gr, c
                 blk = __ldg(&a.list_next[blk]);
                 load_ids();
             }
-            const uint32_t iters = (m + copies - 1u) / copies;
+            const uint32_t iters = (m + copies - 1u) >> (5u - wbits);
             const float* cell = sm.u.cell + copy * (kQuad ? kCellWords : 4);
             if (pairs == 4u) sum_cells<kQuad, kTiny, 4>(t, cell, copies, iters, e2);
             else if (pairs == 3u) sum_cells<kQuad, kTiny, 3>(t, cell, copies, iters, e2);
@@ -418,7 +421,7 @@ __device__ __forceinline__ uint32_t sum_lists(const TraverseArgs& a, uint2 gr, c
         if (cur > 0) {
             copy_wait<1>();
             __syncwarp();
-            const uint32_t iters = (cur + copies - 1u) / copies;
+            const uint32_t iters = (cur + copies - 1u) >> (5u - wbits);
             const float4* src = sm.u.tile[b ^ 1] + copy;
             if (pairs == 4u) sum_tile<kTiny, 4>(t, src, copies, iters, e2);
             else if (pairs == 3u) sum_tile<kTiny, 3>(t, src, copies, iters, e2);
@@ -468,9 +471,9 @@ __global__ __launch_bounds__(kFastWarps * 32, kFastBlocks) void group_eval_fast_
         // (50,000-body sphere in groups of 1 / 2 / 4, lists alone: four slots
         // 627 / 387 / 227 us, 446 / 283 / 172 so; one lane a particle and copy 453 /
         // 301 / 201).
-        const uint32_t width = gcount > 32u ? 8u : (gcount > 4u ? 4u : (gcount > 2u ? 2u : 1u));
-        const uint32_t pairs = (gcount + 2u * width - 1u) / (2u * width);
-        const uint32_t sources = sum_lists<kPrec, kQuad, kTiny>(a, gr, d, sm, lane, width, pairs);
+        const uint32_t wbits = gcount > 32u ? 3u : (gcount > 4u ? 2u : (gcount > 2u ? 1u : 0u));
+        const uint32_t width = 1u << wbits, pairs = (gcount + 2u * width - 1u) >> (wbits + 1u);
+        const uint32_t sources = sum_lists<kPrec, kQuad, kTiny>(a, gr, d, sm, lane, wbits, pairs);
         __syncwarp();
         // Each lane finishes up to two particles: the copies' sums, the
         // far-node expansion, G, and the kick-drift. A particle's own entry
@@ -482,7 +485,7 @@ __global__ __launch_bounds__(kFastWarps * 32, kFastBlocks) void group_eval_fast_
         float fc[kFarCoefs];
         if (d.n_far > 0) load_far<false>(dp->far_co, a.eps2, fc);
         for (uint32_t t = lane; t < gcount; t += 32u) {
-            const uint32_t k = t / width, q = k >> 1, slot = t % width;
+            const uint32_t k = t >> wbits, q = k >> 1, slot = t & (width - 1u);
             float s[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
