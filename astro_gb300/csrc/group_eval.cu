@@ -465,9 +465,8 @@ __global__ __launch_bounds__(kFastWarps * 32, kFastBlocks) void group_eval_fast_
         const GroupDesc* dp = a.desc + (gi - rec.w);
         const GroupDesc d = load_desc(dp);
         // Groups of one to four fill fewer slots, so more lanes split the lists
-        // (50,000-body sphere in groups of 1 / 2 / 4, lists alone: four slots
-        // 627 / 387 / 227 us, 446 / 283 / 172 so; one lane a particle and copy 453 /
-        // 301 / 201).
+        // (a step of a 50,000-body sphere in groups of 1 / 2 / 4: four slots 876 / 557 /
+        // 373 us, 630 / 420 / 310 so; one lane a particle and copy 821 / 600 / 474).
         const uint32_t wbits = gcount > 32u ? 3u : (gcount > 4u ? 2u : (gcount > 2u ? 1u : 0u));
         const uint32_t width = 1u << wbits, pairs = (gcount + 2u * width - 1u) >> (wbits + 1u);
         const uint32_t sources = sum_lists<kPrec, kQuad, kTiny>(a, gr, d, sm, lane, wbits, pairs);

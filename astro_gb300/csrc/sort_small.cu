@@ -418,7 +418,7 @@ uint32_t g_cluster[kMaxDevices] = {};  // largest cluster the device runs; 0: no
 std::mutex g_small_mutex;
 
 void launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, uint32_t blocks,
-                          uint32_t threads, uint32_t slice, cudaStream_t st) {
+                   uint32_t threads, uint32_t slice, cudaStream_t st) {
     *cfg = cudaLaunchConfig_t{};
     cfg->gridDim = dim3(blocks);
     cfg->blockDim = dim3(threads);
